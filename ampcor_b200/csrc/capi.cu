@@ -379,78 +379,46 @@ bool plan_spec_blocked(int R, int W, SpecBlocks& b, std::string& err)
     return false;
 }
 
-// the tensor-core zoom: operand planes, accumulator parts and row tiles; false when Zm does not fit
-// (more than 512 accumulator columns or more shared memory than a CTA has)
-bool plan_zoom_tc(int Cf, int z, ZoomTcGeom& g)
+// the zoom: shared memory of the interpolation matrix and of each team; false when the zoomed
+// surface is too large (two Cf x Z planes and the surface beyond a CTA's shared memory)
+bool plan_zoom(int Cf, int z, ZoomGeomCols& g)
 {
-    std::memset(&g, 0, sizeof(g));
+    g = ZoomGeomCols{};
     g.Cf = Cf;
     g.z = z;
     g.Z = Cf * z;
-    const int KP = (Cf + 7) / 8 * 8;
-    g.KC = KP / 4;
-    g.NG = (Cf + 15) / 16 * 16;
-    if (g.NG > 64) return false;
-    const int zq = (g.Z + 15) / 16 * 16;
-    g.nparts = zq > 256 ? 2 : 1;
-    g.npart = ((zq + g.nparts - 1) / g.nparts + 15) / 16 * 16;
-    if (g.npart > 256) return false;
-    const int full = g.Z / 128, rem = g.Z - 128 * full;
-    g.mtiles = full + (rem ? 1 : 0);
-    g.last_m = (rem == 0 || rem > 64) ? 128 : 64;
-    // accumulators: two buffers of one Zm unit (npart columns) at columns 0 and 256; the row
-    // tiles of T^T at columns 64 mt
-    g.tmem_cols = 512;
-    if (64 * g.mtiles > 512) return false;
-    const long rg = (long)g.KC * 128;
-    const long plane_a = (long)((g.Z + 7) / 8) * rg;
-    const long plane_b = (long)(g.nparts * g.npart / 8) * rg;
-    const long plane_g = (long)(g.NG / 8) * rg;
-    // the last row tile may read row groups past U; they must land in the next plane (U's lo
-    // plane, then the B planes)
-    const long over = (long)(128 * (g.mtiles - 1) + g.last_m - (g.Z + 7) / 8 * 8) / 8 * rg;
-    if (over > plane_b) return false;
-    long off = 0;
-    g.off_ahi = 0;
-    g.off_alo = (int)(off += plane_a);
-    g.off_bhi = (int)(off += plane_a);
-    g.off_blo = (int)(off += plane_b);
-    g.off_ghi = (int)(off += plane_b);
-    g.off_glo = (int)(off += plane_g);
-    off += plane_g;
-    g.off_bar = (int)off;
-    off += 48;  // five mbarriers (the fifth is waited on only by failure-detection tests)
-    g.off_misc = (int)off;
-    off += 256;  // tensor-memory address, error flag, and the block maximum's per-warp slots
-    g.smem_bytes = (int)off;
-    return off <= 227L * 1024;
+    const long limit = 227L * 1024;
+    if ((round4(Cf * Cf) + 2L * Cf * ((g.Z + 7) & ~7) + 64) * 4 > limit) return false;
+    g.kp4 = ((Cf + 3) / 4) | 1;
+    const long row = 16L * g.kp4;
+    g.s = std::max(1, z / 2);
+    g.J = (g.Z + g.s - 1) / g.s;
+    g.Jp = g.J | 1;
+    g.off_team = (int)(g.s * g.Jp * row);
+    // kappa^2: the sum of the squares of the Dirichlet kernel's second derivative at the samples
+    double k2 = 0.0;
+    for (int n = 1; n <= Cf / 2; ++n) k2 += 2.0 / Cf * std::pow(2.0 * M_PI * n / Cf, 4);
+    g.curv = (float)(1.00001 * std::sqrt(k2) * std::pow((double)g.s / z, 2) / 8.0);
+    // G, the kept columns of T, a value per sample, the reduction slots, the kept columns and rows
+    g.g_rows = (Cf + 11) / 12 * 12;
+    g.team_bytes = (int)((g.g_rows + kZoomCols) * row + round4(g.J) * 4L + 64 + 2 * round4(g.Z) * 4L);
+    g.teams = (int)std::min<long>(kZoomTeams, (limit - g.off_team) / g.team_bytes);
+    return g.teams > 0;
 }
 
 double dirichlet(int N, double d);
 
-// hi and lo tf32 planes of U (U[p][a] = D_Cf(p / z - a), an identity row for p % z == 0), rows of
-// K-major core matrices; K past Cf is zero
-std::vector<float> zoom_u_planes(const ZoomTcGeom& g)
+// U[p][a] = D_Cf(p / z - a), an identity row for p % z == 0; rows of 4 kp4 floats, zero past Cf,
+// stored by phase: neighbouring lanes read sampled rows (one phase) and rows of one interval (all
+// phases), and both are an odd number of float4 apart
+std::vector<float> zoom_matrix(const ZoomGeomCols& g)
 {
-    const int rows = (g.Z + 7) / 8 * 8;
-    const size_t plane = (size_t)rows * g.KC * 4;
-    std::vector<float> out(2 * plane, 0.0f);
+    std::vector<float> u((size_t)g.s * g.Jp * g.kp4 * 4, 0.0f);
     for (int p = 0; p < g.Z; ++p)
-        for (int a = 0; a < g.Cf; ++a) {
-            const int s = p % g.z, b = p / g.z;
-            const float u = s == 0 ? (b == a ? 1.0f : 0.0f) : (float)dirichlet(g.Cf, (double)p / g.z - a);
-            // round to tf32: nearest, ties away from zero
-            uint32_t bits;
-            std::memcpy(&bits, &u, 4);
-            bits = (bits + 0x1000u) & 0xFFFFE000u;
-            float hi;
-            std::memcpy(&hi, &bits, 4);
-            const float lo = u - hi;
-            const size_t off = (size_t)((p / 8) * g.KC + a / 4) * 32 + (p % 8) * 4 + a % 4;
-            out[off] = hi;
-            out[plane + off] = lo;
-        }
-    return out;
+        for (int a = 0; a < g.Cf; ++a)
+            u[(size_t)((p % g.s) * g.Jp + p / g.s) * g.kp4 * 4 + a] =
+                p % g.z == 0 ? (p / g.z == a ? 1.0f : 0.0f) : (float)dirichlet(g.Cf, (double)p / g.z - a);
+    return u;
 }
 
 // exp(-2 pi i m / N), m < N, rounded from FP64
@@ -523,7 +491,6 @@ struct ampcor_handle {
     float* d_chip_taps = nullptr;
     float* d_win_taps = nullptr;
     float* d_zoom_taps = nullptr;
-    float* d_zoom_ut = nullptr;
     // arena API
     float2* h_arena = nullptr;
     float2* d_arena = nullptr;
@@ -566,10 +533,9 @@ struct ampcor_handle {
     bool coarse_staged = false, fine_staged = false;
     bool staged_on = false;  // the staged forms are allowed (AMPCOR_STAGED is not 0)
     int sms = 0;
-    // tensor-core zoom (both the tensor-core and the spectral forms), when Zm fits
-    bool zoom_tc = false;
-    ZoomTcGeom ztc{};
-    float* d_zoom_uhl = nullptr;
+    // zoom of the tensor-core and spectral forms
+    ZoomGeomCols zc{};
+    float* d_zoom_u = nullptr;
     float* d_tw_c = nullptr;
     float* d_tw_f = nullptr;
     // refinement by zero-padded FFT (spectral form): twiddles of R, f R, E and f E, in that order;
@@ -600,13 +566,12 @@ struct ampcor_handle {
     // tensor-core form
     TcGeom tcc{}, tcf{};
     NccGeom gsc{}, gsf{};
-    int zoom_smem = 0;
     float* d_inv_c = nullptr;
     float* d_inv_f = nullptr;
     float* d_gam = nullptr;
     FineOut* d_fine_out = nullptr;
     size_t fine_cap = 0;
-    // batches whose tensor-core zoom is made to time out (ampcor_inject_timeout)
+    // batches whose zoom is made to time out (ampcor_inject_timeout)
     int inject_timeouts = 0;
     // per-kernel timing: (start, stop) event pairs of each launch, per kernel kind
     // (0 coarse correlation, 1 refinement, 2 fine correlation, 3 coarse statistics,
@@ -836,22 +801,15 @@ void drop_marks(ampcor_handle* h)
     for (cudaEvent_t e : seen) cudaEventDestroy(e);
 }
 
-// the zoom of a chunk: tensor cores where Zm fits, else the FP32 kernel
+// the zoom of a chunk
 int launch_zoom(ampcor_handle* h, long long c0, unsigned n, const PairSource& src, float2* offsets,
                 PairDiag* diag, cudaStream_t st)
 {
-    const int compat = (h->prm.flags & AMPCOR_FLAG_REF_COMPAT) ? 1 : 0;
-    if (h->zoom_tc) {
-        const unsigned blocks = std::min<unsigned>(n, 148u);
-        tc_zoom_kernel<<<blocks, kTcZoomThreads, h->ztc.smem_bytes, st>>>(
-            h->d_gam, c0, n, src.ref_off, h->ztc, h->d_zoom_uhl, h->d_coarse, h->d_coarse_peak,
-            h->d_fine_out, h->M, h->f, h->m, compat, offsets, diag, h->d_tc_err, h->inject_timeouts > 0 ? 1 : 0);
-    } else {
-        zoom_kernel<<<n, 256, h->zoom_smem, st>>>(h->d_gam, c0, n, src.ref_off, h->zg, h->d_zoom_ut,
-                                                  h->d_coarse, h->d_coarse_peak, h->d_fine_out, h->M,
-                                                  h->f, h->m, compat, offsets, diag);
-    }
-    CK(h, cudaGetLastError(), "launching the zoom kernel");
+    CK(h, launch_zoom_kernel((unsigned)std::max(1, h->sms), st, h->d_gam, c0, n, src.ref_off, h->zc, h->d_zoom_u,
+                             h->d_coarse, h->d_coarse_peak, h->d_fine_out, h->M, h->f, h->m,
+                             (h->prm.flags & AMPCOR_FLAG_REF_COMPAT) ? 1 : 0, offsets, diag, h->d_tc_err,
+                             h->inject_timeouts > 0 ? 1 : 0),
+       "launching the zoom kernel");
     return AMPCOR_OK;
 }
 
@@ -1285,10 +1243,7 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         if (env && std::strcmp(env, "spectral") == 0 && h->spectral_ok) h->form = kFormSpectral;
         h->gsc = stats_layout(h->gc);
         h->gsf = stats_layout(h->gf);
-        const int Zp = (h->Z + 7) & ~7;
-        h->zoom_smem = (round4(h->Cf * h->Cf) + 2 * h->Cf * Zp + 64) * 4;
-        h->zoom_tc = plan_zoom_tc(h->Cf, h->z, h->ztc) && !std::getenv("AMPCOR_ZOOM_FP32");
-        if (!h->zoom_tc && h->zoom_smem > 227 * 1024) {
+        if (!plan_zoom(h->Cf, h->z, h->zc)) {
             delete h;
             return create_fail(AMPCOR_E_SHAPE, "the zoomed surface is too large for this build");
         }
@@ -1324,28 +1279,13 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
                                   kMaxSmem)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(tc_fine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kMaxSmem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(zoom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kMaxSmem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(tc_zoom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kMaxSmem)) != cudaSuccess ||
+        (e = zoom_set_smem_limits()) != cudaSuccess ||
         (e = spec_set_smem_limits()) != cudaSuccess)
         return cuda_create_fail(e, "configuring kernel shared memory");
 
     const std::vector<float> ct = taps_table(h->R, h->f, 1, h->ic.taps_len);
     const std::vector<float> wt = taps_table(h->E, h->f, 1, h->iw.taps_len);
     const std::vector<float> zt = taps_table(h->Cf, h->z, 0, h->zg.taps_len);
-    // transposed zoom interpolation matrix, Ut[l][q] = D_Cf(q / z - l), rows padded to 8
-    std::vector<float> zut;
-    {
-        const int Zp = (h->Z + 7) & ~7;
-        zut.assign((size_t)h->Cf * Zp, 0.0f);
-        for (int l = 0; l < h->Cf; ++l)
-            for (int q = 0; q < h->Z; ++q) {
-                const int s = q % h->z, b = q / h->z;
-                zut[(size_t)l * Zp + q] = s == 0 ? (b == l ? 1.0f : 0.0f)
-                                                 : (float)dirichlet(h->Cf, (double)q / h->z - l);
-            }
-    }
     auto upload = [&](float*& d, const std::vector<float>& v) {
         cudaError_t ue = cudaMalloc(&d, std::max<size_t>(v.size(), 1) * sizeof(float));
         if (ue != cudaSuccess) return ue;
@@ -1353,10 +1293,9 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         return ue;
     };
     if ((e = upload(h->d_chip_taps, ct)) != cudaSuccess || (e = upload(h->d_win_taps, wt)) != cudaSuccess ||
-        (e = upload(h->d_zoom_taps, zt)) != cudaSuccess || (e = upload(h->d_zoom_ut, zut)) != cudaSuccess ||
+        (e = upload(h->d_zoom_taps, zt)) != cudaSuccess || (e = upload(h->d_zoom_u, zoom_matrix(h->zc))) != cudaSuccess ||
         (e = upload(h->d_tw_c, spec_twiddle_table(std::max(h->bc.on ? h->bc.tile.N : h->spc.N, 1)))) != cudaSuccess ||
-        (e = upload(h->d_tw_f, spec_twiddle_table(std::max(h->bf.on ? h->bf.tile.N : h->spf.N, 1)))) != cudaSuccess ||
-        (h->zoom_tc && (e = upload(h->d_zoom_uhl, zoom_u_planes(h->ztc))) != cudaSuccess))
+        (e = upload(h->d_tw_f, spec_twiddle_table(std::max(h->bf.on ? h->bf.tile.N : h->spf.N, 1)))) != cudaSuccess)
         return cuda_create_fail(e, "uploading interpolation taps");
     if (h->refine_fft) {
         std::vector<float> tw;
@@ -1384,7 +1323,7 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_chip_taps);
     cudaFree(h->d_win_taps);
     cudaFree(h->d_zoom_taps);
-    cudaFree(h->d_zoom_ut);
+    cudaFree(h->d_zoom_u);
     cudaFree(h->d_arena);
     cudaFree(h->d_ref_off);
     cudaFree(h->d_tgt_off);
@@ -1405,7 +1344,6 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_fine_out);
     cudaFree(h->d_tw_c);
     cudaFree(h->d_tw_f);
-    cudaFree(h->d_zoom_uhl);
     cudaFree(h->d_tw_refine);
     cudaFree(h->d_amp);
     cudaFree(h->d_vsum);
@@ -1783,8 +1721,8 @@ int ampcor_inject_timeout(ampcor_handle* h, int batches)
 {
     if (!h) return AMPCOR_E_ARG;
     if (batches < 0) return fail(h, AMPCOR_E_ARG, "batches must not be negative");
-    if (!h->zoom_tc || h->form == kFormPlain)
-        return fail(h, AMPCOR_E_STATE, "the worker's form has no bounded tensor-core waits");
+    if (h->form == kFormPlain)
+        return fail(h, AMPCOR_E_STATE, "the worker's form has no bounded waits");
     h->inject_timeouts = batches;
     return AMPCOR_OK;
 }

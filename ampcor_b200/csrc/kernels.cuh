@@ -176,42 +176,34 @@ __global__ void tc_fine_kernel(RealTiles t, long long pair0, long long pairs, Tc
                                const float* inv, const long long* ref_off, FineOut* fout,
                                float* gam, float* surfaces, unsigned int* err);
 
-// zoom of the refined surfaces of a chunk (C^2 floats per chunk-local pair), offsets
-__global__ void zoom_kernel(const float* gam, long long pair0, long long pairs,
-                            const long long* ref_off, ZoomGeom zg, const float* zoom_ut,
-                            const CoarseOut* coarse, const float* coarse_peak, const FineOut* fout,
-                            int margin, int refine_factor, int refine_margin, int ref_compat,
-                            float2* offsets, PairDiag* diag);
+// the zoom of the refined surfaces (zoom_kernel): teams of kZoomTeam threads, a pair each, at most
+// kZoomTeams to a CTA, kZoomCols columns of the zoomed surface at a time
+constexpr int kZoomTeam = 96;
+constexpr int kZoomTeams = 8;
+constexpr int kZoomCols = 36;
 
-// tensor-core zoom (3xTF32): Zm = U G U^T with U the Z x Cf interpolation matrix, as
-// T^T = U G^T then Zm = U T; planes of K-major core matrices (8 rows x 16 bytes), K = Cf padded
-// to KC 16-byte chunks (KC even)
-struct ZoomTcGeom {
-    int Cf, z, Z;
-    int KC;        // 4-float chunks per operand row
-    int NG;        // rows of the G planes (Cf rounded to 16): N of the first product
-    int mtiles;    // tiles of rows (of T^T and of Zm): 128 each, the last one last_m (64 or 128)
-    int last_m;
-    int nparts;    // accumulator parts of Zm columns (1 or 2), npart columns each, 256 apart
-    int npart;
-    int tmem_cols;
-    int off_ahi, off_alo, off_bhi, off_blo, off_ghi, off_glo, off_bar, off_misc;  // smem bytes
-    int smem_bytes;
+struct ZoomGeomCols {
+    int Cf, z, Z;    // refined surface Cf x Cf zoomed to Z x Z, Z = z Cf
+    int s, J;        // stride and number of the sampled rows and columns, J = ceil(Z / s)
+    int Jp;          // U is stored by phase: row p at (p % s) Jp + p / s, Jp odd and at least J
+    float curv;      // h^2 / 8 kappa: the rise between two samples h = s / z apart, per unit of norm
+    int kp4;         // float4 per row of U, G and T: odd, so that rows a thread apart hit other banks
+    int g_rows;      // rows of a team's G: Cf rounded up to whole blocks of rows
+    int teams;       // teams per CTA that fit
+    int off_team;    // shared memory: U (Z rows), then team_bytes per team
+    int team_bytes;
 };
 
-// threads of tc_zoom_kernel: four warps per tensor-memory lane quarter
-constexpr int kTcZoomThreads = 512;
-
-// zoom of the refined surfaces of a chunk on the tensor cores; same outputs as zoom_kernel.
-// uhl: the hi and lo planes of U, contiguous.  One CTA per SM walks the pairs.  stall != 0 (a
-// failure-detection test) makes every CTA's first wait on a barrier nothing completes: the
-// bounded wait runs out before any work is issued and the chunk reports a time-out in err_out.
-__global__ void tc_zoom_kernel(const float* gam, long long pair0, long long pairs,
-                               const long long* ref_off, ZoomTcGeom zt, const float* uhl,
-                               const CoarseOut* coarse, const float* coarse_peak,
-                               const FineOut* fout, int margin, int refine_factor,
-                               int refine_margin, int ref_compat, float2* offsets, PairDiag* diag,
-                               unsigned int* err_out, int stall);
+// zoom of the refined surfaces of a chunk (Cf^2 floats per chunk-local pair), first maximum and
+// offsets.  u: s Jp rows of 4 kp4 floats, the interpolation matrix, zero past Cf.  stall != 0 (a
+// failure-detection test) makes every CTA wait on a barrier nothing completes: the bounded wait
+// runs out and the chunk reports a time-out in err_out.
+cudaError_t launch_zoom_kernel(unsigned sms, cudaStream_t st, const float* gam, long long pair0, unsigned n,
+                               const long long* ref_off, const ZoomGeomCols& g, const float* u,
+                               const CoarseOut* coarse, const float* coarse_peak, const FineOut* fout, int margin,
+                               int refine_factor, int refine_margin, int ref_compat, float2* offsets,
+                               PairDiag* diag, unsigned int* err_out, int stall);
+cudaError_t zoom_set_smem_limits();
 
 // spectral form: FFT correlation of one tile pair per CTA (512 threads, one CTA per SM).  The
 // N x N tile (N = N1 N2 >= W, row stride RS = N + 1 complex samples) holds the window in its real

@@ -149,33 +149,5 @@ __device__ __forceinline__ uint64_t kmajor_desc(uint32_t addr, uint32_t lead, ui
            ((uint64_t)((stride >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// D (tensor memory) [+]= A (smem descriptor) * B (smem descriptor), tf32 inputs (fp32 words whose
-// low 13 mantissa bits the tensor core ignores), FP32 accumulator
-__device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        :
-        : "r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-        : "memory");
-}
-
-// instruction descriptor: tf32 A and B, both K-major, FP32 accumulator, M x N
-__device__ __forceinline__ uint32_t instr_desc_tf32(int m, int n)
-{
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-// x = hi + lo with hi rounded to tf32 (nearest, ties away) and lo = x - hi exact in FP32
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo)
-{
-    uint32_t h;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-    hi = __uint_as_float(h);
-    lo = x - hi;
-}
-
 }  // namespace
 }  // namespace ampcor_b200

@@ -394,10 +394,9 @@ def run_b200(args):
         Cf = 2 * w.refine_factor * w.refine_margin + 1
         f = w.refine_factor
         R, W, Wf = w.chip, w.window, f * E
-        Z = w.zoom_factor * Cf
         # algorithmic work per pair of each kernel kind: the spectral kernels are bounded by the
         # bytes they must move (amplitude tiles in, placement statistics in, surfaces out), the
-        # direct forms by the flops of the direct-form sums, the zoom by its two products
+        # direct forms by the flops of the direct-form sums, the zoom by the surfaces it reads
         if worker.form == "spectral":
             work = {
                 "coarse_correlation": ("hbm", 4.0 * (W * W + R * R + C * C)),
@@ -410,7 +409,7 @@ def run_b200(args):
                 "fine_correlation": ("tensor", 2.0 * Rf ** 2 * Cf ** 2),
                 "refinement": ("tensor", 4.0 * (f * f - 1) * (R ** 3 + E ** 3)),
             }
-        work["zoom"] = ("tensor", 2.0 * (Z * Cf * Cf + Z * Z * Cf))
+        work["zoom"] = ("hbm", 4.0 * Cf * Cf + 8.0)
         names = {
             "coarse_correlation": {"tensor": "tc_coarse_kernel", "spectral": "spec_staged_kernel (coarse)"}
             .get(worker.form, "coarse_kernel"),
@@ -421,7 +420,7 @@ def run_b200(args):
             .get(worker.form, "window_stats_cplx_kernel"),
             "fine_statistics": {"spectral": "spec_chip_stats_kernel + spec_tile_stats_kernel (blocked fine stage)"}
             .get(worker.form, "window_stats_real_kernel"),
-            "zoom": "tc_zoom_kernel (zoom_kernel where Zm exceeds the tensor memory)",
+            "zoom": "zoom_kernel",
         }
         peaks = {}
         try:
@@ -443,8 +442,6 @@ def run_b200(args):
             amount = per_pair * pairs_per_region
             region_ms = k_ms / regions
             peak, unit, scale = peak_of[bound]
-            if k == "zoom":
-                peak = peak / 2.0  # tf32 runs at half the bf16 rate
             achieved = amount / (region_ms / 1000.0) / scale
             tr = traffic_table.get(names[k])
             kernels[k] = {"kernel": names[k], "bound": bound, "achieved": achieved, "peak": peak,
