@@ -432,6 +432,24 @@ std::vector<float> spec_twiddle_table(int N)
     return t;
 }
 
+// the tables of the refinement of N x N tiles: the twiddles, then for each position of the
+// transform (N2 k1 + k2 holds frequency k = k1 + N1 k2) the half-sample phase exp(i pi k / N) / N of
+// the signed frequency, 0 for the Nyquist bin
+std::vector<float> half_shift_table(int N)
+{
+    std::vector<float> t = spec_twiddle_table(N);
+    int n1 = 1, n2 = N;
+    refine_half_radices(N, n1, n2);
+    for (int p = 0; p < N; ++p) {
+        int k = p / n2 + n1 * (p % n2);
+        if (2 * k > N) k -= N;
+        const double w = 2 * k == N ? 0.0 : 1.0 / N;
+        t.push_back((float)(w * std::cos(M_PI * k / N)));
+        t.push_back((float)(w * std::sin(M_PI * k / N)));
+    }
+    return t;
+}
+
 // shared memory of the statistics kernels: the staged window and the FP64 column-sum chunk
 // (unpadded window rows: the statistics walk columns, one thread per column; the chunk of
 // column sums shrinks until two CTAs fit on an SM)
@@ -531,21 +549,15 @@ struct ampcor_handle {
     // multiprocessors
     SpecGeom spc_st{}, spf_st{};
     bool coarse_staged = false, fine_staged = false;
-    bool staged_on = false;  // the staged forms are allowed (AMPCOR_STAGED is not 0)
     int sms = 0;
     // zoom of the tensor-core and spectral forms
     ZoomGeomCols zc{};
     float* d_zoom_u = nullptr;
     float* d_tw_c = nullptr;
     float* d_tw_f = nullptr;
-    // refinement by zero-padded FFT (spectral form): twiddles of R, f R, E and f E, in that order;
-    // tiles too large to stage whole go through a per-pair buffer (d_upy, chunk x upy_len)
+    // refinement by FFT (spectral form): the tables of R, then of E (half_shift_table)
     bool refine_fft = false;
     float* d_tw_refine = nullptr;
-    bool refine_big = false;
-    bool refine_strips = false;  // every refinement through the strip kernel (AMPCOR_REFINE_STRIPS)
-    float2* d_upy = nullptr;
-    long long upy_len = 0;
     // blocked spectral stages (coarse, fine): chip statistics, placement statistics, partial
     // numerators and their scalars, all per chunk
     SpecBlocks bc{}, bf{};
@@ -667,14 +679,12 @@ void free_chunk_scratch(ampcor_handle* h)
     cudaFree(h->d_inv_blk);
     cudaFree(h->d_part);
     cudaFree(h->d_scal);
-    cudaFree(h->d_upy);
     h->d_refined = nullptr;
     h->d_inv_c = h->d_inv_f = h->d_gam = nullptr;
     h->d_cstat = nullptr;
     h->d_inv_blk = nullptr;
     h->d_part = nullptr;
     h->d_scal = nullptr;
-    h->d_upy = nullptr;
 }
 
 // a failed chunk-scratch allocation releases what was allocated, so that the next call starts
@@ -717,9 +727,6 @@ int ensure_refined(ampcor_handle* h)
             cudaMalloc(&h->d_scal, n * K * 2 * sizeof(double)) != cudaSuccess)
             return scratch_fail(h, "allocating blocked-correlation scratch");
     }
-    if (h->form == kFormSpectral && h->refine_big &&
-        cudaMalloc(&h->d_upy, n * (size_t)h->upy_len * sizeof(float2)) != cudaSuccess)
-        return scratch_fail(h, "allocating refinement scratch");
     return AMPCOR_OK;
 }
 
@@ -988,15 +995,6 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         raster_map(wmap, r.amp_tgt, src.tgt_count / src.tgt_stride, src.tgt_stride, h->spc_st.stage_rs, h->W) &&
         raster_map(cmap, r.amp_ref, src.ref_count / src.ref_stride, src.ref_stride, (h->R + 6) & ~3, h->R) &&
         raster_map(imap, r.inv_c.base, r.rows, src.tgt_stride, h->spc_st.inv_rs, h->C);
-    // the window refinement of a raster job in the staged form: its tiles come from the secondary
-    // raster (as floats, two a sample) through a tensor map
-    CUtensorMap rmap{};
-    int rs_smem = 0, rs_box = 0;
-    const bool refine_st =
-        h->staged_on && h->refine_fft && !h->refine_strips && !(h->prm.flags & AMPCOR_FLAG_DERAMP) &&
-        src.tgt_lines > 0 && src.tgt_stride > 0 && spec_refine_staged_supported(h->E, h->f, rs_smem, rs_box) &&
-        raster_map(rmap, reinterpret_cast<const float*>(src.tgt_base), src.tgt_count / src.tgt_stride,
-                   2 * src.tgt_stride, rs_box, h->E);
     for (long long c0 = p0; c0 < p1; c0 += (long long)h->chunk) {
         const unsigned n = (unsigned)std::min<long long>((long long)h->chunk, p1 - c0);
         cudaEvent_t b = mark(h, st);
@@ -1035,23 +1033,15 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         cudaEvent_t c = mark(h, st);
         keep(h, 0, b, c, h->bc.on ? 2 : 1);
         if (h->refine_fft) {
-            const float2* tw = reinterpret_cast<const float2*>(h->d_tw_refine);
-            CK(h, launch_spec_refine(h->R, n, st, src.ref_base, src.ref_off, src.ref_stride, nullptr, c0,
-                                     n, src.ref_off, tw, tw + h->R, h->d_refined, h->refined_stride, 0,
-                                     (h->prm.flags & AMPCOR_FLAG_DERAMP) ? 1 : 0, h->d_upy, h->refine_strips),
+            const float2* tab = reinterpret_cast<const float2*>(h->d_tw_refine);
+            const bool deramp = (h->prm.flags & AMPCOR_FLAG_DERAMP) != 0;
+            CK(h, launch_refine_half(h->R, n, st, src.ref_base, src.ref_off, src.ref_stride, nullptr, c0, n,
+                                     src.ref_off, tab, h->d_refined, h->refined_stride, 0, deramp),
                "launching the chip refinement");
-            if (refine_st)
-                CK(h, launch_spec_refine_staged(h->E, (unsigned)h->sms, st, &rmap, src.tgt_off, src.tgt_stride,
-                                                h->d_coarse, c0, n, src.ref_off, tw + h->R + h->Rf,
-                                                tw + h->R + h->Rf + h->E, h->d_refined, h->refined_stride,
-                                                (long long)h->Rf * h->Rf, h->d_tc_err),
-                   "launching the staged window refinement");
-            else
-                CK(h, launch_spec_refine(h->E, n, st, src.tgt_base, src.tgt_off, src.tgt_stride, h->d_coarse,
-                                         c0, n, src.ref_off, tw + h->R + h->Rf, tw + h->R + h->Rf + h->E,
-                                         h->d_refined, h->refined_stride, (long long)h->Rf * h->Rf,
-                                         (h->prm.flags & AMPCOR_FLAG_DERAMP) ? 1 : 0, h->d_upy, h->refine_strips),
-                   "launching the window refinement");
+            CK(h, launch_refine_half(h->E, n, st, src.tgt_base, src.tgt_off, src.tgt_stride, h->d_coarse, c0, n,
+                                     src.ref_off, tab + 2 * h->R, h->d_refined, h->refined_stride,
+                                     (long long)h->Rf * h->Rf, deramp),
+               "launching the window refinement");
         } else {
             refine_kernel<<<n, kThreads, h->refine_smem, st>>>(src, c0, n, h->d_coarse, h->ic, h->iw,
                                                                h->d_chip_taps, h->d_win_taps,
@@ -1194,18 +1184,9 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         h->plain_ok = plan_ncc(h->R, h->W, 0, 0, h->gc, perr) &&
                       plan_ncc(h->Rf, h->Wf, h->Cf * h->Z, h->z * h->zg.taps_len, h->gf, perr) && interp_ok;
         h->tensor_ok = h->plain_ok && plan_tc(h->R, h->W, 8, h->tcc, terr) && plan_tc(h->Rf, h->Wf, 4, h->tcf, terr);
-        int sm_c = 0, sm_w = 0;
-        const bool small_c = spec_refine_supported(h->R, h->f, sm_c), small_w = spec_refine_supported(h->E, h->f, sm_w);
-        const bool big_c = !small_c && spec_refine_big_supported(h->R, h->f, sm_c);
-        const bool big_w = !small_w && spec_refine_big_supported(h->E, h->f, sm_w);
-        h->refine_fft = (small_c || big_c) && (small_w || big_w) &&
+        int n1 = 0, n2 = 0;
+        h->refine_fft = h->f == 2 && refine_half_radices(h->R, n1, n2) && refine_half_radices(h->E, n1, n2) &&
                         !(std::getenv("AMPCOR_REFINE_TAPS") && interp_ok);
-        int sm_sc = 0, sm_sw = 0;
-        h->refine_strips = h->refine_fft && std::getenv("AMPCOR_REFINE_STRIPS") &&
-                           std::atoi(std::getenv("AMPCOR_REFINE_STRIPS")) == 1 &&
-                           spec_refine_big_supported(h->R, h->f, sm_sc) && spec_refine_big_supported(h->E, h->f, sm_sw);
-        h->refine_big = h->refine_fft && (big_c || big_w || h->refine_strips);
-        h->upy_len = std::max((long long)h->R * h->Rf, (long long)h->E * h->Wf);
         const bool direct_c = plan_spec(h->R, h->W, h->spc, serr);
         const bool coarse_ok = direct_c || plan_spec_blocked(h->R, h->W, h->bc, serr);
         const bool direct_f = coarse_ok && plan_spec(h->Rf, h->Wf, h->spf, serr);
@@ -1213,7 +1194,6 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         // pair are dense rows of one buffer, staged whole when its rows are 16-byte multiples
         const char* stg = std::getenv("AMPCOR_STAGED");
         const bool staged_on = !(stg && std::strcmp(stg, "0") == 0);
-        h->staged_on = staged_on;
         h->coarse_staged = staged_on && direct_c && plan_spec_staged(h->R, h->W, false, h->spc_st);
         h->fine_staged = staged_on && direct_f &&
                          plan_spec_staged(h->Rf, h->Wf, h->Rf % 2 == 0 && h->Wf % 2 == 0, h->spf_st) &&
@@ -1280,7 +1260,7 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         (e = cudaFuncSetAttribute(tc_fine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kMaxSmem)) != cudaSuccess ||
         (e = zoom_set_smem_limits()) != cudaSuccess ||
-        (e = spec_set_smem_limits()) != cudaSuccess)
+        (e = refine_half_set_smem_limits()) != cudaSuccess || (e = spec_set_smem_limits()) != cudaSuccess)
         return cuda_create_fail(e, "configuring kernel shared memory");
 
     const std::vector<float> ct = taps_table(h->R, h->f, 1, h->ic.taps_len);
@@ -1299,8 +1279,8 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         return cuda_create_fail(e, "uploading interpolation taps");
     if (h->refine_fft) {
         std::vector<float> tw;
-        for (int n : {h->R, h->Rf, h->E, h->Wf}) {
-            const std::vector<float> t = spec_twiddle_table(n);
+        for (int n : {h->R, h->E}) {
+            const std::vector<float> t = half_shift_table(n);
             tw.insert(tw.end(), t.begin(), t.end());
         }
         if ((e = upload(h->d_tw_refine, tw)) != cudaSuccess)
@@ -1352,7 +1332,6 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_inv_blk);
     cudaFree(h->d_part);
     cudaFree(h->d_scal);
-    cudaFree(h->d_upy);
     drop_marks(h);
     if (h->h_arena) cudaFreeHost(h->h_arena);
     if (h->h_offsets) cudaFreeHost(h->h_offsets);

@@ -286,28 +286,15 @@ bool spec_radices(int n, int& n1, int& n2);
 int spec_next_length(int w);
 // allow every instantiation its shared memory; call once per device
 cudaError_t spec_set_smem_limits();
-// refinement by zero-padded FFT for an N x N tile and factor f, when compiled (smem: its bytes)
-bool spec_refine_supported(int n, int f, int& smem);
-// refinement in strips through a per-pair buffer of N x 2N complex samples in global memory
-// (ybuf, blocks of them): tiles too large for one CTA's shared memory (N in 96 .. 160, f = 2), and
-// with `strips` the shorter compiled lengths too (less shared memory, more CTAs per SM)
-bool spec_refine_big_supported(int n, int f, int& smem);
-// refinement of raster windows by the staged kernel (one resident CTA per SM, the next tile copied
-// in by the copy engine): whether compiled for N x N tiles and factor f, its shared memory and the
-// width (floats) of the tensor map's box; tmap maps the secondary raster as floats (2 per sample)
-// with boxes of box_x x N floats
-bool spec_refine_staged_supported(int n, int f, int& smem, int& box_x);
-cudaError_t launch_spec_refine_staged(int n, unsigned sms, cudaStream_t st, const CUtensorMap* tmap,
-                                      const long long* off, long long stride, const CoarseOut* coarse,
-                                      long long pair0, long long pairs, const long long* valid,
-                                      const float2* twn, const float2* twf, float* refined,
-                                      long long refined_stride, long long out_off, unsigned int* errs);
-cudaError_t launch_spec_refine(int n, unsigned blocks, cudaStream_t st, const float2* base,
-                               const long long* off, long long stride, const CoarseOut* coarse,
-                               long long pair0, long long pairs, const long long* valid,
-                               const float2* twn, const float2* twf, float* refined,
-                               long long refined_stride, long long out_off, int deramp,
-                               float2* ybuf, bool strips);
+// refinement of N x N complex tiles by 2 (refine_fft.cu): the radices of a compiled N; the kernel
+// over a chunk's chips (coarse null) or nudged windows.  tab: N twiddles, then the half-sample
+// phases over N of the frequencies at the transform's positions.
+bool refine_half_radices(int n, int& n1, int& n2);
+cudaError_t refine_half_set_smem_limits();
+cudaError_t launch_refine_half(int n, unsigned blocks, cudaStream_t st, const float2* base, const long long* off,
+                               long long stride, const CoarseOut* coarse, long long pair0, long long pairs,
+                               const long long* valid, const float2* tab, float* refined, long long refined_stride,
+                               long long out_off, bool deramp);
 
 // blocked spectral correlation (windows too large for one tile; see spectral.cu): per chunk of
 // pairs the chip statistics, the placement statistics when no raster gives them, the partial

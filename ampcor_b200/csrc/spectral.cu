@@ -44,12 +44,6 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-__device__ __forceinline__ void cp_async8_g(void* dst, const void* src)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
@@ -969,315 +963,6 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
     }
 }
 
-// ------------------------------------------------------------------------------------------
-// refinement by zero-padded FFT (the reference's band-limited upsampling, refine.cu / cuFFT)
-// ------------------------------------------------------------------------------------------
-
-// Upsample the N x N complex tile at src (rows stride apart) by F / N and write its amplitudes
-// (F x F, dense, row stride F) to out: the tile's 2-D forward transform (N-point FFTs along the
-// rows, then down the N columns), F-point inverses down the N columns that pad each column's
-// spectrum on the fly (F x N), then CB rows at a time the F-point inverses along the rows, again
-// padding on the fly, and the amplitudes out.  Scaled by 1 / N^2.  Transforming both axes forward
-// before padding either costs N + N + N + F transforms, against N + N + F + F when the rows are
-// upsampled first.
-template <int N1, int N2, int F1, int F2>
-struct UpsampleGeom {
-    static constexpr int N = N1 * N2, F = F1 * F2;
-    static constexpr int RSN = N + 1, RSY = N + 1, RSB = F + 1;
-    // output rows per block: the block buffer reuses the tile's space
-    static constexpr int CBX = N * RSN / RSB;
-    static constexpr int CB = CBX < 32 ? CBX : 32;
-    static constexpr int smem = (N * RSN + F * RSY + N + F) * 8;
-    static_assert(CB >= 1, "the row block must fit in the tile's space");
-    // staged form (spec_refine_staged_kernel): the tile as copied from the raster, N rows of SWS
-    // floats (2 N + 2 from the 16-byte boundary at or before its first sample), then the copy's
-    // mbarrier and the CTA's wait-failure flag
-    static constexpr int SWS = (2 * N + 5) & ~3;
-    static constexpr int off_stage = (smem + 127) / 128 * 128;
-    static constexpr int off_bar = off_stage + N * SWS * 4;
-    static constexpr int smem_staged = off_bar + 16;
-};
-
-template <int N1, int N2, int F1, int F2>
-__device__ void upsample_core(unsigned char* sm, float2 mu, float* __restrict__ out);
-
-template <int N1, int N2, int F1, int F2, bool DERAMP>
-__device__ void fft_upsample(const float2* __restrict__ src, long long stride, unsigned char* sm,
-                             const float2* __restrict__ twn_g, const float2* __restrict__ twf_g,
-                             float* __restrict__ out)
-{
-    using G = UpsampleGeom<N1, N2, F1, F2>;
-    constexpr int N = G::N, F = G::F, RSN = G::RSN, RSY = G::RSY, RSB = G::RSB, CB = G::CB;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float2* X = reinterpret_cast<float2*>(sm);   // the tile, later a block of F-point rows
-    float2* Y = X + N * RSN;                     // columns upsampled: F x N
-    float2* twn = Y + F * RSY;
-    float2* twf = twn + N;
-    for (int k = tid; k < N; k += kThreads) twn[k] = __ldg(twn_g + k);
-    for (int k = tid; k < F; k += kThreads) twf[k] = __ldg(twf_g + k);
-    float2 mu;
-    if constexpr (DERAMP) {
-        for (int y = warp; y < N; y += kWarps)
-            for (int x = lane; x < N; x += 32) cp_async8_g(X + y * RSN + x, src + y * stride + x);
-        cp_async_wait_all();
-        __syncthreads();
-        // the upsampled-columns buffer is free until the columns are written: the deramp's scratch
-        deramp_tile(X, RSN, N, reinterpret_cast<double*>(Y));
-        // the tile's mean comes off as the rows are read and back on with the amplitudes
-        mu = tile_mean<false, false>(X, RSN, N, 0.0f, 0.0f, reinterpret_cast<double*>(Y));
-    } else {
-        // the tile through registers, its sum taken on the way (tile_mean's order: FP32 sums per
-        // thread over samples tid, tid + kThreads, ..., FP64 across the block); the mean comes
-        // off as the rows are read and back on with the amplitudes
-        constexpr int KT = (N * N + kThreads - 1) / kThreads;
-        float2 v[KT];
-#pragma unroll
-        for (int q = 0; q < KT; ++q) {
-            const int k = tid + q * kThreads;
-            v[q] = k < N * N ? __ldg(src + (k / N) * stride + k % N) : make_float2(0.0f, 0.0f);
-        }
-        float sx = 0.0f, sy = 0.0f;
-#pragma unroll
-        for (int q = 0; q < KT; ++q) {
-            const int k = tid + q * kThreads;
-            if (k < N * N) {
-                X[(k / N) * RSN + k % N] = v[q];
-                sx += v[q].x;
-                sy += v[q].y;
-            }
-        }
-        double* red = reinterpret_cast<double*>(Y);
-        const double a = warp_sum((double)sx), b = warp_sum((double)sy);
-        if (lane == 0) {
-            red[2 * warp] = a;
-            red[2 * warp + 1] = b;
-        }
-        __syncthreads();
-        double ta = 0.0, tb = 0.0;
-        for (int w = 0; w < kWarps; ++w) {
-            ta += red[2 * w];
-            tb += red[2 * w + 1];
-        }
-        const double cells = (double)N * (double)N;
-        mu = make_float2((float)(ta / cells), (float)(tb / cells));
-    }
-    upsample_core<N1, N2, F1, F2>(sm, mu, out);
-}
-
-// the transforms of fft_upsample and the amplitudes out, from the tile in place (X) with its mean
-// mu and the twiddles in shared memory
-template <int N1, int N2, int F1, int F2>
-__device__ void upsample_core(unsigned char* sm, float2 mu, float* __restrict__ out)
-{
-    using G = UpsampleGeom<N1, N2, F1, F2>;
-    constexpr int N = G::N, F = G::F, RSN = G::RSN, RSY = G::RSY, RSB = G::RSB, CB = G::CB;
-    const int tid = threadIdx.x;
-    float2* X = reinterpret_cast<float2*>(sm);
-    float2* Y = X + N * RSN;
-    const float2* twn = Y + F * RSY;
-    const float2* twf = twn + N;
-    // rows: forward N
-    for (int t = tid; t < N * N2; t += kThreads) fft::fwd_a_minus<N1, N2>(X + (t % N) * RSN, 1, t / N, twn, mu);
-    __syncthreads();
-    for (int t = tid; t < N * N1; t += kThreads) fft::step_b<N1, N2, -1>(X + (t % N) * RSN, 1, t / N);
-    __syncthreads();
-    // columns: forward N
-    for (int t = tid; t < N * N2; t += kThreads) fft::fwd_a<N1, N2>(X + t % N, RSN, t / N, twn);
-    __syncthreads();
-    for (int t = tid; t < N * N1; t += kThreads) fft::step_b<N1, N2, -1>(X + t % N, RSN, t / N);
-    __syncthreads();
-    // columns: inverse F, the first step padding each column's spectrum as it reads it
-    for (int t = tid; t < N * F1; t += kThreads)
-        fft::step_b_pad<N1, N2, F1, F2>(X + t % N, RSN, Y + t % N, RSY, t / N);
-    __syncthreads();
-    for (int t = tid; t < N * F2; t += kThreads) fft::inv_a<F1, F2>(Y + t % N, RSY, t / N, twf);
-    __syncthreads();
-    const float scale = 1.0f / ((float)N * (float)N);
-    for (int r0 = 0; r0 < F; r0 += CB) {
-        const int nr = F - r0 < CB ? F - r0 : CB;
-        // a block of rows: inverse F (padding on the fly), amplitudes out
-        for (int t = tid; t < CB * F1; t += kThreads) {
-            const int r = t % CB;
-            if (r < nr) fft::step_b_pad<N1, N2, F1, F2>(Y + (r0 + r) * RSY, 1, X + r * RSB, 1, t / CB);
-        }
-        __syncthreads();
-        // the last step writes the amplitudes of its outputs straight to global memory; lanes take
-        // consecutive outputs of a row, so the stores coalesce
-        for (int t = tid; t < CB * F2; t += kThreads) {
-            const int r = t / F2, n2 = t - r * F2;
-            if (r < nr) {
-                float* row = out + (long long)(r0 + r) * F;
-                fft::inv_a_store<F1, F2>(X + r * RSB, 1, n2, twf, [&](int n, float2 v) {
-                    const float re = fmaf(v.x, scale, mu.x), im = fmaf(v.y, scale, mu.y);
-                    row[n] = sqrtf(re * re + im * im);
-                });
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// one tile of every pair of a chunk: the chip (coarse == nullptr) or the nudged window; two CTAs
-// per SM where their shared memory allows
-template <int N1, int N2, int F1, int F2, bool DERAMP>
-__global__ void __launch_bounds__(kThreads, UpsampleGeom<N1, N2, F1, F2>::smem <= 113 * 1024 ? 2 : 1)
-spec_refine_kernel(const float2* base, const long long* off, long long stride,
-                   const CoarseOut* coarse, long long pair0, long long pairs, const long long* valid,
-                   const float2* twn, const float2* twf, float* refined, long long refined_stride,
-                   long long out_off)
-{
-    extern __shared__ __align__(16) unsigned char rsm[];
-    if (blockIdx.x >= pairs) return;
-    const long long p = pair0 + blockIdx.x;
-    if (valid[p] < 0) return;
-    const float2* src = base + off[p];
-    if (coarse) {
-        const CoarseOut co = coarse[p];
-        src += co.top * stride + co.left;
-    }
-    fft_upsample<N1, N2, F1, F2, DERAMP>(
-        src, stride, rsm, twn, twf, refined + (long long)blockIdx.x * refined_stride + out_off);
-}
-
-// Refinement of the windows of a raster job, staged: one resident CTA per SM walks the pairs of
-// the chunk, and the copy engine brings the next pair's tile (the box of the secondary raster,
-// as floats, at the nudged corner of its coarse result) into a buffer of its own while this
-// pair's transforms run.  The tile goes from that buffer into place with its sum taken in
-// fft_upsample's order, so the amplitudes are fft_upsample's bit for bit.  Every wait is
-// bounded; one that runs out is counted in errs, the CTA lets its copy land (bounded) and returns.
-template <int N1, int N2, int F1, int F2>
-__global__ void __launch_bounds__(kThreads, 1)
-spec_refine_staged_kernel(const __grid_constant__ CUtensorMap tmap, const long long* off, long long stride,
-                          const CoarseOut* coarse, long long pair0, long long pairs, const long long* valid,
-                          const float2* twn_g, const float2* twf_g, float* refined, long long refined_stride,
-                          long long out_off, unsigned int* errs)
-{
-    extern __shared__ __align__(16) unsigned char rsm[];
-    using G = UpsampleGeom<N1, N2, F1, F2>;
-    constexpr int N = G::N, F = G::F, RSN = G::RSN, RSY = G::RSY, SWS = G::SWS;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float2* X = reinterpret_cast<float2*>(rsm);
-    float2* Y = X + N * RSN;
-    float2* twn = Y + F * RSY;
-    float2* twf = twn + N;
-    float* stage = reinterpret_cast<float*>(rsm + G::off_stage);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(rsm + G::off_bar);
-    int& s_err = *reinterpret_cast<int*>(rsm + G::off_bar + 8);
-    for (int k = tid; k < N; k += kThreads) twn[k] = __ldg(twn_g + k);
-    for (int k = tid; k < F; k += kThreads) twf[k] = __ldg(twf_g + k);
-    if (tid == 0) {
-        s_err = 0;
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    // first sample of chunk pair b's tile: line y, sample x of the raster
-    auto corner = [&](long long b, int& x, int& y) {
-        const long long p = pair0 + b;
-        const CoarseOut co = coarse[p];
-        const long long o = off[p] + co.top * stride + co.left;
-        const long long yy = o / stride;
-        y = (int)yy;
-        x = (int)(o - yy * stride);
-    };
-    // thread 0: chunk pair b's tile into the staging buffer; a pair without tiles copies nothing
-    auto issue = [&](long long b) {
-        if (valid[pair0 + b] < 0) {
-            mbar_arrive(bar);
-            return;
-        }
-        int x, y;
-        corner(b, x, y);
-        mbar_expect_tx(bar, (unsigned)(N * SWS * 4));
-        tensor_to_smem(stage, &tmap, (2 * x) & ~3, y, bar);
-    };
-    if (tid == 0 && blockIdx.x < pairs) issue(blockIdx.x);
-    uint32_t parity = 0;
-    bool inflight = blockIdx.x < pairs;
-    for (long long b = blockIdx.x; b < pairs; b += gridDim.x) {
-        const long long p = pair0 + b;
-        const long long bn = b + gridDim.x;
-        const bool ok = valid[p] >= 0;
-        int of = 0;
-        if (ok) {
-            int x, y;
-            corner(b, x, y);
-            of = (2 * x) & 3;
-        }
-        const bool landed = mbar_wait(bar, parity, &s_err);
-        if (__syncthreads_or(!landed)) break;
-        parity ^= 1u;
-        inflight = false;
-        if (!ok) {
-            if (bn < pairs) {
-                fence_async_smem();
-                __syncthreads();
-                if (tid == 0) issue(bn);
-                inflight = true;
-            }
-            continue;
-        }
-        // the tile into place, its sum taken on the way (fft_upsample's order)
-        constexpr int KT = (N * N + kThreads - 1) / kThreads;
-        float sx = 0.0f, sy = 0.0f;
-#pragma unroll
-        for (int q = 0; q < KT; ++q) {
-            const int k = tid + q * kThreads;
-            if (k < N * N) {
-                const int y = k / N, x = k % N;
-                const float2 v = *reinterpret_cast<const float2*>(stage + y * SWS + of + 2 * x);
-                X[y * RSN + x] = v;
-                sx += v.x;
-                sy += v.y;
-            }
-        }
-        double* red = reinterpret_cast<double*>(Y);
-        const double a = warp_sum((double)sx), c = warp_sum((double)sy);
-        if (lane == 0) {
-            red[2 * warp] = a;
-            red[2 * warp + 1] = c;
-        }
-        // the staging buffer is read: the next pair's tile comes in while this one is transformed
-        fence_async_smem();
-        __syncthreads();
-        if (bn < pairs) {
-            if (tid == 0) issue(bn);
-            inflight = true;
-        }
-        double ta = 0.0, tb = 0.0;
-        for (int w = 0; w < kWarps; ++w) {
-            ta += red[2 * w];
-            tb += red[2 * w + 1];
-        }
-        const double cells = (double)N * (double)N;
-        const float2 mu = make_float2((float)(ta / cells), (float)(tb / cells));
-        upsample_core<N1, N2, F1, F2>(rsm, mu, refined + b * refined_stride + out_off);
-    }
-    if (s_err) {
-        // a wait ran out: count it once per CTA and let the copy in flight land before the shared
-        // memory is given up
-        if (tid == 0) {
-            atomicAdd(errs, 1u);
-            if (inflight) {
-                const long long t0 = clock64();
-                while (!mbar_try(bar, parity) && clock64() - t0 < kSpinCycles) {
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// refinement (N, F = 2 N) pairs that are compiled: N, N1, N2, F1, F2
-#define AMPCOR_REFINE_PAIRS(X) \
-    X(16, 4, 4, 4, 8)          \
-    X(24, 4, 6, 6, 8)          \
-    X(32, 4, 8, 8, 8)          \
-    X(40, 5, 8, 8, 10)         \
-    X(48, 6, 8, 8, 12)         \
-    X(64, 8, 8, 8, 16)         \
-    X(80, 8, 10, 10, 16)
-
 // transform lengths: N, N1, N2 (N1 N2 = N)
 #define AMPCOR_SPEC_LENGTHS(X) \
     X(16, 4, 4)                \
@@ -1563,168 +1248,6 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
     }
 }
 
-// The linear-phase steps of an n x n complex tile in global memory (rows `stride` apart), as
-// deramp_tile measures them: the phases of the lag-one autocorrelations along samples and lines.
-// red: 4 kWarps doubles; every thread gets both phases; ends with a barrier.
-__device__ void deramp_phases_global(const float2* t, long long stride, int n, double* red, float& ps, float& pl)
-{
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float sr = 0.0f, si = 0.0f, lr = 0.0f, li = 0.0f;
-    for (int k = tid; k < n * n; k += kThreads) {
-        const int y = k / n, x = k - y * n;
-        const float2 z = __ldg(t + y * stride + x);
-        if (x + 1 < n) {
-            const float2 w = __ldg(t + y * stride + x + 1);
-            sr = fmaf(w.x, z.x, fmaf(w.y, z.y, sr));
-            si = fmaf(w.y, z.x, fmaf(-w.x, z.y, si));
-        }
-        if (y + 1 < n) {
-            const float2 w = __ldg(t + (y + 1) * stride + x);
-            lr = fmaf(w.x, z.x, fmaf(w.y, z.y, lr));
-            li = fmaf(w.y, z.x, fmaf(-w.x, z.y, li));
-        }
-    }
-    double v[4] = {sr, si, lr, li};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = warp_sum(v[q]);
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) red[4 * warp + q] = v[q];
-    __syncthreads();
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int w = 0; w < kWarps; ++w)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) a[q] += red[4 * w + q];
-    ps = (float)atan2(a[1], a[0]);
-    pl = (float)atan2(a[3], a[2]);
-    __syncthreads();
-}
-
-// Band-limited upsampling of tiles too large to stage whole (N up to 160, F = 2 N): the transforms
-// of fft_upsample in the rows-first order (the mean off as there), a strip of ST rows at a time (N-point FFTs, F-point
-// padded inverses) into a per-pair buffer in global memory (N x F complex, row-major), then the
-// columns of that buffer CB at a time (N-point FFTs, F-point padded inverses, amplitudes out).
-template <int N1, int N2, int F1, int F2>
-struct BigUpsampleGeom {
-    static constexpr int N = N1 * N2, F = F1 * F2, ST = 32, CB = 32;
-    static constexpr int XS = ST * (N + 1) > N * (CB + 1) ? ST * (N + 1) : N * (CB + 1);  // float2
-    static constexpr int YS = ST * (F + 1) > F * (CB + 1) ? ST * (F + 1) : F * (CB + 1);
-    static constexpr int smem = (XS + YS + N + F) * 8 + 4 * kWarps * 8;
-};
-
-template <int N1, int N2, int F1, int F2, bool DERAMP>
-__global__ void __launch_bounds__(kThreads, BigUpsampleGeom<N1, N2, F1, F2>::smem <= 113 * 1024 ? 2 : 1)
-spec_refine_big_kernel(const float2* base, const long long* off, long long stride, const CoarseOut* coarse,
-                       long long pair0, long long pairs, const long long* valid, const float2* twn_g,
-                       const float2* twf_g, float2* ybuf, float* refined, long long refined_stride,
-                       long long out_off)
-{
-    using G = BigUpsampleGeom<N1, N2, F1, F2>;
-    constexpr int N = G::N, F = G::F, ST = G::ST, CB = G::CB;
-    constexpr int RSN = N + 1, RSF = F + 1, CBS = CB + 1;
-    extern __shared__ __align__(16) unsigned char rsm[];
-    if (blockIdx.x >= pairs) return;
-    const long long p = pair0 + blockIdx.x;
-    if (valid[p] < 0) return;
-    const float2* src = base + off[p];
-    if (coarse) {
-        const CoarseOut co = coarse[p];
-        src += co.top * stride + co.left;
-    }
-    float2* X = reinterpret_cast<float2*>(rsm);
-    float2* Y = X + G::XS;
-    float2* twn = Y + G::YS;
-    float2* twf = twn + N;
-    double* red = reinterpret_cast<double*>(twf + F);
-    float2* yg = ybuf + (long long)blockIdx.x * N * F;
-    float* out = refined + (long long)blockIdx.x * refined_stride + out_off;
-    const int tid = threadIdx.x;
-    for (int q = tid; q < N; q += kThreads) twn[q] = __ldg(twn_g + q);
-    for (int q = tid; q < F; q += kThreads) twf[q] = __ldg(twf_g + q);
-    float ps = 0.0f, pl = 0.0f;
-    if (DERAMP) deramp_phases_global(src, stride, N, red, ps, pl);
-    // the tile's mean comes off as the strips are read and back on with the amplitudes
-    const float2 mu = tile_mean<true, DERAMP>(src, stride, N, ps, pl, red);
-    // rows, a strip at a time, into the buffer
-    for (int r0 = 0; r0 < N; r0 += ST) {
-        const int nr = N - r0 < ST ? N - r0 : ST;
-        for (int t = tid; t < nr * N; t += kThreads) {
-            const int y = t / N, x = t - y * N;
-            float2 z = __ldg(src + (long long)(r0 + y) * stride + x);
-            if (DERAMP) {
-                float s, c;
-                sincosf(fmaf(ps, (float)x, pl * (float)(r0 + y)), &s, &c);
-                z = make_float2(fmaf(z.x, c, z.y * s), fmaf(z.y, c, -z.x * s));
-            }
-            X[y * RSN + x] = make_float2(z.x - mu.x, z.y - mu.y);
-        }
-        __syncthreads();
-        for (int t = tid; t < nr * N2; t += kThreads) fft::fwd_a<N1, N2>(X + (t % nr) * RSN, 1, t / nr, twn);
-        __syncthreads();
-        for (int t = tid; t < nr * N1; t += kThreads) fft::step_b<N1, N2, -1>(X + (t % nr) * RSN, 1, t / nr);
-        __syncthreads();
-        for (int t = tid; t < nr * F1; t += kThreads)
-            fft::step_b_pad<N1, N2, F1, F2>(X + (t % nr) * RSN, 1, Y + (t % nr) * RSF, 1, t / nr);
-        __syncthreads();
-        for (int t = tid; t < nr * F2; t += kThreads) fft::inv_a<F1, F2>(Y + (t % nr) * RSF, 1, t / nr, twf);
-        __syncthreads();
-        for (int t = tid; t < nr * F; t += kThreads) {
-            const int y = t / F, x = t - y * F;
-            yg[(long long)(r0 + y) * F + x] = Y[y * RSF + x];
-        }
-        __syncthreads();
-    }
-    // columns of the buffer, CB at a time
-    const float scale = 1.0f / ((float)N * (float)N);
-    for (int c0 = 0; c0 < F; c0 += CB) {
-        const int nc = F - c0 < CB ? F - c0 : CB;
-        for (int t = tid; t < N * CB; t += kThreads) {
-            const int y = t / CB, cc = t - y * CB;
-            if (cc < nc) X[y * CBS + cc] = yg[(long long)y * F + c0 + cc];
-        }
-        __syncthreads();
-        for (int t = tid; t < CB * N2; t += kThreads) {
-            const int cc = t % CB;
-            if (cc < nc) fft::fwd_a<N1, N2>(X + cc, CBS, t / CB, twn);
-        }
-        __syncthreads();
-        for (int t = tid; t < CB * N1; t += kThreads) {
-            const int cc = t % CB;
-            if (cc < nc) fft::step_b<N1, N2, -1>(X + cc, CBS, t / CB);
-        }
-        __syncthreads();
-        for (int t = tid; t < CB * F1; t += kThreads) {
-            const int cc = t % CB;
-            if (cc < nc) fft::step_b_pad<N1, N2, F1, F2>(X + cc, CBS, Y + cc, CBS, t / CB);
-        }
-        __syncthreads();
-        for (int t = tid; t < CB * F2; t += kThreads) {
-            const int cc = t % CB;
-            if (cc < nc) {
-                float* col = out + c0 + cc;
-                fft::inv_a_store<F1, F2>(Y + cc, CBS, t / CB, twf, [&](int n, float2 v) {
-                    const float re = fmaf(v.x, scale, mu.x), im = fmaf(v.y, scale, mu.y);
-                    col[(long long)n * F] = sqrtf(re * re + im * im);
-                });
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// refinement lengths of the strip kernel: N, N1, N2, F1, F2 (F = 2 N); 96 and up are too large for
-// fft_upsample, the shorter ones may run either way (AMPCOR_REFINE_STRIPS)
-#define AMPCOR_REFINE_BIG(X) \
-    X(32, 4, 8, 8, 8)        \
-    X(48, 6, 8, 8, 12)       \
-    X(64, 8, 8, 8, 16)       \
-    X(80, 8, 10, 10, 16)     \
-    X(96, 8, 12, 12, 16)     \
-    X(120, 8, 15, 15, 16)    \
-    X(128, 8, 16, 16, 16)    \
-    X(144, 12, 12, 12, 24)   \
-    X(160, 10, 16, 16, 20)
-
 }  // namespace
 
 __global__ void detect_kernel(const float2* __restrict__ src, long long n, float* __restrict__ dst)
@@ -1886,118 +1409,10 @@ int spec_next_length(int w)
     return 0;
 }
 
-bool spec_refine_supported(int n, int f, int& smem)
-{
-    if (f != 2) return false;
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D)                \
-    if (n == NN) {                                        \
-        smem = UpsampleGeom<A, B, C, D>::smem;           \
-        return smem <= 227 * 1024;                        \
-    }
-    AMPCOR_REFINE_PAIRS(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
-    return false;
-}
-
-bool spec_refine_big_supported(int n, int f, int& smem)
-{
-    if (f != 2) return false;
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D)              \
-    if (n == NN) {                                      \
-        smem = BigUpsampleGeom<A, B, C, D>::smem;       \
-        return smem <= 227 * 1024;                      \
-    }
-    AMPCOR_REFINE_BIG(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
-    return false;
-}
-
-cudaError_t launch_spec_refine(int n, unsigned blocks, cudaStream_t st, const float2* base,
-                               const long long* off, long long stride, const CoarseOut* coarse,
-                               long long pair0, long long pairs, const long long* valid,
-                               const float2* twn, const float2* twf, float* refined,
-                               long long refined_stride, long long out_off, int deramp,
-                               float2* ybuf, bool strips)
-{
-    int small_smem = 0;
-    if ((strips || !spec_refine_supported(n, 2, small_smem)) && ybuf) {
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D)                                                              \
-        if (n == NN) {                                                                                  \
-            if (deramp)                                                                                 \
-                spec_refine_big_kernel<A, B, C, D, true><<<blocks, kThreads, BigUpsampleGeom<A, B, C, D>::smem, st>>>( \
-                    base, off, stride, coarse, pair0, pairs, valid, twn, twf, ybuf, refined, refined_stride, out_off); \
-            else                                                                                        \
-                spec_refine_big_kernel<A, B, C, D, false><<<blocks, kThreads, BigUpsampleGeom<A, B, C, D>::smem, st>>>( \
-                    base, off, stride, coarse, pair0, pairs, valid, twn, twf, ybuf, refined, refined_stride, out_off); \
-            return cudaGetLastError();                                                                  \
-        }
-        AMPCOR_REFINE_BIG(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
-        return cudaErrorInvalidValue;
-    }
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D)                                                           \
-    if (n == NN) {                                                                                   \
-        constexpr int smem = UpsampleGeom<A, B, C, D>::smem;                                         \
-        if (deramp)                                                                                  \
-            spec_refine_kernel<A, B, C, D, true><<<blocks, kThreads, smem, st>>>(                    \
-                base, off, stride, coarse, pair0, pairs, valid, twn, twf, refined, refined_stride, out_off); \
-        else                                                                                         \
-            spec_refine_kernel<A, B, C, D, false><<<blocks, kThreads, smem, st>>>(                   \
-                base, off, stride, coarse, pair0, pairs, valid, twn, twf, refined, refined_stride, out_off); \
-        return cudaGetLastError();                                                                   \
-    }
-    AMPCOR_REFINE_PAIRS(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
-    return cudaErrorInvalidValue;
-}
-
-bool spec_refine_staged_supported(int n, int f, int& smem, int& box_x)
-{
-    smem = box_x = 0;
-    if (f != 2) return false;
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D)                        \
-    if (n == NN) {                                                \
-        smem = UpsampleGeom<A, B, C, D>::smem_staged;             \
-        box_x = UpsampleGeom<A, B, C, D>::SWS;                    \
-        return smem <= 227 * 1024 && box_x <= 256;                \
-    }
-    AMPCOR_REFINE_PAIRS(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
-    return false;
-}
-
-cudaError_t launch_spec_refine_staged(int n, unsigned sms, cudaStream_t st, const CUtensorMap* tmap,
-                                      const long long* off, long long stride, const CoarseOut* coarse,
-                                      long long pair0, long long pairs, const long long* valid,
-                                      const float2* twn, const float2* twf, float* refined,
-                                      long long refined_stride, long long out_off, unsigned int* errs)
-{
-    if (pairs <= 0) return cudaSuccess;
-    const unsigned blocks = (unsigned)std::min<long long>(pairs, std::max(1u, sms));
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D)                                                           \
-    if (n == NN) {                                                                                   \
-        spec_refine_staged_kernel<A, B, C, D><<<blocks, kThreads, UpsampleGeom<A, B, C, D>::smem_staged, st>>>( \
-            *tmap, off, stride, coarse, pair0, pairs, valid, twn, twf, refined, refined_stride, out_off, errs); \
-        return cudaGetLastError();                                                                   \
-    }
-    AMPCOR_REFINE_PAIRS(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
-    return cudaErrorInvalidValue;
-}
-
 cudaError_t spec_set_smem_limits()
 {
     const int limit = 227 * 1024;
     cudaError_t e = cudaFuncSetAttribute(box_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D) \
-    if (e == cudaSuccess)                  \
-        e = cudaFuncSetAttribute(spec_refine_kernel<A, B, C, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
-    if (e == cudaSuccess)                  \
-        e = cudaFuncSetAttribute(spec_refine_kernel<A, B, C, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
-    if (e == cudaSuccess && UpsampleGeom<A, B, C, D>::smem_staged <= limit) \
-        e = cudaFuncSetAttribute(spec_refine_staged_kernel<A, B, C, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
-    AMPCOR_REFINE_PAIRS(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
 #define AMPCOR_SPEC_CASE(NN, A, B) \
     if (e == cudaSuccess)          \
         e = cudaFuncSetAttribute(spec_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
@@ -2009,13 +1424,6 @@ cudaError_t spec_set_smem_limits()
         e = cudaFuncSetAttribute(spec_block_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     AMPCOR_SPEC_LENGTHS(AMPCOR_SPEC_CASE)
 #undef AMPCOR_SPEC_CASE
-#define AMPCOR_REFINE_CASE(NN, A, B, C, D) \
-    if (e == cudaSuccess)                  \
-        e = cudaFuncSetAttribute(spec_refine_big_kernel<A, B, C, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
-    if (e == cudaSuccess)                  \
-        e = cudaFuncSetAttribute(spec_refine_big_kernel<A, B, C, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
-    AMPCOR_REFINE_BIG(AMPCOR_REFINE_CASE)
-#undef AMPCOR_REFINE_CASE
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(spec_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     if (e == cudaSuccess)

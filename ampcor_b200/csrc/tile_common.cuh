@@ -184,13 +184,14 @@ __device__ __forceinline__ void window_stats(const float* win, const NccGeom& g,
 // phi_l = arg sum z(y + 1, x) conj z(y, x) (lag-one autocorrelations along samples and lines,
 // whose phases are the ramp's steps), then z(y, x) *= exp(-i (phi_s x + phi_l y)).  A Doppler
 // ramp moves the tile's spectrum off baseband, where the zero padding of a band-limited
-// interpolation would cut through it.  One block of kThreads threads; red holds 4 kWarps
+// interpolation would cut through it.  One block of NT threads; red holds 4 NT / 32
 // doubles; ends with a barrier.
+template <int NT = kThreads>
 __device__ inline void deramp_tile(float2* t, int stride, int n, double* red)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float sr = 0.0f, si = 0.0f, lr = 0.0f, li = 0.0f;
-    for (int k = tid; k < n * n; k += kThreads) {
+    for (int k = tid; k < n * n; k += NT) {
         const int y = k / n, x = k - y * n;
         const float2 z = t[y * stride + x];
         if (x + 1 < n) {
@@ -212,12 +213,12 @@ __device__ inline void deramp_tile(float2* t, int stride, int n, double* red)
         for (int k = 0; k < 4; ++k) red[4 * warp + k] = v[k];
     __syncthreads();
     double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int w = 0; w < kWarps; ++w)
+    for (int w = 0; w < NT / 32; ++w)
 #pragma unroll
         for (int k = 0; k < 4; ++k) a[k] += red[4 * w + k];
     const float ps = (float)atan2(a[1], a[0]), pl = (float)atan2(a[3], a[2]);
     __syncthreads();
-    for (int k = tid; k < n * n; k += kThreads) {
+    for (int k = tid; k < n * n; k += NT) {
         const int y = k / n, x = k - y * n;
         float s, c;
         sincosf(fmaf(ps, (float)x, pl * (float)y), &s, &c);
@@ -232,14 +233,14 @@ __device__ inline void deramp_tile(float2* t, int stride, int n, double* red)
 // when DERAMP.  Band-limited upsampling keeps a constant as it is, so a caller that takes the
 // mean off the tile before its transforms and adds it back to every output gets the same
 // interpolation, with the transforms rounding on the tile's variation instead of on a strong
-// steady return.  FP32 sums per thread, FP64 across the block.  red: 2 kWarps doubles; ends with
+// steady return.  FP32 sums per thread, FP64 across the block.  red: 2 NT / 32 doubles; ends with
 // a barrier.
-template <bool GLOBAL, bool DERAMP>
+template <bool GLOBAL, bool DERAMP, int NT = kThreads>
 __device__ inline float2 tile_mean(const float2* t, long long stride, int n, float ps, float pl, double* red)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float sx = 0.0f, sy = 0.0f;
-    for (int k = tid; k < n * n; k += kThreads) {
+    for (int k = tid; k < n * n; k += NT) {
         const int y = k / n, x = k - y * n;
         float2 z = GLOBAL ? __ldg(t + y * stride + x) : t[y * stride + x];
         if (DERAMP) {
@@ -258,7 +259,7 @@ __device__ inline float2 tile_mean(const float2* t, long long stride, int n, flo
     __syncthreads();
     a = 0.0;
     b = 0.0;
-    for (int w = 0; w < kWarps; ++w) {
+    for (int w = 0; w < NT / 32; ++w) {
         a += red[2 * w];
         b += red[2 * w + 1];
     }
