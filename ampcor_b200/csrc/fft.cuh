@@ -111,8 +111,32 @@ HD float tw_sin(int i)
 
 // ---- complex helpers ----------------------------------------------------------------------
 
-HD float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-HD float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// On the device both parts go in one packed instruction (the same roundings; the refinement of
+// 7,400 tiles of 80, 64 and 48 samples: 508, 282, 166 -> 493, 269, 159 us).
+HD float2 cadd(float2 a, float2 b)
+{
+#ifdef __CUDA_ARCH__
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(r)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return *reinterpret_cast<float2*>(&r);
+#else
+    return make_float2(a.x + b.x, a.y + b.y);
+#endif
+}
+HD float2 csub(float2 a, float2 b)
+{
+#ifdef __CUDA_ARCH__
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;"
+        : "=l"(r)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return *reinterpret_cast<float2*>(&r);
+#else
+    return make_float2(a.x - b.x, a.y - b.y);
+#endif
+}
 HD float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 // a * conj(b)
 HD float2 cmulc(float2 a, float2 b) { return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y); }

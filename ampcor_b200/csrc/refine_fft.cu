@@ -180,9 +180,9 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
     X(24, 3, 8, 96, 24, 8)       \
     X(32, 4, 8, 128, 32, 6)      \
     X(40, 5, 8, 160, 40, 5)      \
-    X(48, 3, 16, 256, 48, 4)     \
-    X(64, 4, 16, 256, 64, 3)     \
-    X(80, 5, 16, 256, 80, 2)     \
+    X(48, 3, 16, 192, 48, 5)     \
+    X(64, 4, 16, 256, 32, 4)     \
+    X(80, 5, 16, 256, 32, 3)     \
     X(96, 6, 16, 256, 32, 2)     \
     X(120, 8, 15, 480, 60, 1)    \
     X(128, 8, 16, 512, 64, 1)    \
