@@ -267,10 +267,14 @@ bool plan_spec(int R, int W, SpecGeom& g, std::string& err)
 // not a multiple of 4) get 3 + W floats rounded up to 16 bytes.
 constexpr int kStagePieces = 5;  // spec_staged_kernel's PJ
 
-bool plan_spec_staged(int R, int W, bool dense, SpecGeom& g)
+// `threads` to a CTA (a multiple of 32, at least W).
+bool plan_spec_staged(int R, int W, bool dense, int threads, SpecGeom& g)
 {
     std::string e;
     if (!plan_spec(R, W, g, e)) return false;
+    const int warps = threads / 32;
+    g.threads = threads;
+    g.ctas = 1;
     auto up = [](long x, long a) { return (x + a - 1) / a * a; };
     const int N = g.N, C = g.C;
     const long row = (long)g.RS * 8, tile = (long)N * row;
@@ -280,10 +284,10 @@ bool plan_spec_staged(int R, int W, bool dense, SpecGeom& g)
     const long kept = (long)(C + np <= N ? C + np : C) * row;
     const long S = up(std::max(kept, tile - stage), 128);
     if (2L * C * W * 4 > S) return false;
-    const int y0 = (int)std::min<long>(N, S / row) / kSpecWarps * kSpecWarps;
-    const int JN = (N + kSpecWarps - 1) / kSpecWarps;
+    const int y0 = (int)std::min<long>(N, S / row) / warps * warps;
+    const int JN = (N + warps - 1) / warps;
     for (int j0 = 0; j0 < JN; j0 += kStagePieces) {
-        const long y1 = (long)std::min(j0 + kStagePieces, JN) * kSpecWarps;
+        const long y1 = (long)std::min(j0 + kStagePieces, JN) * warps;
         if (y1 <= y0 || y1 >= W) continue;
         if (y1 * row > S + y1 * g.stage_rs * 4) return false;
     }
@@ -303,7 +307,7 @@ bool plan_spec_staged(int R, int W, bool dense, SpecGeom& g)
     off = up(off + (long)C * C * 4, 16);
     g.off_gam = (int)off;  // the surface; before the last step, the statistics' partial sums
     const long limit = 227L * 1024 - 32;
-    g.nseg = std::max(1, kSpecThreads / W);
+    g.nseg = std::max(1, threads / W);
     while (g.nseg > 1 && off + 32L * g.nseg * W > limit) --g.nseg;
     off = up(off + std::max<long>((long)C * C * 4, 32L * g.nseg * W), 128);
     // raster statistics as the copy engine brings them (rows from the window's 16-byte boundary)
@@ -314,6 +318,24 @@ bool plan_spec_staged(int R, int W, bool dense, SpecGeom& g)
     off += 32;  // the copy's mbarrier, the wait-failure flag, the failure-detection test's mbarrier
     g.smem_staged = off <= 227L * 1024 ? (int)off : 0;
     return g.smem_staged > 0;
+}
+
+// The staged form with several CTAs to an SM, for short transforms.  A 64-sample tile takes 33 KB
+// and has one task per thread and pass for a CTA of 512 threads, so that such a CTA mostly waits at
+// barriers; CTAs of 128 to 256 threads side by side fill each other's waits.  Measured on B200,
+// 23,625 pairs: 64-sample coarse stage 1,667 us with one CTA of 512 threads, 1,111 with 3 x 256
+// (1,151 with 4 x 192, 1,235 with 4 x 128); 96-sample fine stage 2,847, 2,076 with 2 x 192 (2,149
+// with 2 x 256, 2,161 with 2 x 384); 24,000 pairs of 48 and 80 samples: 1,506 -> 719 with 4 x 192,
+// 2,684 -> 1,925 with 2 x 256 (3 x 160: 2,369).  The rule
+// looks at the geometry alone: a pair's sums then take the same order in every chunk (a chunk of at
+// most one pair per multiprocessor would be done 3 us sooner by CTAs of 512 threads).
+bool plan_spec_shared(int R, int W, bool dense, SpecGeom& g)
+{
+    const int n = spec_next_length(W);
+    int threads = 0, ctas = 0;
+    if (!spec_shared(n, threads, ctas) || !plan_spec_staged(R, W, dense, threads, g)) return false;
+    g.ctas = (int)std::min<long>(ctas, 228L * 1024 / (g.smem_staged + 1024));
+    return g.ctas > 1;
 }
 
 // A stage of the spectral form whose window is too large for one tile: the chip splits into nb x nb
@@ -1194,10 +1216,13 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         // pair are dense rows of one buffer, staged whole when its rows are 16-byte multiples
         const char* stg = std::getenv("AMPCOR_STAGED");
         const bool staged_on = !(stg && std::strcmp(stg, "0") == 0);
-        h->coarse_staged = staged_on && direct_c && plan_spec_staged(h->R, h->W, false, h->spc_st);
+        h->coarse_staged = staged_on && direct_c && plan_spec_staged(h->R, h->W, false, kSpecThreads, h->spc_st);
         h->fine_staged = staged_on && direct_f &&
-                         plan_spec_staged(h->Rf, h->Wf, h->Rf % 2 == 0 && h->Wf % 2 == 0, h->spf_st) &&
+                         plan_spec_staged(h->Rf, h->Wf, h->Rf % 2 == 0 && h->Wf % 2 == 0, kSpecThreads, h->spf_st) &&
                          h->spf_st.stage_rs == h->Wf;
+        SpecGeom several;
+        if (h->coarse_staged && plan_spec_shared(h->R, h->W, false, several)) h->spc_st = several;
+        if (h->fine_staged && plan_spec_shared(h->Rf, h->Wf, true, several)) h->spf_st = several;
         const bool fine_ok = coarse_ok && (direct_f || plan_spec_blocked(h->Rf, h->Wf, h->bf, serr));
         h->spectral_ok = fine_ok && (h->refine_fft || interp_ok);
         if (direct_c || !h->spectral_ok) h->bc = SpecBlocks{};

@@ -223,10 +223,11 @@ struct SpecGeom {
     // window's W rows of stage_rs floats at off_stage (over the tile's last rows), the copy's
     // mbarrier at off_bar (and the CTA's wait-failure flag right after it);
     // tile rows below stage_y0 are written straight from the staged copy, the rows from stage_y0 on
-    // in groups of stage_pj x 16 rows read whole before they are written
+    // in groups of stage_pj rows a warp read whole before they are written
     int off_stage, off_bar, stage_y0, stage_pj, stage_rs;
     int off_inv_raw, inv_rs;  // raster statistics as copied: C rows of inv_rs floats
     int smem_staged;  // 0: no staged form for this stage
+    int threads, ctas;  // of a CTA, and resident CTAs per SM
 };
 
 // float amplitude tiles of chunk-local pair b (global pair pair0 + b): at base + off[pair0 + b]
@@ -316,7 +317,9 @@ cudaError_t launch_spec_reduce(const SpecGeom& full, int K, unsigned blocks, cud
 cudaError_t launch_spec(const SpecGeom& g, unsigned blocks, cudaStream_t st, SpecSource src,
                         long long pair0, long long pairs, const long long* valid, InvSource inv,
                         const float2* tw, SpecOut out);
-// the staged form: min(pairs, sms) resident CTAs walk the chunk; a bounded wait that runs out is
+// threads and CTAs per SM of the staged kernel where its tile leaves room for two CTAs or more
+bool spec_shared(int n, int& threads, int& ctas);
+// the staged form: g.ctas resident CTAs per SM walk the chunk; a bounded wait that runs out is
 // counted in errs.  Refined tiles: wmap and cmap null, no statistics given.  Raster windows:
 // wmap, cmap and imap 2-D maps of the secondary and reference amplitude rasters and of the
 // secondary's box statistics (inv) with boxes of stage_rs x W, (R + 6 & ~3) x R and inv_rs x C

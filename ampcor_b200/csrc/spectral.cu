@@ -617,17 +617,18 @@ __device__ __forceinline__ void tensor_prefetch_l2(const CUtensorMap* map, int x
 // box of wmap (stage_rs x W floats) whose first column is the 16-byte boundary at or before the
 // window's first sample, with the box of the raster's statistics (imap, inv_rs x C floats) at the
 // same corner, the chip's box of cmap sent toward L2
-template <int N1, int N2, bool RASTER>
-__global__ void __launch_bounds__(kSpecThreads, 1)
+template <int N1, int N2, bool RASTER, int NT, int CTAS>
+__global__ void __launch_bounds__(NT, CTAS)
 spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
                    InvSource inv, const float2* tw_g, SpecOut out, unsigned int* errs,
                    const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap cmap,
                    const __grid_constant__ CUtensorMap imap, int stall)
 {
     extern __shared__ __align__(16) unsigned char ssm[];
+    constexpr int NW = NT / 32;
     constexpr int N = N1 * N2;
     constexpr int RS = N + 1;
-    constexpr int JN = (N + kSpecWarps - 1) / kSpecWarps, IN = (N + 31) / 32;
+    constexpr int JN = (N + NW - 1) / NW, IN = (N + 31) / 32;
     constexpr int PJ = 5;  // row groups of a piece read whole before it is written
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int W = g.W, R = g.R, C = g.C, SW = g.stage_rs;
@@ -644,9 +645,9 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
     uint64_t* bar = reinterpret_cast<uint64_t*>(ssm + g.off_bar);
     int& s_err = *reinterpret_cast<int*>(ssm + g.off_bar + 8);  // a wait ran out (CTA-wide)
     const long long cs = src.chip_stride, ws = src.win_stride;
-    const int jA = g.stage_y0 / kSpecWarps;
+    const int jA = g.stage_y0 / NW;
 
-    for (int k = tid; k < N; k += kSpecThreads) {
+    for (int k = tid; k < N; k += NT) {
         tw[k] = __ldg(tw_g + k);
         neg[k] = fft::neg_pos<N1, N2>(k);
     }
@@ -735,7 +736,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             for (int j = 0; j < JN; ++j)
 #pragma unroll
                 for (int i = 0; i < IN; ++i) {
-                    const int y = warp + kSpecWarps * j, x = lane + 32 * i;
+                    const int y = warp + NW * j, x = lane + 32 * i;
                     cr[j][i] = y < R && x < R ? __ldg(chip + y * cs + x) : 0.0f;
                 }
         };
@@ -743,7 +744,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         if constexpr (RASTER) {
             load_chip();
             // the raster's placement statistics, copied with the window, into their C x C layout
-            for (int u = warp; u < C; u += kSpecWarps)
+            for (int u = warp; u < C; u += NW)
                 for (int v = lane; v < C; v += 32) invs[u * C + v] = inv_raw[u * g.inv_rs + xo + v];
             // the chip's FP64 mean (spec_kernel's first sweep)
             double c1 = 0.0;
@@ -755,7 +756,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             if (lane == 0) red[warp] = c1;
             __syncthreads();
             double t1 = 0.0;
-            for (int w = 0; w < kSpecWarps; ++w) t1 += red[w];
+            for (int w = 0; w < NW; ++w) t1 += red[w];
             mean_c = t1 / ((double)R * (double)R);
             __syncthreads();
         }
@@ -777,7 +778,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             const float4* s4 = reinterpret_cast<const float4*>(stage);
             const int n4 = (W * W) >> 2;
 #pragma unroll 4
-            for (int k = tid; k < n4; k += kSpecThreads) {
+            for (int k = tid; k < n4; k += NT) {
                 const float4 v = s4[k];
                 const float t[4] = {v.x - pk, v.y - pk, v.z - pk, v.w - pk};
 #pragma unroll
@@ -788,7 +789,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             }
             wsum[0] = sw;
             wsum[1] = sw2;
-            block_sum2<kSpecWarps>(wsum[0], wsum[1], red);
+            block_sum2<NW>(wsum[0], wsum[1], red);
         }
         const double cells_c = (double)R * (double)R, cells_w = (double)W * (double)W;
         double mean_w = (double)pk + wsum[0] / cells_w;
@@ -800,7 +801,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         if constexpr (!RASTER) {
             double* part = reinterpret_cast<double*>(ssm + g.off_gam);
             const StatSlots vs{Zf, reinterpret_cast<float*>(part + 4 * g.nseg * W), g.off_stage / 4, 1};
-            spec_box_stats<kSpecThreads>(wat, g, sx, vs, part, invs);
+            spec_box_stats<NT>(wat, g, sx, vs, part, invs);
         }
 
         // window (real parts) and chip (imaginary parts; its bytes were sent toward L2 with the
@@ -814,7 +815,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         double c1 = 0.0, c2 = 0.0;
         float sw = 0.0f, sw2 = 0.0f, sc2 = 0.0f;
         auto put = [&](int j, int i, float t) {
-            const int y = warp + kSpecWarps * j, x = lane + 32 * i;
+            const int y = warp + NW * j, x = lane + 32 * i;
             if (y < N && x < N) {
                 float c = cr[j][i];
                 if constexpr (RASTER) {
@@ -835,7 +836,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             }
         };
         auto staged = [&](int j, int i) {
-            const int y = warp + kSpecWarps * j, x = lane + 32 * i;
+            const int y = warp + NW * j, x = lane + 32 * i;
             return y < W && x < W ? wat(y, x) : 0.0f;
         };
         // rows below stage_y0 lie below the staged bytes: written as they are read
@@ -873,7 +874,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             }
             __syncthreads();
             ss = 0.0;
-            for (int w = 0; w < kSpecWarps; ++w) {
+            for (int w = 0; w < NW; ++w) {
                 ss += red[3 * w];
                 wsum[0] += red[3 * w + 1];
                 wsum[1] += red[3 * w + 2];
@@ -890,7 +891,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             }
             __syncthreads();
             double s1 = 0.0, s2 = 0.0;
-            for (int w = 0; w < kSpecWarps; ++w) {
+            for (int w = 0; w < NW; ++w) {
                 s1 += red[2 * w];
                 s2 += red[2 * w + 1];
             }
@@ -913,7 +914,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         int bi = INT_MAX;
         int flagged = 0;
         fft::correlate_tile<N1, N2, RASTER ? 2 : 0>(
-            Z, RS, W, C, tw, neg, half, centre, tid, kSpecThreads, BlockSync{},
+            Z, RS, W, C, tw, neg, half, centre, tid, NT, BlockSync{},
             [&](int u, int v, float2 val) {
                 if (v < C) {
                     const int idx = u * C + v;
@@ -938,7 +939,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
 
         float* surf = out.surfaces ? out.surfaces + (size_t)p * C * C : nullptr;
         float* gam = out.stage == 1 ? out.gam + b * C * C : nullptr;
-        spec_surface<kSpecThreads>(G, red, g, invs, inv_sigma, mean_c, ebox, chip, cs, win, ws, gam, surf, bv, bi,
+        spec_surface<NT>(G, red, g, invs, inv_sigma, mean_c, ebox, chip, cs, win, ws, gam, surf, bv, bi,
                                    flagged);
         if (tid == 0) spec_result(out, p, R, W, C, bv, bi);
     }
@@ -1409,6 +1410,31 @@ int spec_next_length(int w)
     return 0;
 }
 
+// CTAs of NT threads that the staged kernel runs side by side on an SM, for the tile lengths of
+// which two or more fit: N, N1, N2, NT, CTAS
+#define AMPCOR_SPEC_SHARED(X) \
+    X(16, 4, 4, 128, 6)       \
+    X(24, 4, 6, 128, 6)       \
+    X(32, 4, 8, 128, 6)       \
+    X(40, 5, 8, 128, 6)       \
+    X(48, 6, 8, 192, 4)       \
+    X(64, 8, 8, 256, 3)       \
+    X(80, 8, 10, 256, 2)      \
+    X(96, 8, 12, 192, 2)
+
+bool spec_shared(int n, int& threads, int& ctas)
+{
+#define AMPCOR_SPEC_CASE(NN, A, B, NT, CTAS) \
+    if (n == NN) {                           \
+        threads = NT;                        \
+        ctas = CTAS;                         \
+        return true;                         \
+    }
+    AMPCOR_SPEC_SHARED(AMPCOR_SPEC_CASE)
+#undef AMPCOR_SPEC_CASE
+    return false;
+}
+
 cudaError_t spec_set_smem_limits()
 {
     const int limit = 227 * 1024;
@@ -1417,12 +1443,19 @@ cudaError_t spec_set_smem_limits()
     if (e == cudaSuccess)          \
         e = cudaFuncSetAttribute(spec_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
     if (e == cudaSuccess)          \
-        e = cudaFuncSetAttribute(spec_staged_kernel<A, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
+        e = cudaFuncSetAttribute(spec_staged_kernel<A, B, true, kSpecThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
     if (e == cudaSuccess)          \
-        e = cudaFuncSetAttribute(spec_staged_kernel<A, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
+        e = cudaFuncSetAttribute(spec_staged_kernel<A, B, false, kSpecThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
     if (e == cudaSuccess)          \
         e = cudaFuncSetAttribute(spec_block_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     AMPCOR_SPEC_LENGTHS(AMPCOR_SPEC_CASE)
+#undef AMPCOR_SPEC_CASE
+#define AMPCOR_SPEC_CASE(NN, A, B, NT, CTAS) \
+    if (e == cudaSuccess)                    \
+        e = cudaFuncSetAttribute(spec_staged_kernel<A, B, true, NT, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
+    if (e == cudaSuccess)                    \
+        e = cudaFuncSetAttribute(spec_staged_kernel<A, B, false, NT, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    AMPCOR_SPEC_SHARED(AMPCOR_SPEC_CASE)
 #undef AMPCOR_SPEC_CASE
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(spec_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
@@ -1514,18 +1547,24 @@ cudaError_t launch_spec_staged(const SpecGeom& g, unsigned sms, cudaStream_t st,
                                const CUtensorMap* cmap, const CUtensorMap* imap, int stall)
 {
     if (pairs <= 0) return cudaSuccess;
-    const unsigned blocks = (unsigned)std::min<long long>(pairs, std::max(1u, sms));
-#define AMPCOR_SPEC_CASE(NN, A, B)                                                                      \
-    if (g.N == NN) {                                                                                    \
-        if (wmap)                                                                                       \
-            spec_staged_kernel<A, B, true><<<blocks, kSpecThreads, g.smem_staged, st>>>(                      \
-                src, pair0, pairs, valid, g, inv, tw, out, errs, *wmap, *cmap, *imap, stall);               \
-        else                                                                                            \
-            spec_staged_kernel<A, B, false><<<blocks, kSpecThreads, g.smem_staged, st>>>(                     \
-                src, pair0, pairs, valid, g, inv, tw, out, errs, CUtensorMap{}, CUtensorMap{}, CUtensorMap{},  \
-                stall);                                                                             \
-        return cudaGetLastError();                                                                      \
-    }
+    const unsigned blocks = (unsigned)std::min<long long>(pairs, std::max(1u, sms) * (long long)g.ctas);
+    auto run = [&](auto raster, auto dense) {
+        if (wmap)
+            raster<<<blocks, g.threads, g.smem_staged, st>>>(src, pair0, pairs, valid, g, inv, tw, out, errs, *wmap,
+                                                             *cmap, *imap, stall);
+        else
+            dense<<<blocks, g.threads, g.smem_staged, st>>>(src, pair0, pairs, valid, g, inv, tw, out, errs,
+                                                            CUtensorMap{}, CUtensorMap{}, CUtensorMap{}, stall);
+        return cudaGetLastError();
+    };
+#define AMPCOR_SPEC_CASE(NN, A, B, NT, CTAS) \
+    if (g.N == NN && g.threads == NT)        \
+        return run(spec_staged_kernel<A, B, true, NT, CTAS>, spec_staged_kernel<A, B, false, NT, CTAS>);
+    AMPCOR_SPEC_SHARED(AMPCOR_SPEC_CASE)
+#undef AMPCOR_SPEC_CASE
+#define AMPCOR_SPEC_CASE(NN, A, B) \
+    if (g.N == NN)                 \
+        return run(spec_staged_kernel<A, B, true, kSpecThreads, 1>, spec_staged_kernel<A, B, false, kSpecThreads, 1>);
     AMPCOR_SPEC_LENGTHS(AMPCOR_SPEC_CASE)
 #undef AMPCOR_SPEC_CASE
     return cudaErrorInvalidValue;
