@@ -283,7 +283,11 @@ bool plan_spec_staged(int R, int W, bool dense, int threads, SpecGeom& g)
     const int np = (C + 1) / 2;
     const long kept = (long)(C + np <= N ? C + np : C) * row;
     const long S = up(std::max(kept, tile - stage), 128);
-    if (2L * C * W * 4 > S) return false;
+    // refined windows: the statistics' column sums and partial sums below the staged bytes
+    g.nseg = std::max(1, 2 * threads / W);
+    auto scratch = [&](int nseg) { return up(2L * C * W * 4, 16) + 32L * nseg * W; };
+    while (dense && g.nseg > 1 && scratch(g.nseg) > S) --g.nseg;
+    if (dense && scratch(g.nseg) > S) return false;
     const int y0 = (int)std::min<long>(N, S / row) / warps * warps;
     const int JN = (N + warps - 1) / warps;
     for (int j0 = 0; j0 < JN; j0 += kStagePieces) {
@@ -305,11 +309,8 @@ bool plan_spec_staged(int R, int W, bool dense, int threads, SpecGeom& g)
     off += 4L * kSpecWarps * 8;
     g.off_inv = (int)off;
     off = up(off + (long)C * C * 4, 16);
-    g.off_gam = (int)off;  // the surface; before the last step, the statistics' partial sums
-    const long limit = 227L * 1024 - 32;
-    g.nseg = std::max(1, threads / W);
-    while (g.nseg > 1 && off + 32L * g.nseg * W > limit) --g.nseg;
-    off = up(off + std::max<long>((long)C * C * 4, 32L * g.nseg * W), 128);
+    g.off_gam = (int)off;  // the surface
+    off = up(off + (long)C * C * 4, 128);
     // raster statistics as the copy engine brings them (rows from the window's 16-byte boundary)
     g.inv_rs = (C + 6) & ~3;
     g.off_inv_raw = dense ? 0 : (int)off;
@@ -580,10 +581,11 @@ struct ampcor_handle {
     // refinement by FFT (spectral form): the tables of R, then of E (half_shift_table)
     bool refine_fft = false;
     float* d_tw_refine = nullptr;
-    // blocked spectral stages (coarse, fine): chip statistics, placement statistics, partial
-    // numerators and their scalars, all per chunk
+    // the statistics of a chunk's chips, refined chips and refined windows, chunk entries each
+    TileStat* d_tstat = nullptr;
+    // blocked spectral stages (coarse, fine): placement statistics, partial numerators and their
+    // scalars, all per chunk
     SpecBlocks bc{}, bf{};
-    ChipStat* d_cstat = nullptr;
     float* d_inv_blk = nullptr;
     float* d_part = nullptr;
     double* d_scal = nullptr;
@@ -697,13 +699,13 @@ void free_chunk_scratch(ampcor_handle* h)
     cudaFree(h->d_inv_c);
     cudaFree(h->d_inv_f);
     cudaFree(h->d_gam);
-    cudaFree(h->d_cstat);
+    cudaFree(h->d_tstat);
     cudaFree(h->d_inv_blk);
     cudaFree(h->d_part);
     cudaFree(h->d_scal);
     h->d_refined = nullptr;
     h->d_inv_c = h->d_inv_f = h->d_gam = nullptr;
-    h->d_cstat = nullptr;
+    h->d_tstat = nullptr;
     h->d_inv_blk = nullptr;
     h->d_part = nullptr;
     h->d_scal = nullptr;
@@ -738,13 +740,14 @@ int ensure_refined(ampcor_handle* h)
         return scratch_fail(h, "allocating placement statistics scratch");
     if (h->form != kFormPlain && cudaMalloc(&h->d_gam, n * h->Cf * h->Cf * sizeof(float)) != cudaSuccess)
         return scratch_fail(h, "allocating refined-surface scratch");
+    if (h->form == kFormSpectral && cudaMalloc(&h->d_tstat, 3 * n * sizeof(TileStat)) != cudaSuccess)
+        return scratch_fail(h, "allocating tile statistics");
     if (h->form == kFormSpectral && (h->bc.on || h->bf.on)) {
         const size_t K = (size_t)std::max(h->bc.on ? h->bc.K : 0, h->bf.on ? h->bf.K : 0);
         const size_t parts = std::max(h->bc.on ? (size_t)h->bc.K * h->C * h->C : 0,
                                       h->bf.on ? (size_t)h->bf.K * h->Cf * h->Cf : 0);
         const size_t cells = std::max(h->bc.on ? (size_t)h->C * h->C : 0, h->bf.on ? (size_t)h->Cf * h->Cf : 0);
-        if (cudaMalloc(&h->d_cstat, n * sizeof(ChipStat)) != cudaSuccess ||
-            cudaMalloc(&h->d_inv_blk, n * cells * sizeof(float)) != cudaSuccess ||
+        if (cudaMalloc(&h->d_inv_blk, n * cells * sizeof(float)) != cudaSuccess ||
             cudaMalloc(&h->d_part, n * parts * sizeof(float)) != cudaSuccess ||
             cudaMalloc(&h->d_scal, n * K * 2 * sizeof(double)) != cudaSuccess)
             return scratch_fail(h, "allocating blocked-correlation scratch");
@@ -1019,32 +1022,48 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         raster_map(imap, r.inv_c.base, r.rows, src.tgt_stride, h->spc_st.inv_rs, h->C);
     for (long long c0 = p0; c0 < p1; c0 += (long long)h->chunk) {
         const unsigned n = (unsigned)std::min<long long>((long long)h->chunk, p1 - c0);
+        TileStat* const st_raw = h->d_tstat;               // the chips
+        TileStat* const st_chip = st_raw + h->chunk;       // the refined chips
+        TileStat* const st_win = st_chip + h->chunk;       // the refined windows
+        const float2* tab = reinterpret_cast<const float2*>(h->d_tw_refine);
+        const bool deramp = (h->prm.flags & AMPCOR_FLAG_DERAMP) != 0;
+        // the chips' refinement needs no coarse result, and gives the coarse stage their statistics
         cudaEvent_t b = mark(h, st);
+        if (h->refine_fft) {
+            CK(h, launch_refine_half(h->R, n, st, src.ref_base, src.ref_off, src.ref_stride, nullptr, c0, n,
+                                     src.ref_off, tab, h->d_refined, h->refined_stride, 0, deramp, st_raw, st_chip),
+               "launching the chip refinement");
+            cudaEvent_t b1 = mark(h, st);
+            keep(h, 1, b, b1);
+            b = b1;
+        } else {
+            CK(h, launch_spec_chip_stats(n, st, cs, c0, n, src.ref_off, h->R, st_raw),
+               "launching the chip statistics");
+            cudaEvent_t b1 = mark(h, st);
+            keep(h, 3, b, b1);
+            b = b1;
+        }
         const SpecOut co{0, h->m, h->d_coarse, h->d_coarse_peak, nullptr, nullptr, coarse_surfaces};
         if (h->bc.on) {
             InvSource ic = r.inv_c;
-            CK(h, launch_spec_chip_stats(n, st, cs, c0, n, src.ref_off, h->R, h->d_cstat),
-               "launching the chip statistics");
-            int kernels = 1;
             if (!ic.base) {
                 CK(h, launch_spec_tile_stats(n, st, cs, c0, n, src.ref_off, h->R, h->W, h->d_inv_blk),
                    "launching the placement statistics");
                 ic = InvSource{h->d_inv_blk, nullptr, 0};
-                ++kernels;
+                cudaEvent_t b2 = mark(h, st);
+                keep(h, 3, b, b2);
+                b = b2;
             }
-            cudaEvent_t b2 = mark(h, st);
-            keep(h, 3, b, b2, kernels);
-            b = b2;
             CK(h, launch_spec_block(h->bc.tile, h->bc.nb, n * (unsigned)h->bc.K, st, cs, c0, n, src.ref_off,
-                                    h->d_cstat, reinterpret_cast<const float2*>(h->d_tw_c), h->d_part, h->d_scal),
+                                    st_raw, reinterpret_cast<const float2*>(h->d_tw_c), h->d_part, h->d_scal),
                "launching the blocked coarse correlation");
-            CK(h, launch_spec_reduce(h->bc.full, h->bc.K, n, st, cs, c0, n, src.ref_off, h->d_cstat, ic,
+            CK(h, launch_spec_reduce(h->bc.full, h->bc.K, n, st, cs, c0, n, src.ref_off, st_raw, ic,
                                      h->d_part, h->d_scal, co),
                "launching the coarse reduction");
         } else {
             if (coarse_st)
                 CK(h, launch_spec_staged(h->spc_st, (unsigned)h->sms, st, cs, c0, n, src.ref_off, r.inv_c,
-                                         reinterpret_cast<const float2*>(h->d_tw_c), co, h->d_tc_err,
+                                         reinterpret_cast<const float2*>(h->d_tw_c), co, st_raw, nullptr, h->d_tc_err,
                                          &wmap, &cmap, &imap, h->inject_timeouts > 0 ? 1 : 0),
                    "launching the staged coarse correlation");
             else
@@ -1055,14 +1074,9 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         cudaEvent_t c = mark(h, st);
         keep(h, 0, b, c, h->bc.on ? 2 : 1);
         if (h->refine_fft) {
-            const float2* tab = reinterpret_cast<const float2*>(h->d_tw_refine);
-            const bool deramp = (h->prm.flags & AMPCOR_FLAG_DERAMP) != 0;
-            CK(h, launch_refine_half(h->R, n, st, src.ref_base, src.ref_off, src.ref_stride, nullptr, c0, n,
-                                     src.ref_off, tab, h->d_refined, h->refined_stride, 0, deramp),
-               "launching the chip refinement");
             CK(h, launch_refine_half(h->E, n, st, src.tgt_base, src.tgt_off, src.tgt_stride, h->d_coarse, c0, n,
                                      src.ref_off, tab + 2 * h->R, h->d_refined, h->refined_stride,
-                                     (long long)h->Rf * h->Rf, deramp),
+                                     (long long)h->Rf * h->Rf, deramp, nullptr, st_win),
                "launching the window refinement");
         } else {
             refine_kernel<<<n, kThreads, h->refine_smem, st>>>(src, c0, n, h->d_coarse, h->ic, h->iw,
@@ -1071,27 +1085,35 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
             CK(h, cudaGetLastError(), "launching the refinement kernel");
         }
         cudaEvent_t e = mark(h, st);
-        keep(h, 1, c, e, h->refine_fft ? 2 : 1);
+        keep(h, 1, c, e);
+        if (!h->refine_fft) {
+            const SpecSource wins{fs.win, fs.win_stride, nullptr, fs.win_step, fs.win, fs.win_stride, nullptr, fs.win_step};
+            CK(h, launch_spec_chip_stats(n, st, fs, c0, n, src.ref_off, h->Rf, st_chip),
+               "launching the refined chip statistics");
+            CK(h, launch_spec_chip_stats(n, st, wins, c0, n, src.ref_off, h->Wf, st_win),
+               "launching the refined window statistics");
+            cudaEvent_t e1 = mark(h, st);
+            keep(h, 4, e, e1, 2);
+            e = e1;
+        }
         const SpecOut fo{1, 0, nullptr, nullptr, h->d_fine_out, h->d_gam, refined_surfaces};
         if (h->bf.on) {
-            CK(h, launch_spec_chip_stats(n, st, fs, c0, n, src.ref_off, h->Rf, h->d_cstat),
-               "launching the refined chip statistics");
             CK(h, launch_spec_tile_stats(n, st, fs, c0, n, src.ref_off, h->Rf, h->Wf, h->d_inv_blk),
                "launching the refined placement statistics");
             cudaEvent_t e2 = mark(h, st);
-            keep(h, 4, e, e2, 2);
+            keep(h, 4, e, e2);
             e = e2;
             CK(h, launch_spec_block(h->bf.tile, h->bf.nb, n * (unsigned)h->bf.K, st, fs, c0, n, src.ref_off,
-                                    h->d_cstat, reinterpret_cast<const float2*>(h->d_tw_f), h->d_part, h->d_scal),
+                                    st_chip, reinterpret_cast<const float2*>(h->d_tw_f), h->d_part, h->d_scal),
                "launching the blocked fine correlation");
-            CK(h, launch_spec_reduce(h->bf.full, h->bf.K, n, st, fs, c0, n, src.ref_off, h->d_cstat,
+            CK(h, launch_spec_reduce(h->bf.full, h->bf.K, n, st, fs, c0, n, src.ref_off, st_chip,
                                      InvSource{h->d_inv_blk, nullptr, 0}, h->d_part, h->d_scal, fo),
                "launching the fine reduction");
         } else {
             if (h->fine_staged)
                 CK(h, launch_spec_staged(h->spf_st, (unsigned)h->sms, st, fs, c0, n, src.ref_off,
                                          InvSource{nullptr, nullptr, 0},
-                                         reinterpret_cast<const float2*>(h->d_tw_f), fo, h->d_tc_err,
+                                         reinterpret_cast<const float2*>(h->d_tw_f), fo, st_chip, st_win, h->d_tc_err,
                                          nullptr, nullptr, nullptr, h->inject_timeouts > 0 ? 1 : 0),
                    "launching the staged fine correlation");
             else
@@ -1353,7 +1375,7 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_amp);
     cudaFree(h->d_vsum);
     cudaFree(h->d_inv_raster);
-    cudaFree(h->d_cstat);
+    cudaFree(h->d_tstat);
     cudaFree(h->d_inv_blk);
     cudaFree(h->d_part);
     cudaFree(h->d_scal);

@@ -214,9 +214,10 @@ struct SpecGeom {
     int RS;           // tile row stride (complex samples)
     int off_z, off_tw, off_neg, off_half, off_red, off_inv, off_gam;  // shared-memory byte offsets
     // placement statistics computed in the kernel (no InvSource given): nseg threads per window
-    // column, their FP64 partial sums (4 nseg W doubles) at off_gam (the surface buffer, idle
-    // until the last transform step), the column sums in the tile's imaginary parts and, past the
-    // tile, right after the partial sums
+    // column (staged form: per two columns), their FP64 partial sums (4 nseg W doubles) at off_gam
+    // (the surface buffer, idle until the last transform step), the column sums in the tile's
+    // imaginary parts and, past the tile, right after the partial sums; the staged form keeps both
+    // in the tile's first bytes
     int nseg;
     int smem_bytes;
     // staged form (spec_staged_kernel, windows copied in while the previous pair finishes): the
@@ -276,10 +277,12 @@ struct InvSource {
     long long stride;
 };
 
-// per-pair chip statistics of a blocked spectral stage: the chip's FP64 mean and 1/|r - mean|
-struct ChipStat {
+// FP64 statistics of an amplitude tile: its mean, 1/|t - mean| (0 for a tile flat to its own
+// rounding) and |t - mean|
+struct TileStat {
     double mean;
-    double inv_sigma;
+    double inv_norm;
+    double norm;
 };
 
 // the transform lengths that are compiled, with their radices
@@ -292,27 +295,29 @@ cudaError_t spec_set_smem_limits();
 // phases over N of the frequencies at the transform's positions.
 bool refine_half_radices(int n, int& n1, int& n2);
 cudaError_t refine_half_set_smem_limits();
+// Statistics of the tiles, one per chunk-local pair: raw (unless null) of the amplitudes as they are,
+// fine of the upsampled ones.
 cudaError_t launch_refine_half(int n, unsigned blocks, cudaStream_t st, const float2* base, const long long* off,
                                long long stride, const CoarseOut* coarse, long long pair0, long long pairs,
                                const long long* valid, const float2* tab, float* refined, long long refined_stride,
-                               long long out_off, bool deramp);
+                               long long out_off, bool deramp, TileStat* raw, TileStat* fine);
 
 // blocked spectral correlation (windows too large for one tile; see spectral.cu): per chunk of
 // pairs the chip statistics, the placement statistics when no raster gives them, the partial
 // numerators of every (pair, chip block) and their per-pair reduction to the stage's outputs
 cudaError_t launch_spec_chip_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                   long long pairs, const long long* valid, int R, ChipStat* out);
+                                   long long pairs, const long long* valid, int R, TileStat* out);
 int spec_tile_stats_rows(int W, int C, int& smem);
 cudaError_t launch_spec_tile_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
                                    long long pairs, const long long* valid, int R, int W, float* inv);
 cudaError_t launch_spec_block(const SpecGeom& tile, int nb, unsigned blocks, cudaStream_t st,
                               SpecSource src, long long pair0, long long pairs,
-                              const long long* valid, const ChipStat* cstat, const float2* tw,
+                              const long long* valid, const TileStat* cstat, const float2* tw,
                               float* part, double* scal);
 int spec_reduce_smem(int C);
 cudaError_t launch_spec_reduce(const SpecGeom& full, int K, unsigned blocks, cudaStream_t st,
                                SpecSource src, long long pair0, long long pairs,
-                               const long long* valid, const ChipStat* cstat, InvSource inv,
+                               const long long* valid, const TileStat* cstat, InvSource inv,
                                const float* part, const double* scal, SpecOut out);
 cudaError_t launch_spec(const SpecGeom& g, unsigned blocks, cudaStream_t st, SpecSource src,
                         long long pair0, long long pairs, const long long* valid, InvSource inv,
@@ -323,10 +328,12 @@ bool spec_shared(int n, int& threads, int& ctas);
 // counted in errs.  Refined tiles: wmap and cmap null, no statistics given.  Raster windows:
 // wmap, cmap and imap 2-D maps of the secondary and reference amplitude rasters and of the
 // secondary's box statistics (inv) with boxes of stage_rs x W, (R + 6 & ~3) x R and inv_rs x C
-// floats.  stall: the failure-detection test's wait on a barrier that nothing completes.
+// floats.  cstat (and wstat for refined tiles): the statistics of the chips (and windows).  stall:
+// the failure-detection test's wait on a barrier that nothing completes.
 cudaError_t launch_spec_staged(const SpecGeom& g, unsigned sms, cudaStream_t st, SpecSource src,
                                long long pair0, long long pairs, const long long* valid, InvSource inv,
-                               const float2* tw, SpecOut out, unsigned int* errs, const CUtensorMap* wmap,
+                               const float2* tw, SpecOut out, const TileStat* cstat, const TileStat* wstat,
+                               unsigned int* errs, const CUtensorMap* wmap,
                                const CUtensorMap* cmap, const CUtensorMap* imap, int stall);
 
 }  // namespace ampcor_b200

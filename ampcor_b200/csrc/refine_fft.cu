@@ -57,7 +57,7 @@ template <int N1, int N2, int NT, int SR, int CTAS, bool DERAMP>
 __global__ void __launch_bounds__(NT, CTAS)
 refine_half_kernel(const float2* base, const long long* off, long long stride, const CoarseOut* coarse,
                    long long pair0, long long pairs, const long long* valid, const float2* tab, float* refined,
-                   long long refined_stride, long long out_off)
+                   long long refined_stride, long long out_off, TileStat* raw, TileStat* fine)
 {
     using G = HalfGeom<N1, N2, NT, SR, CTAS>;
     constexpr int N = G::N, F = 2 * N, RS = G::RS;
@@ -123,6 +123,12 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
         mu = make_float2((float)(ta / ((double)N * N)), (float)(tb / ((double)N * N)));
     }
 
+    // The amplitudes' sums and sums of squares, of the tile itself (even) and of the rest: FP32 per
+    // thread about one of the tile's own amplitudes, FP64 from there on, so that a strong steady
+    // return costs no digits of their variance
+    const float pivot = amplitude(X[(tid % N) * RS + (7 * tid) % N]);
+    float e1 = 0.0f, e2 = 0.0f, r1 = 0.0f, r2 = 0.0f;
+    int lines = 0;  // tasks done: N1 outputs of each kind per task
     // Output rows 2 y + odd: row y of the tile (less m, with add back on: the tile as it was loaded
     // gives its own amplitudes exactly) and S of it, a strip at a time
     auto rows = [&](int odd, float2 m, float2 add) {
@@ -154,9 +160,21 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
                 float2* o = out + (long long)(2 * (r0 + y) + odd) * N;
                 fft::inv_a_store<N1, N2>(Y + y * RS, 1, n2, tw, [&](int n, float2 v) {
                     const float2 e = row[n];
-                    o[n] = make_float2(amplitude(make_float2(e.x + add.x, e.y + add.y)),
-                                       amplitude(make_float2(v.x + mu.x, v.y + mu.y)));
+                    const float2 z = make_float2(amplitude(make_float2(e.x + add.x, e.y + add.y)),
+                                                 amplitude(make_float2(v.x + mu.x, v.y + mu.y)));
+                    o[n] = z;
+                    const float de = z.x - pivot, dv = z.y - pivot;
+                    if (odd == 0) {
+                        e1 += de;
+                        e2 = fmaf(de, de, e2);
+                    } else {
+                        r1 += de;
+                        r2 = fmaf(de, de, r2);
+                    }
+                    r1 += dv;
+                    r2 = fmaf(dv, dv, r2);
                 });
+                ++lines;
             }
             __syncthreads();
         }
@@ -170,7 +188,27 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
     __syncthreads();
     for (int t = tid; t < N * N2; t += NT) fft::inv_a<N1, N2>(X + t % N, RS, t / N, tw);
     __syncthreads();
+    const int even = lines * N1;  // outputs of the tile itself, and as many beside them
     rows(1, zero, mu);
+    const double pv = pivot, ne = even, nr = lines * 2 * N1 - even;
+    double sum[4] = {ne * pv + (double)e1, (double)e2 + pv * (2.0 * (double)e1 + ne * pv),
+                     nr * pv + (double)r1, (double)r2 + pv * (2.0 * (double)r1 + nr * pv)};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        sum[q] = warp_sum(sum[q]);
+        if (lane == 0) red[4 * warp + q] = sum[q];
+    }
+    __syncthreads();
+    if (tid < 2) {
+        // thread 0: the tile itself, thread 1: all four phases
+        double s1 = 0.0, s2 = 0.0;
+        for (int w = 0; w < NT / 32; ++w) {
+            s1 += red[4 * w] + (tid ? red[4 * w + 2] : 0.0);
+            s2 += red[4 * w + 1] + (tid ? red[4 * w + 3] : 0.0);
+        }
+        TileStat* to = tid ? fine : raw;
+        if (to) to[blockIdx.x] = tile_stat(s1, s2, tid ? (double)F * F : (double)N * N);
+    }
 }
 
 // compiled tiles: N, N1, N2, threads, rows of a strip, CTAs per SM.  N2 = 16 where it divides: the
@@ -219,13 +257,14 @@ cudaError_t refine_half_set_smem_limits()
 cudaError_t launch_refine_half(int n, unsigned blocks, cudaStream_t st, const float2* base, const long long* off,
                                long long stride, const CoarseOut* coarse, long long pair0, long long pairs,
                                const long long* valid, const float2* tab, float* refined, long long refined_stride,
-                               long long out_off, bool deramp)
+                               long long out_off, bool deramp, TileStat* raw, TileStat* fine)
 {
 #define AMPCOR_REFINE_CASE(NN, A, B, NT, SR, CTAS)                                                             \
     if (n == NN) {                                                                                             \
         (deramp ? refine_half_kernel<A, B, NT, SR, CTAS, true> : refine_half_kernel<A, B, NT, SR, CTAS, false>) \
             <<<blocks, NT, HalfGeom<A, B, NT, SR, CTAS>::smem, st>>>(base, off, stride, coarse, pair0, pairs,  \
-                                                                     valid, tab, refined, refined_stride, out_off); \
+                                                                     valid, tab, refined, refined_stride, out_off, \
+                                                                     raw, fine);                              \
         return cudaGetLastError();                                                                             \
     }
     AMPCOR_REFINE_TILES(AMPCOR_REFINE_CASE)

@@ -306,6 +306,195 @@ __device__ void spec_box_stats(Win win, const SpecGeom& g, float sx, StatSlots v
     __syncthreads();
 }
 
+// two floats at a time
+using pair_t = unsigned long long;
+__device__ __forceinline__ pair_t pk_of(float x, float y)
+{
+    return (pair_t)__float_as_uint(x) | (pair_t)__float_as_uint(y) << 32;
+}
+__device__ __forceinline__ float pk_lo(pair_t v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float pk_hi(pair_t v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ pair_t pk_add(pair_t a, pair_t b)
+{
+    pair_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair_t pk_sub(pair_t a, pair_t b)
+{
+    pair_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair_t pk_fma(pair_t a, pair_t b, pair_t c)
+{
+    pair_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// spec_box_stats for a staged refined window (W dense floats a row, W a multiple of 4): the same sums
+// in the same precision, two columns to a thread in packed FP32, and the box sums' first warp sum
+// carries both moments at once (one half of the warp each).  V: 2 C W floats, part: 4 nseg W
+// doubles, both in the tile's first bytes.  @@MEAS4@@
+template <int NT>
+__device__ void staged_box_stats(const float* win, const SpecGeom& g, float sx, float* V, double* part, float* invs)
+{
+    const int R = g.R, W = g.W, C = g.C, nseg = g.nseg, D = C - 1, W2 = W >> 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int s = tid / W2, x = 2 * (tid - s * W2);
+    const pair_t* col = reinterpret_cast<const pair_t*>(win + x);
+    const pair_t msx = pk_of(-sx, -sx), m2sx = pk_of(-2.0f * sx, -2.0f * sx);
+    const int d0 = s * D / nseg, d1 = (s + 1) * D / nseg;
+    constexpr int kRun = 8, kA = 4;
+    if (s < nseg) {
+        double b1x = 0.0, b1y = 0.0, b2x = 0.0, b2y = 0.0;
+        for (int y0 = s * R / nseg, y1 = (s + 1) * R / nseg; y0 < y1; y0 += kRun) {
+            pair_t r1 = 0, r2 = 0;
+#pragma unroll
+            for (int k = 0; k < kRun; ++k)
+                if (y0 + k < y1) {
+                    const pair_t t = pk_add(col[(y0 + k) * W2], msx);
+                    r1 = pk_add(r1, t);
+                    r2 = pk_fma(t, t, r2);
+                }
+            b1x += (double)pk_lo(r1);
+            b1y += (double)pk_hi(r1);
+            b2x += (double)pk_lo(r2);
+            b2y += (double)pk_hi(r2);
+        }
+        pair_t e1 = 0, e2 = 0;
+        for (int i0 = d0; i0 < d1; i0 += kA) {
+            pair_t a[kA], b[kA];
+#pragma unroll
+            for (int k = 0; k < kA; ++k) {
+                const int i = min(i0 + k, d1 - 1);
+                a[k] = col[(i + R) * W2];
+                b[k] = col[i * W2];
+            }
+#pragma unroll
+            for (int k = 0; k < kA; ++k)
+                if (i0 + k < d1) {
+                    const pair_t d = pk_sub(a[k], b[k]);
+                    e1 = pk_add(e1, d);
+                    e2 = pk_fma(d, pk_add(pk_add(a[k], b[k]), m2sx), e2);
+                }
+        }
+        double2* out = reinterpret_cast<double2*>(part + s * W + x);
+        out[0 * nseg * W2] = make_double2(b1x, b1y);
+        out[1 * nseg * W2] = make_double2(b2x, b2y);
+        out[2 * nseg * W2] = make_double2((double)pk_lo(e1), (double)pk_hi(e1));
+        out[3 * nseg * W2] = make_double2((double)pk_lo(e2), (double)pk_hi(e2));
+    }
+    __syncthreads();
+    if (s < nseg) {
+        double v1x = 0.0, v1y = 0.0, v2x = 0.0, v2y = 0.0;
+        auto take = [&](int q, int k) {
+            const double2 p1 = *reinterpret_cast<const double2*>(part + (q * nseg + k) * W + x);
+            const double2 p2 = *reinterpret_cast<const double2*>(part + ((q + 1) * nseg + k) * W + x);
+            v1x += p1.x;
+            v1y += p1.y;
+            v2x += p2.x;
+            v2y += p2.y;
+        };
+        for (int k = 0; k < nseg; ++k) take(0, k);
+        for (int k = 0; k < s; ++k) take(2, k);
+        const float h1x = (float)v1x, h1y = (float)v1y, h2x = (float)v2x, h2y = (float)v2y;
+        const pair_t h1 = pk_of(h1x, h1y), l1 = pk_of((float)(v1x - (double)h1x), (float)(v1y - (double)h1y));
+        const pair_t h2 = pk_of(h2x, h2y), l2 = pk_of((float)(v2x - (double)h2x), (float)(v2y - (double)h2y));
+        pair_t p1 = 0, p2 = 0;
+        pair_t* o1 = reinterpret_cast<pair_t*>(V + x);
+        pair_t* o2 = reinterpret_cast<pair_t*>(V + C * W + x);
+        for (int i0 = d0; i0 < d1; i0 += kA) {
+            pair_t a[kA], b[kA];
+#pragma unroll
+            for (int k = 0; k < kA; ++k) {
+                const int i = min(i0 + k, d1 - 1);
+                a[k] = col[(i + R) * W2];
+                b[k] = col[i * W2];
+            }
+#pragma unroll
+            for (int k = 0; k < kA; ++k)
+                if (i0 + k < d1) {
+                    o1[(i0 + k) * W2] = pk_add(h1, pk_add(l1, p1));
+                    o2[(i0 + k) * W2] = pk_add(h2, pk_add(l2, p2));
+                    const pair_t d = pk_sub(a[k], b[k]);
+                    p1 = pk_add(p1, d);
+                    p2 = pk_fma(d, pk_add(pk_add(a[k], b[k]), m2sx), p2);
+                }
+        }
+        if (s == nseg - 1) {
+            o1[D * W2] = pk_add(h1, pk_add(l1, p1));
+            o2[D * W2] = pk_add(h2, pk_add(l2, p2));
+        }
+    }
+    __syncthreads();
+    const double rcells = 1.0 / ((double)R * (double)R);
+    constexpr int NW = NT / 32, KR = 3;
+    for (int u0 = warp; u0 < C; u0 += KR * NW) {
+        const float* row1[KR];
+        float* to[KR];
+        bool keep[KR];
+        double m[KR];  // lanes below 16: the first box's sum, the others: its sum of squares
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+            const int u = min(u0 + r * NW, C - 1);
+            row1[r] = V + u * W;
+            to[r] = invs + u * C;
+            keep[r] = u0 + r * NW < C;
+            float f1 = 0.0f, f2 = 0.0f;
+            for (int c = lane; c < R; c += 32) {
+                f1 += row1[r][c];
+                f2 += row1[r][C * W + c];
+            }
+            const double mine = lane < 16 ? f1 : f2, other = lane < 16 ? f2 : f1;
+            m[r] = mine + __shfl_xor_sync(kFull, other, 16);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int r = 0; r < KR; ++r) m[r] += __shfl_xor_sync(kFull, m[r], o);
+        double s1[KR], s2[KR];
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+            s1[r] = __shfl_sync(kFull, m[r], 0);
+            s2[r] = __shfl_sync(kFull, m[r], 16);
+            if (lane == 0 && keep[r]) to[r][0] = box_inv_of(s1[r], s2[r], rcells);
+        }
+        for (int j0 = 0; j0 < D; j0 += 32) {
+            const int j = j0 + lane;
+            float i1[KR], i2[KR];
+#pragma unroll
+            for (int r = 0; r < KR; ++r) {
+                i1[r] = j < D ? row1[r][j + R] - row1[r][j] : 0.0f;
+                i2[r] = j < D ? row1[r][C * W + j + R] - row1[r][C * W + j] : 0.0f;
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+                for (int r = 0; r < KR; ++r) {
+                    const float y1 = __shfl_up_sync(kFull, i1[r], o);
+                    const float y2 = __shfl_up_sync(kFull, i2[r], o);
+                    if (lane >= o) {
+                        i1[r] += y1;
+                        i2[r] += y2;
+                    }
+                }
+#pragma unroll
+            for (int r = 0; r < KR; ++r)
+                if (j < D && keep[r])
+                    to[r][j + 1] = box_inv_of(s1[r] + (double)i1[r], s2[r] + (double)i2[r], rcells);
+            if (j0 + 32 < D)
+#pragma unroll
+                for (int r = 0; r < KR; ++r) {
+                    s1[r] += (double)__shfl_sync(kFull, i1[r], 31);
+                    s2[r] += (double)__shfl_sync(kFull, i2[r], 31);
+                }
+        }
+    }
+    __syncthreads();
+}
+
 // The normalised surface G (C x C in shared memory, formed by the last transform step) -> its
 // first maximum (valid in every thread) and optional copies; a CTA of NT threads, red holding
 // NT / 32 floats and as many ints.  On entry every thread holds the
@@ -568,12 +757,13 @@ spec_kernel(SpecSource src, long long pair0, long long pairs, const long long* v
 // blockIdx.x + gridDim.x, ...: once a pair's inverse column pass is done (from then on its
 // correlation touches only the tile's first rows) the bulk-copy engine brings the next pair's
 // window (W x W dense floats, one cp.async.bulk completing on an mbarrier) into the tile's last
-// bytes, and the chip's bytes are sent toward L2.  A pair then starts with its window in shared
-// memory: the window's sums and placement statistics read from the staged copy (the tile's first
-// bytes are the statistics' scratch), then one pass that writes the window and the chip (loaded
-// from L2 meanwhile) into the tile and takes the chip's FP64 sums; the first transform pass takes
-// both means off.  The numerics are spec_kernel's.  Every wait is bounded; one that
-// runs out is counted in errs, the CTA lets the copy in flight land (again bounded) and returns.
+// bytes, and the chip's bytes are sent toward L2.  The statistics of the chips and of the refined
+// windows come from the refinement, which forms them on the way out.  A pair then starts with its
+// window in shared memory: the placement statistics of a refined window read from the staged copy
+// (the tile's first bytes are their scratch), then one pass that writes the window and the chip
+// (loaded from L2 meanwhile) into the tile; the first transform pass takes the window's mean (and
+// a refined chip's) off.  Every wait is bounded; one that runs out is counted in errs, the CTA lets
+// the copy in flight land (again bounded) and returns.
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes)
 {
@@ -620,8 +810,8 @@ __device__ __forceinline__ void tensor_prefetch_l2(const CUtensorMap* map, int x
 template <int N1, int N2, bool RASTER, int NT, int CTAS>
 __global__ void __launch_bounds__(NT, CTAS)
 spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
-                   InvSource inv, const float2* tw_g, SpecOut out, unsigned int* errs,
-                   const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap cmap,
+                   InvSource inv, const float2* tw_g, SpecOut out, const TileStat* cstat, const TileStat* wstat,
+                   unsigned int* errs, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap cmap,
                    const __grid_constant__ CUtensorMap imap, int stall)
 {
     extern __shared__ __align__(16) unsigned char ssm[];
@@ -666,36 +856,45 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         mbar_wait(bar + 2, 0u, &s_err, kStallCycles);
         __syncthreads();
     }
-    // warp 0: the window rows of chunk pair b into the staging bytes, the chip rows toward L2; a
-    // pair without tiles (its offsets are -1) copies nothing and completes the phase at once
+    // Lane 0 of warp 0 brings in the windows: `look` finds out early where chunk pair b's tiles lie
+    // (loads and divisions whose latency must not hold up the copy), `issue` copies its window into
+    // the staging bytes and sends its chip toward L2.  A pair without tiles (its offsets are -1)
+    // copies nothing and completes the phase at once.
+    bool next_ok = false;
+    int nwx = 0, nwy = 0, ncx = 0, ncy = 0;
+    auto look = [&](long long b) {
+        next_ok = valid[pair0 + b] >= 0;
+        if constexpr (RASTER) {
+            if (!next_ok) return;
+            const long long wo = src.win_off[pair0 + b], co = src.chip_off[pair0 + b];
+            nwy = (int)(wo / ws);
+            nwx = (int)(wo - (long long)nwy * ws);
+            ncy = (int)(co / cs);
+            ncx = (int)(co - (long long)ncy * cs);
+        }
+    };
     auto issue = [&](long long b) {
-        if (valid[pair0 + b] < 0) {
-            if (lane == 0) mbar_arrive(bar);
+        if (!next_ok) {
+            mbar_arrive(bar);
             return;
         }
-        const float* w = spec_win(src, pair0, b);
-        const float* c = spec_chip(src, pair0, b);
         if constexpr (!RASTER) {
-            if (lane == 0) {
-                const unsigned bytes = (unsigned)W * (unsigned)W * 4u;
-                mbar_expect_tx(bar, bytes);
-                bulk_to_smem(stage, w, bytes, bar);
-                bulk_prefetch_l2(c, (unsigned)R * (unsigned)cs * 4u);
-            }
+            const unsigned bytes = (unsigned)W * (unsigned)W * 4u;
+            mbar_expect_tx(bar, bytes);
+            bulk_to_smem(stage, spec_win(src, pair0, b), bytes, bar);
+            bulk_prefetch_l2(spec_chip(src, pair0, b), (unsigned)R * (unsigned)cs * 4u);
         } else {
-            if (lane == 0) {
-                const long long wo = src.win_off[pair0 + b], co = src.chip_off[pair0 + b];
-                const int wy = (int)(wo / ws), wx = (int)(wo - (long long)wy * ws);
-                const int cy = (int)(co / cs), cx = (int)(co - (long long)cy * cs);
-                mbar_expect_tx(bar, ((unsigned)W * (unsigned)SW + (unsigned)C * (unsigned)g.inv_rs) * 4u);
-                tensor_to_smem(stage, &wmap, wx & ~3, wy, bar);
-                tensor_to_smem(inv_raw, &imap, wx & ~3, wy, bar);
-                tensor_prefetch_l2(&cmap, cx & ~3, cy);
-            }
+            mbar_expect_tx(bar, ((unsigned)W * (unsigned)SW + (unsigned)C * (unsigned)g.inv_rs) * 4u);
+            tensor_to_smem(stage, &wmap, nwx & ~3, nwy, bar);
+            tensor_to_smem(inv_raw, &imap, nwx & ~3, nwy, bar);
+            tensor_prefetch_l2(&cmap, ncx & ~3, ncy);
         }
     };
     const bool run = !stall || !s_err;
-    if (warp == 0 && blockIdx.x < pairs && run) issue(blockIdx.x);
+    if (tid == 0 && blockIdx.x < pairs && run) {
+        look(blockIdx.x);
+        issue(blockIdx.x);
+    }
     uint32_t parity = 0;
     bool inflight = blockIdx.x < pairs && run;
     long long b_left = blockIdx.x;  // (raster windows) the first pair left without a result
@@ -705,6 +904,15 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         const bool ok = valid[p] >= 0;
         const float* chip = spec_chip(src, pair0, b);
         const float* win = spec_win(src, pair0, b);
+        // the chip's mean (as two floats) and 1/|r'|; a refined window's mean and |t'|
+        const double mean_c = cstat[b].mean;
+        const float mc_hi = (float)mean_c, mc_lo = (float)(mean_c - (double)mc_hi);
+        const float inv_sigma = (float)cstat[b].inv_norm;
+        float sx = 0.0f, norm_w = 0.0f;
+        if constexpr (!RASTER) {
+            sx = (float)wstat[b].mean;
+            norm_w = (float)wstat[b].norm;
+        }
         const bool landed = mbar_wait(bar, parity, &s_err);
         if (__syncthreads_or(!landed)) {
             if constexpr (RASTER) b_left = b;
@@ -712,6 +920,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         }
         parity ^= 1u;
         inflight = false;
+        if (tid == 0 && bn < pairs) look(bn);
         if (!ok) {
             if (out.stage == 0 && tid == 0) {
                 out.coarse[p] = CoarseOut{-1, -1, -1, -1};
@@ -720,7 +929,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             if (bn < pairs) {
                 fence_async_smem();
                 __syncthreads();
-                if (warp == 0) issue(bn);
+                if (tid == 0) issue(bn);
                 inflight = true;
             }
             continue;
@@ -740,25 +949,11 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
                     cr[j][i] = y < R && x < R ? __ldg(chip + y * cs + x) : 0.0f;
                 }
         };
-        double mean_c = 0.0;
         if constexpr (RASTER) {
             load_chip();
             // the raster's placement statistics, copied with the window, into their C x C layout
             for (int u = warp; u < C; u += NW)
                 for (int v = lane; v < C; v += 32) invs[u * C + v] = inv_raw[u * g.inv_rs + xo + v];
-            // the chip's FP64 mean (spec_kernel's first sweep)
-            double c1 = 0.0;
-#pragma unroll
-            for (int j = 0; j < JN; ++j)
-#pragma unroll
-                for (int i = 0; i < IN; ++i) c1 += (double)cr[j][i];
-            c1 = warp_sum(c1);
-            if (lane == 0) red[warp] = c1;
-            __syncthreads();
-            double t1 = 0.0;
-            for (int w = 0; w < NW; ++w) t1 += red[w];
-            mean_c = t1 / ((double)R * (double)R);
-            __syncthreads();
         }
         auto wat = [&](int y, int x) {
             if constexpr (RASTER)
@@ -767,70 +962,30 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
                 return stage[y * W + x];
         };
 
-        // the window's sums of t - k and (t - k)^2 about a pivot k (its first sample), as
-        // spec_kernel takes them (in another order): here for the refined window, whose
-        // statistics are centred on its mean; as the tile is written for a raster window
-        const float pk = wat(0, 0);
-        double wsum[2] = {0.0, 0.0};
-        if constexpr (!RASTER) {
-            float sw = 0.0f, sw2 = 0.0f;
-            // four samples a load
-            const float4* s4 = reinterpret_cast<const float4*>(stage);
-            const int n4 = (W * W) >> 2;
-#pragma unroll 4
-            for (int k = tid; k < n4; k += NT) {
-                const float4 v = s4[k];
-                const float t[4] = {v.x - pk, v.y - pk, v.z - pk, v.w - pk};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    sw += t[q];
-                    sw2 = fmaf(t[q], t[q], sw2);
-                }
-            }
-            wsum[0] = sw;
-            wsum[1] = sw2;
-            block_sum2<NW>(wsum[0], wsum[1], red);
-        }
-        const double cells_c = (double)R * (double)R, cells_w = (double)W * (double)W;
-        double mean_w = (double)pk + wsum[0] / cells_w;
-        double st = fmax(wsum[1] - wsum[0] * wsum[0] / cells_w, 0.0) + 1e-5 * wsum[1];
-        float sx = (float)mean_w;
-
-        // placement statistics from the staged window where none are given; their scratch is the
+        // placement statistics of a refined window from the staged copy; their scratch is the
         // tile's first bytes
-        if constexpr (!RASTER) {
-            double* part = reinterpret_cast<double*>(ssm + g.off_gam);
-            const StatSlots vs{Zf, reinterpret_cast<float*>(part + 4 * g.nseg * W), g.off_stage / 4, 1};
-            spec_box_stats<NT>(wat, g, sx, vs, part, invs);
-        }
+        if constexpr (!RASTER)
+            staged_box_stats<NT>(stage, g, sx, Zf, reinterpret_cast<double*>(Zf + ((2 * C * W + 3) & ~3)), invs);
 
         // window (real parts) and chip (imaginary parts; its bytes were sent toward L2 with the
-        // window) into the tile, zeros around them.  Raster windows: the chip goes in zero-mean
-        // and |r'|^2 is summed as spec_kernel sums it, the window's sums are taken on the way.
-        // Refined tiles: the chip goes in as it is, its FP64 sum and sum of squares taken on the
-        // way (every product of two floats is exact in FP64), and the first transform pass takes
-        // its mean off.
+        // window) into the tile, zeros around them.  Raster windows: the chip goes in zero-mean, and
+        // the window's sums of t - k and (t - k)^2 about a pivot k (its first sample) are taken on
+        // the way, as spec_kernel takes them (in another order).  Refined tiles: the first transform
+        // pass takes the chip's mean off.
+        const float pk = wat(0, 0);
         if constexpr (!RASTER) load_chip();
-        const float mc_hi = (float)mean_c, mc_lo = (float)(mean_c - (double)mc_hi);
-        double c1 = 0.0, c2 = 0.0;
-        float sw = 0.0f, sw2 = 0.0f, sc2 = 0.0f;
+        float sw = 0.0f, sw2 = 0.0f;
         auto put = [&](int j, int i, float t) {
             const int y = warp + NW * j, x = lane + 32 * i;
             if (y < N && x < N) {
                 float c = cr[j][i];
                 if constexpr (RASTER) {
-                    if (y < R && x < R) {
-                        c = (c - mc_hi) - mc_lo;
-                        sc2 = fmaf(c, c, sc2);
-                    }
+                    if (y < R && x < R) c = (c - mc_hi) - mc_lo;
                     if (y < W && x < W) {
                         const float d = t - pk;
                         sw += d;
                         sw2 = fmaf(d, d, sw2);
                     }
-                } else {
-                    c1 += (double)c;
-                    c2 = fma((double)c, (double)c, c2);
                 }
                 Z[y * RS + x] = make_float2(t, c);
             }
@@ -863,53 +1018,31 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
 #pragma unroll
                     for (int i = 0; i < IN; ++i) put(j0 + q, i, v[q][i]);
         }
-        double ss;
         fft::Centre centre{sx, W};
         if constexpr (RASTER) {
-            const double d0 = warp_sum((double)sc2), d1 = warp_sum((double)sw), d2 = warp_sum((double)sw2);
+            const double d1 = warp_sum((double)sw), d2 = warp_sum((double)sw2);
             if (lane == 0) {
-                red[3 * warp] = d0;
-                red[3 * warp + 1] = d1;
-                red[3 * warp + 2] = d2;
-            }
-            __syncthreads();
-            ss = 0.0;
-            for (int w = 0; w < NW; ++w) {
-                ss += red[3 * w];
-                wsum[0] += red[3 * w + 1];
-                wsum[1] += red[3 * w + 2];
-            }
-            mean_w = (double)pk + wsum[0] / cells_w;
-            st = fmax(wsum[1] - wsum[0] * wsum[0] / cells_w, 0.0) + 1e-5 * wsum[1];
-            centre.sx = (float)mean_w;
-        } else {
-            c1 = warp_sum(c1);
-            c2 = warp_sum(c2);
-            if (lane == 0) {
-                red[2 * warp] = c1;
-                red[2 * warp + 1] = c2;
+                red[2 * warp] = d1;
+                red[2 * warp + 1] = d2;
             }
             __syncthreads();
             double s1 = 0.0, s2 = 0.0;
+#pragma unroll
             for (int w = 0; w < NW; ++w) {
                 s1 += red[2 * w];
                 s2 += red[2 * w + 1];
             }
-            // |r'|^2 = S2 - S1^2 / R^2 of the zero-mean chip; a chip flat to within its own
-            // rounding (a constant: its zero-mean values are exactly 0) gets 0, as the sum of the
-            // squared zero-mean values gives it
-            mean_c = s1 / cells_c;
-            ss = s2 - s1 * mean_c;
-            if (!(ss > 1e-14 * s2)) ss = 0.0;
-            const float hi = (float)mean_c;
-            centre.ci_hi = hi;
-            centre.ci_lo = (float)(mean_c - (double)hi);
+            const double cells = (double)W * (double)W;
+            centre.sx = (float)((double)pk + s1 / cells);
+            norm_w = sqrtf((float)(fmax(s2 - s1 * s1 / cells, 0.0) + 1e-5 * s2));
+        } else {
+            centre.ci_hi = mc_hi;
+            centre.ci_lo = mc_lo;
             centre.ci = R;
+            __syncthreads();
         }
-        const float inv_sigma = ss > 0.0 ? (float)(1.0 / sqrt(ss)) : 0.0f;
-
         const float scale = (float)(1.0 / (4.0 * (double)N * (double)N));
-        const float ebox = kSpecErr * (float)sqrt(st);
+        const float ebox = kSpecErr * norm_w;
         float bv = -INFINITY;
         int bi = INT_MAX;
         int flagged = 0;
@@ -932,14 +1065,14 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
                 fence_async_smem();
                 __syncthreads();
                 if (bn < pairs) {
-                    if (warp == 0) issue(bn);
+                    if (tid == 0) issue(bn);
                     inflight = true;
                 }
             });
 
         float* surf = out.surfaces ? out.surfaces + (size_t)p * C * C : nullptr;
         float* gam = out.stage == 1 ? out.gam + b * C * C : nullptr;
-        spec_surface<NT>(G, red, g, invs, inv_sigma, mean_c, ebox, chip, cs, win, ws, gam, surf, bv, bi,
+        spec_surface<NT>(G, red, g, invs, inv_sigma, (double)mc_hi + (double)mc_lo, ebox, chip, cs, win, ws, gam, surf, bv, bi,
                                    flagged);
         if (tid == 0) spec_result(out, p, R, W, C, bv, bi);
     }
@@ -997,14 +1130,14 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
 // one CTA of 256 threads per pair: FP64 mean and 1/|r - mean| of the R x R chip
 __global__ void __launch_bounds__(256)
 spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, int R,
-                       ChipStat* out)
+                       TileStat* out)
 {
     __shared__ double red[16];
     if (blockIdx.x >= pairs) return;
     const long long p = pair0 + blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (valid[p] < 0) {
-        if (tid == 0) out[blockIdx.x] = ChipStat{0.0, 0.0};
+        if (tid == 0) out[blockIdx.x] = TileStat{0.0, 0.0, 0.0};
         return;
     }
     const float* chip = spec_chip(src, pair0, blockIdx.x);
@@ -1029,10 +1162,7 @@ spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const l
             a += red[2 * w];
             b += red[2 * w + 1];
         }
-        const double cells = (double)R * (double)R;
-        const double mean = a / cells;
-        const double ss = b - cells * mean * mean;
-        out[blockIdx.x] = ChipStat{mean, ss > 0.0 ? 1.0 / sqrt(ss) : 0.0};
+        out[blockIdx.x] = tile_stat(a, b, (double)R * (double)R);
     }
 }
 
@@ -1058,7 +1188,7 @@ spec_tile_stats_kernel(SpecSource src, long long pair0, long long pairs, const l
 template <int N1, int N2>
 __global__ void __launch_bounds__(kSpecThreads, 1)
 spec_block_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
-                  int nb, const ChipStat* cstat, const float2* tw_g, float* part, double* scal)
+                  int nb, const TileStat* cstat, const float2* tw_g, float* part, double* scal)
 {
     extern __shared__ __align__(16) unsigned char ssm[];
     const int K = nb * nb;
@@ -1080,7 +1210,7 @@ spec_block_kernel(SpecSource src, long long pair0, long long pairs, const long l
     const long long cs = src.chip_stride, ws = src.win_stride;
     const float* chip = spec_chip(src, pair0, b) + i0 * cs + j0;
     const float* win = spec_win(src, pair0, b) + i0 * ws + j0;
-    const ChipStat cst = cstat[b];
+    const TileStat cst = cstat[b];
     const float mc_hi = (float)cst.mean, mc_lo = (float)(cst.mean - (double)mc_hi);
 
     // the block of the chip, centred on the whole chip's mean, to registers; the sub-window to the
@@ -1174,7 +1304,7 @@ spec_block_kernel(SpecSource src, long long pair0, long long pairs, const long l
 // placement statistics and the surface (C^2 floats each) and a reduction scratch.
 __global__ void __launch_bounds__(kThreads, 1)
 spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
-                   int K, const ChipStat* cstat, InvSource inv, const float* part, const double* scal,
+                   int K, const TileStat* cstat, InvSource inv, const float* part, const double* scal,
                    SpecOut out)
 {
     extern __shared__ __align__(16) unsigned char ssm[];
@@ -1204,8 +1334,8 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
         corr += sc[2 * k];
         errs += sc[2 * k + 1];
     }
-    const ChipStat cst = cstat[blockIdx.x];
-    const float inv_sigma = (float)cst.inv_sigma;
+    const TileStat cst = cstat[blockIdx.x];
+    const float inv_sigma = (float)cst.inv_norm;
     const float ebox = kSpecErr * (float)errs * inv_sigma;
     __syncthreads();
     float bv = -INFINITY;
@@ -1465,7 +1595,7 @@ cudaError_t spec_set_smem_limits()
 }
 
 cudaError_t launch_spec_chip_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                   long long pairs, const long long* valid, int R, ChipStat* out)
+                                   long long pairs, const long long* valid, int R, TileStat* out)
 {
     spec_chip_stats_kernel<<<blocks, 256, 0, st>>>(src, pair0, pairs, valid, R, out);
     return cudaGetLastError();
@@ -1496,7 +1626,7 @@ cudaError_t launch_spec_tile_stats(unsigned blocks, cudaStream_t st, SpecSource 
 
 cudaError_t launch_spec_block(const SpecGeom& tile, int nb, unsigned blocks, cudaStream_t st,
                               SpecSource src, long long pair0, long long pairs,
-                              const long long* valid, const ChipStat* cstat, const float2* tw,
+                              const long long* valid, const TileStat* cstat, const float2* tw,
                               float* part, double* scal)
 {
 #define AMPCOR_SPEC_CASE(NN, A, B)                                                                   \
@@ -1517,7 +1647,7 @@ int spec_reduce_smem(int C)
 
 cudaError_t launch_spec_reduce(const SpecGeom& full, int K, unsigned blocks, cudaStream_t st,
                                SpecSource src, long long pair0, long long pairs,
-                               const long long* valid, const ChipStat* cstat, InvSource inv,
+                               const long long* valid, const TileStat* cstat, InvSource inv,
                                const float* part, const double* scal, SpecOut out)
 {
     spec_reduce_kernel<<<blocks, kThreads, spec_reduce_smem(full.C), st>>>(src, pair0, pairs, valid, full, K,
@@ -1543,17 +1673,18 @@ cudaError_t launch_spec(const SpecGeom& g, unsigned blocks, cudaStream_t st, Spe
 
 cudaError_t launch_spec_staged(const SpecGeom& g, unsigned sms, cudaStream_t st, SpecSource src,
                                long long pair0, long long pairs, const long long* valid, InvSource inv,
-                               const float2* tw, SpecOut out, unsigned int* errs, const CUtensorMap* wmap,
-                               const CUtensorMap* cmap, const CUtensorMap* imap, int stall)
+                               const float2* tw, SpecOut out, const TileStat* cstat, const TileStat* wstat,
+                               unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap,
+                               const CUtensorMap* imap, int stall)
 {
     if (pairs <= 0) return cudaSuccess;
     const unsigned blocks = (unsigned)std::min<long long>(pairs, std::max(1u, sms) * (long long)g.ctas);
     auto run = [&](auto raster, auto dense) {
         if (wmap)
-            raster<<<blocks, g.threads, g.smem_staged, st>>>(src, pair0, pairs, valid, g, inv, tw, out, errs, *wmap,
-                                                             *cmap, *imap, stall);
+            raster<<<blocks, g.threads, g.smem_staged, st>>>(src, pair0, pairs, valid, g, inv, tw, out, cstat, wstat, errs,
+                                                             *wmap, *cmap, *imap, stall);
         else
-            dense<<<blocks, g.threads, g.smem_staged, st>>>(src, pair0, pairs, valid, g, inv, tw, out, errs,
+            dense<<<blocks, g.threads, g.smem_staged, st>>>(src, pair0, pairs, valid, g, inv, tw, out, cstat, wstat, errs,
                                                             CUtensorMap{}, CUtensorMap{}, CUtensorMap{}, stall);
         return cudaGetLastError();
     };

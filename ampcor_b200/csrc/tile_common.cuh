@@ -93,6 +93,17 @@ __device__ void block_argmax_n(float& bv, int& bi, float* redf, int* redi)
     __syncthreads();
 }
 
+// the statistics of a tile of n amplitudes from their FP64 sum and sum of squares: S2 - S1^2 / n; a
+// tile flat to within its own rounding (a constant: its deviations are exactly 0) has norm 0
+__device__ __forceinline__ TileStat tile_stat(double s1, double s2, double n)
+{
+    const double mean = s1 / n;
+    double ss = s2 - s1 * mean;
+    if (!(ss > 1e-14 * s2)) ss = 0.0;
+    const double norm = sqrt(ss);
+    return TileStat{mean, norm > 0.0 ? 1.0 / norm : 0.0, norm};
+}
+
 // exclusive prefix sum of row[0..n) written in place, with the total in row[n] (one warp)
 __device__ void warp_prefix(double* row, int n)
 {
