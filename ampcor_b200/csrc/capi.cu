@@ -551,7 +551,8 @@ struct ampcor_handle {
     unsigned int* h_status = nullptr;
     // refined amplitudes of one chunk of pairs
     float* d_refined = nullptr;
-    size_t chunk = 0;
+    size_t chunk = 0;      // pairs per chunk
+    size_t chunk_cap = 0;  // pairs the scratch holds: the chunk, or all of a smaller job
     size_t chunk_override = 0;
     long long refined_stride = 0;
     // host-path staging
@@ -681,20 +682,27 @@ int ensure_pairs(ampcor_handle* h, size_t pairs)
     return AMPCOR_OK;
 }
 
-// the chunk of pairs whose refined amplitudes are resident at once: a few waves of CTAs,
-// small enough that the refined tiles mostly stay in L2 between the refine and fine kernels
-size_t default_chunk()
+// The chunk of pairs whose refined amplitudes are resident at once, unless configured or set by
+// AMPCOR_CHUNK: as many waves of 592 pairs (four to a multiprocessor) as keep the scratch of a pair
+// (refined amplitudes and surface) within half a gigabyte in all, at least one.  Each chunk costs
+// five launches whose last waves leave multiprocessors idle, and reading the refined tiles from HBM
+// instead of L2 costs less than that: 23,625 pairs of 32 px chips in 40 chunks of 592 take 5.38 ms,
+// in 3 chunks 4.07 ms; the scratch of a worker is what bounds the chunk.
+size_t default_chunk(const ampcor_handle* h)
 {
     const char* env = std::getenv("AMPCOR_CHUNK");
     if (env) {
         long v = std::strtol(env, nullptr, 10);
         if (v > 0) return (size_t)v;
     }
-    return 148 * 4;
+    const size_t pair = ((size_t)h->Rf * h->Rf + (size_t)h->Wf * h->Wf + (size_t)h->Cf * h->Cf) * sizeof(float);
+    const size_t wave = 148 * 4;
+    return std::max<size_t>(1, (size_t)512 * 1024 * 1024 / (pair * wave)) * wave;
 }
 
 void free_chunk_scratch(ampcor_handle* h)
 {
+    h->chunk_cap = 0;
     cudaFree(h->d_refined);
     cudaFree(h->d_inv_c);
     cudaFree(h->d_inv_f);
@@ -720,18 +728,21 @@ int scratch_fail(ampcor_handle* h, const std::string& what)
     return fail(h, AMPCOR_E_NOMEM, what);
 }
 
-int ensure_refined(ampcor_handle* h)
+// the scratch of a job of `pairs` pairs: a chunk's, or less where the job is smaller
+int ensure_refined(ampcor_handle* h, size_t pairs)
 {
-    if (h->d_refined) return AMPCOR_OK;
-    h->chunk = h->chunk_override ? h->chunk_override : default_chunk();
+    h->chunk = h->chunk_override ? h->chunk_override : default_chunk(h);
+    const size_t n = std::min(h->chunk, std::max<size_t>(pairs, 1));
+    if (h->d_refined && h->chunk_cap >= n) return AMPCOR_OK;
+    free_chunk_scratch(h);
     h->refined_stride = (long long)h->Rf * h->Rf + (long long)h->Wf * h->Wf;
     // 16 floats of slack: staged copies round rows out to 16-byte boundaries
-    cudaError_t e = cudaMalloc(&h->d_refined, (h->chunk * h->refined_stride + 16) * sizeof(float));
+    cudaError_t e = cudaMalloc(&h->d_refined, (n * h->refined_stride + 16) * sizeof(float));
     if (e != cudaSuccess) {
         h->d_refined = nullptr;
         return scratch_fail(h, std::string("allocating refinement scratch: ") + cudaGetErrorName(e));
     }
-    const size_t n = h->chunk;
+    h->chunk_cap = n;
     // per-pair placement statistics: only the tensor-core form stages them in memory (the
     // spectral form takes them from the raster or computes them in the correlation kernel)
     if (h->form == kFormTensor &&
@@ -792,7 +803,7 @@ int run_plain(ampcor_handle* h, const PairSource& src, long long pairs, float2* 
               PairDiag* diag, float* coarse_surfaces, float* refined_surfaces, cudaStream_t st)
 {
     if (pairs == 0) return AMPCOR_OK;
-    int rc = ensure_refined(h);
+    int rc = ensure_refined(h, (size_t)pairs);
     if (rc) return rc;
     cudaEvent_t a = mark(h, st);
     coarse_kernel<<<(unsigned)pairs, kThreads, h->gc.smem_bytes, st>>>(
@@ -851,7 +862,7 @@ int run_tensor(ampcor_handle* h, const PairSource& src, long long pairs, float2*
                PairDiag* diag, float* coarse_surfaces, float* refined_surfaces, cudaStream_t st)
 {
     if (pairs == 0) return AMPCOR_OK;
-    int rc = ensure_refined(h);
+    int rc = ensure_refined(h, (size_t)pairs);
     if (rc) return rc;
     if ((rc = ensure_fine_out(h, (size_t)pairs))) return rc;
     const RealTiles rt{h->d_refined, h->refined_stride, 0, (long long)h->Rf * h->Rf};
@@ -939,7 +950,7 @@ bool raster_map(CUtensorMap& m, const float* base, long long lines, long long sa
 
 int spec_rasters(ampcor_handle* h, const PairSource& src, long long pairs, SpecRasters& r)
 {
-    int rc = ensure_refined(h);
+    int rc = ensure_refined(h, (size_t)pairs);
     if (rc) return rc;
     if ((rc = ensure_fine_out(h, (size_t)pairs))) return rc;
     r.shared = src.ref_base == src.tgt_base;
@@ -1023,8 +1034,8 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
     for (long long c0 = p0; c0 < p1; c0 += (long long)h->chunk) {
         const unsigned n = (unsigned)std::min<long long>((long long)h->chunk, p1 - c0);
         TileStat* const st_raw = h->d_tstat;               // the chips
-        TileStat* const st_chip = st_raw + h->chunk;       // the refined chips
-        TileStat* const st_win = st_chip + h->chunk;       // the refined windows
+        TileStat* const st_chip = st_raw + h->chunk_cap;       // the refined chips
+        TileStat* const st_win = st_chip + h->chunk_cap;       // the refined windows
         const float2* tab = reinterpret_cast<const float2*>(h->d_tw_refine);
         const bool deramp = (h->prm.flags & AMPCOR_FLAG_DERAMP) != 0;
         // the chips' refinement needs no coarse result, and gives the coarse stage their statistics
@@ -1756,7 +1767,7 @@ int ampcor_inject_timeout(ampcor_handle* h, int batches)
 int ampcor_chunk(const ampcor_handle* h, uint64_t* chunk)
 {
     if (!h || !chunk) return AMPCOR_E_ARG;
-    *chunk = h->chunk_override ? h->chunk_override : default_chunk();
+    *chunk = h->chunk_override ? h->chunk_override : default_chunk(h);
     return AMPCOR_OK;
 }
 
