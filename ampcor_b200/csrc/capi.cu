@@ -345,8 +345,9 @@ bool plan_spec_shared(int R, int W, bool dense, SpecGeom& g)
 // reduction.
 struct SpecBlocks {
     bool on = false;
+    bool staged = false;  // the tile's staged form is planned
     int B = 0, nb = 0, K = 0;
-    SpecGeom tile{};
+    SpecGeom tile{}, tile_st{};
     SpecGeom full{};
 };
 
@@ -374,6 +375,62 @@ bool plan_spec_tile(int B, int S, int C, SpecGeom& g)
     return off <= 227L * 1024;
 }
 
+// The staged form of a block's tile (spec_block_staged_kernel, K blocks to a pair): plan_spec_staged's
+// layout for windows that may sit off 16-byte boundaries, without the statistics and the surface.
+// Where the summed spectrum of the blocks fits beside the tile, with the staged bytes at the tile's
+// end: a block's tile is free once its spectrum is summed, only the last block's inverse still uses
+// the first rows, so that its copy waits (`late`) if those reach the staged bytes.  Otherwise block
+// by block, where the staged bytes fit beside the rows of every inverse (searches of +-64 px, 129
+// placement rows of a 160-sample tile, keep spec_block_kernel: a copy after the inverse hides
+// nothing, 963 us against 914 for 900 pairs of 64 px chips).
+bool plan_spec_block_staged(int K, SpecGeom& g)
+{
+    auto up = [](long x, long a) { return (x + a - 1) / a * a; };
+    const int N = g.N, C = g.C, S = g.W, warps = kSpecWarps;
+    const long limit = 227L * 1024, row = (long)g.RS * 8, tile = (long)N * row;
+    g.stage_rs = (S + 6) & ~3;
+    if (g.stage_rs > 256 || S > 256) return false;
+    const long bytes = (long)S * g.stage_rs * 4;
+    const int np = (C + 1) / 2;
+    const long kept = (long)(C + np <= N ? C + np : C) * row;
+    const long sum = (long)(N / 2 + 1) * N * 8;
+    auto layout = [&](long at) {
+        const int y0 = (int)std::min<long>(N, at / row) / warps * warps;
+        const int JN = (N + warps - 1) / warps;
+        for (int j0 = 0; j0 < JN; j0 += kStagePieces) {
+            const long y1 = (long)std::min(j0 + kStagePieces, JN) * warps;
+            if (y1 <= y0 || y1 >= S) continue;
+            if (y1 * row > at + y1 * g.stage_rs * 4) return limit + 1;
+        }
+        g.off_stage = (int)at;
+        g.stage_y0 = y0;
+        g.stage_pj = kStagePieces;
+        long off = up(std::max(tile, at + bytes), 16);
+        g.off_tw = (int)off;
+        off = up(off + (long)N * 8, 16);
+        g.off_neg = (int)off;
+        off = up(off + (long)N * 4, 16);
+        g.off_half = (int)off;
+        off = up(off + (long)(N / 2 + 1) * 4, 16);
+        g.off_red = (int)off;
+        off += 4L * kSpecWarps * 8;
+        g.off_bar = (int)off;
+        off += 32;
+        g.off_gam = (int)off;
+        return off;
+    };
+    if (K > 1 && N <= 128 && tile >= bytes) {
+        const long at = up(tile - bytes, 128);
+        g.acc = 1;
+        g.late = kept > at ? 1 : 0;
+        g.smem_staged = (int)(layout(at) + sum);
+        if (g.smem_staged <= limit) return true;
+    }
+    g.acc = g.late = 0;
+    g.smem_staged = (int)layout(up(std::max(kept, tile - bytes), 128));
+    return N >= 128 && g.smem_staged <= limit;
+}
+
 bool plan_spec_blocked(int R, int W, SpecBlocks& b, std::string& err)
 {
     b = SpecBlocks{};
@@ -396,6 +453,8 @@ bool plan_spec_blocked(int R, int W, SpecBlocks& b, std::string& err)
         b.full.R = R;
         b.full.W = W;
         b.full.C = C;
+        b.tile_st = b.tile;
+        b.staged = plan_spec_block_staged(b.K, b.tile_st);
         return true;
     }
     err = "no block of the chip fits the spectral form (the search margin is too large)";
@@ -573,6 +632,7 @@ struct ampcor_handle {
     // multiprocessors
     SpecGeom spc_st{}, spf_st{};
     bool coarse_staged = false, fine_staged = false;
+    bool staged_on = false;  // the staged forms are allowed (AMPCOR_STAGED is not 0)
     int sms = 0;
     // zoom of the tensor-core and spectral forms
     ZoomGeomCols zc{};
@@ -948,6 +1008,22 @@ bool raster_map(CUtensorMap& m, const float* base, long long lines, long long sa
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// the same of `pairs` dense float tiles of n x n samples, `stride` floats apart
+bool tiles_map(CUtensorMap& m, const float* base, int n, long long pairs, long long stride, int bx, int by)
+{
+    const EncodeTiledFn fn = encode_tiled();
+    if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || (n & 3) || (stride & 3) || pairs < 1 || bx % 4 || bx < 4 ||
+        bx > 256 || by < 1 || by > 256)
+        return false;
+    const cuuint64_t dim[3] = {(cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)pairs};
+    const cuuint64_t strides[2] = {(cuuint64_t)n * 4, (cuuint64_t)stride * 4};
+    const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
+    const cuuint32_t es[3] = {1, 1, 1};
+    return fn(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dim, strides, box, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int spec_rasters(ampcor_handle* h, const PairSource& src, long long pairs, SpecRasters& r)
 {
     int rc = ensure_refined(h, (size_t)pairs);
@@ -1031,6 +1107,19 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         raster_map(wmap, r.amp_tgt, src.tgt_count / src.tgt_stride, src.tgt_stride, h->spc_st.stage_rs, h->W) &&
         raster_map(cmap, r.amp_ref, src.ref_count / src.ref_stride, src.ref_stride, (h->R + 6) & ~3, h->R) &&
         raster_map(imap, r.inv_c.base, r.rows, src.tgt_stride, h->spc_st.inv_rs, h->C);
+    // the blocked stages through the copy engine: the coarse windows and chips of two rasters, the
+    // refined ones of the chunk's tiles
+    CUtensorMap bwc{}, bcc{}, bwf{}, bcf{};
+    const bool bc_st = h->staged_on && h->bc.on && h->bc.staged && src.tgt_lines > 0 && src.tgt_stride > 0 && src.ref_stride > 0 &&
+                       raster_map(bwc, r.amp_tgt, src.tgt_count / src.tgt_stride, src.tgt_stride,
+                                  h->bc.tile_st.stage_rs, h->bc.tile_st.W) &&
+                       raster_map(bcc, r.amp_ref, src.ref_count / src.ref_stride, src.ref_stride, (h->bc.B + 6) & ~3,
+                                  h->bc.B);
+    const bool bf_st = h->staged_on && h->bf.on && h->bf.staged &&
+                       tiles_map(bwf, h->d_refined + (long long)h->Rf * h->Rf, h->Wf, (long long)h->chunk_cap,
+                                 h->refined_stride, h->bf.tile_st.stage_rs, h->bf.tile_st.W) &&
+                       tiles_map(bcf, h->d_refined, h->Rf, (long long)h->chunk_cap, h->refined_stride,
+                                 (h->bf.B + 6) & ~3, h->bf.B);
     for (long long c0 = p0; c0 < p1; c0 += (long long)h->chunk) {
         const unsigned n = (unsigned)std::min<long long>((long long)h->chunk, p1 - c0);
         TileStat* const st_raw = h->d_tstat;               // the chips
@@ -1065,10 +1154,16 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
                 keep(h, 3, b, b2);
                 b = b2;
             }
-            CK(h, launch_spec_block(h->bc.tile, h->bc.nb, n * (unsigned)h->bc.K, st, cs, c0, n, src.ref_off,
-                                    st_raw, reinterpret_cast<const float2*>(h->d_tw_c), h->d_part, h->d_scal),
-               "launching the blocked coarse correlation");
-            CK(h, launch_spec_reduce(h->bc.full, h->bc.K, n, st, cs, c0, n, src.ref_off, st_raw, ic,
+            if (bc_st)
+                CK(h, launch_spec_block_staged(h->bc.tile_st, h->bc.nb, (unsigned)h->sms, st, cs, c0, n, src.ref_off,
+                                               st_raw, reinterpret_cast<const float2*>(h->d_tw_c), h->d_part,
+                                               h->d_scal, h->d_tc_err, &bwc, &bcc, 1),
+                   "launching the staged blocked coarse correlation");
+            else
+                CK(h, launch_spec_block(h->bc.tile, h->bc.nb, n * (unsigned)h->bc.K, st, cs, c0, n, src.ref_off,
+                                        st_raw, reinterpret_cast<const float2*>(h->d_tw_c), h->d_part, h->d_scal),
+                   "launching the blocked coarse correlation");
+            CK(h, launch_spec_reduce(h->bc.full, h->bc.K, bc_st && h->bc.tile_st.acc ? 1 : h->bc.K, n, st, cs, c0, n, src.ref_off, st_raw, ic,
                                      h->d_part, h->d_scal, co),
                "launching the coarse reduction");
         } else {
@@ -1114,10 +1209,16 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
             cudaEvent_t e2 = mark(h, st);
             keep(h, 4, e, e2);
             e = e2;
-            CK(h, launch_spec_block(h->bf.tile, h->bf.nb, n * (unsigned)h->bf.K, st, fs, c0, n, src.ref_off,
-                                    st_chip, reinterpret_cast<const float2*>(h->d_tw_f), h->d_part, h->d_scal),
-               "launching the blocked fine correlation");
-            CK(h, launch_spec_reduce(h->bf.full, h->bf.K, n, st, fs, c0, n, src.ref_off, st_chip,
+            if (bf_st)
+                CK(h, launch_spec_block_staged(h->bf.tile_st, h->bf.nb, (unsigned)h->sms, st, fs, c0, n, src.ref_off,
+                                               st_chip, reinterpret_cast<const float2*>(h->d_tw_f), h->d_part,
+                                               h->d_scal, h->d_tc_err, &bwf, &bcf, 0),
+                   "launching the staged blocked fine correlation");
+            else
+                CK(h, launch_spec_block(h->bf.tile, h->bf.nb, n * (unsigned)h->bf.K, st, fs, c0, n, src.ref_off,
+                                        st_chip, reinterpret_cast<const float2*>(h->d_tw_f), h->d_part, h->d_scal),
+                   "launching the blocked fine correlation");
+            CK(h, launch_spec_reduce(h->bf.full, h->bf.K, bf_st && h->bf.tile_st.acc ? 1 : h->bf.K, n, st, fs, c0, n, src.ref_off, st_chip,
                                      InvSource{h->d_inv_blk, nullptr, 0}, h->d_part, h->d_scal, fo),
                "launching the fine reduction");
         } else {
@@ -1249,6 +1350,7 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         // pair are dense rows of one buffer, staged whole when its rows are 16-byte multiples
         const char* stg = std::getenv("AMPCOR_STAGED");
         const bool staged_on = !(stg && std::strcmp(stg, "0") == 0);
+        h->staged_on = staged_on;
         h->coarse_staged = staged_on && direct_c && plan_spec_staged(h->R, h->W, false, kSpecThreads, h->spc_st);
         h->fine_staged = staged_on && direct_f &&
                          plan_spec_staged(h->Rf, h->Wf, h->Rf % 2 == 0 && h->Wf % 2 == 0, kSpecThreads, h->spf_st) &&

@@ -635,8 +635,13 @@ HD void half_positions(int* out)
 // the inverse step B of column x back into the group (of both groups when x is its own partner:
 // the columns of frequencies 0 and N/2).  Every (column, group) belongs to one task, so the pass
 // runs in place without a barrier between its steps.
-template <int N1, int N2, bool K0>
-HD void spectrum_groups(float2* Z, int RS, int x, int xn, int k1)
+//
+// With ACC the spectra of several tiles are summed before the inverse: acc holds the sum so far (the
+// task's value k2 at acc[k2 stride]), read unless this tile is the first and, unless it is the last,
+// written instead of the inverse.
+template <int N1, int N2, bool K0, bool ACC = false>
+HD void spectrum_groups(float2* Z, int RS, int x, int xn, int k1, float2* acc = nullptr, int stride = 0,
+                        bool first = true, bool last = true)
 {
     const int k1n = K0 ? 0 : N1 - k1;
     const bool self_col = x == xn, self = self_col && k1 == k1n;
@@ -659,6 +664,16 @@ HD void spectrum_groups(float2* Z, int RS, int x, int xn, int k1)
         const int k2n = K0 ? (N2 - k2) % N2 : N2 - 1 - k2;
         const float2 c = corr_cell(a[k2], b[k2n]);
         a[k2] = c;
+    }
+    if constexpr (ACC) {
+        if (!first)
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) a[k2] = cadd(a[k2], acc[k2 * stride]);
+        if (!last) {
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) acc[k2 * stride] = a[k2];
+            return;
+        }
     }
     if (self_col && !self) {
 #pragma unroll
@@ -700,10 +715,12 @@ struct NoHook {
 
 // PAIR: 2 runs every pass two tasks at a time, 1 only the passes of N1-point steps (fewer
 // registers), 0 none
-template <int N1, int N2, int PAIR = 0, class Sync, class Store, class Hook = NoHook>
-HD void correlate_tile(float2* Z, int RS, int rows_in, int rows_out, const float2* tw,
-                       const int* neg, const int* half, const Centre& centre, int tid, int nt,
-                       Sync sync, Store store, Hook cols_done = Hook{})
+//
+// The forward transform but for its last step: rows (centring the tile on the way in), then the
+// columns' step A.
+template <int N1, int N2, int PAIR, class Cen, class Sync>
+HD void correlate_forward(float2* Z, int RS, int rows_in, const float2* tw, const Cen& centre, int tid, int nt,
+                          Sync sync)
 {
     constexpr int N = N1 * N2;
     // forward along rows (centring the tile on the way in): lanes take consecutive rows
@@ -731,19 +748,14 @@ HD void correlate_tile(float2* Z, int RS, int rows_in, int rows_out, const float
     else
         for (int t = tid; t < N * N2; t += nt) fwd_a<N1, N2>(Z + t % N, RS, t / N, tw);
     sync();
-    // the columns' forward step B, the correlation spectrum and the inverse's step B on the
-    // columns of the Hermitian half, one task per pair of column groups
-    constexpr int NH = half_count<N1, N2>();
-    for (int t = tid; t < NH * N1; t += nt) {
-        const int c = t % NH, k1 = t / NH;
-        const int x = half[c], xn = neg[x];
-        if (x == xn && k1 > (N1 - k1) % N1) continue;  // done by the task of the partner group
-        if (k1 == 0)
-            spectrum_groups<N1, N2, true>(Z, RS, x, xn, k1);
-        else
-            spectrum_groups<N1, N2, false>(Z, RS, x, xn, k1);
-    }
-    sync();
+}
+
+// The inverse transform from the columns' step A on.
+template <int N1, int N2, int PAIR, class Sync, class Store, class Hook>
+HD void correlate_inverse(float2* Z, int RS, int rows_out, const float2* tw, const int* neg, const int* half, int tid,
+                          int nt, Sync sync, Store store, Hook cols_done)
+{
+    constexpr int N = N1 * N2, NH = half_count<N1, N2>();
     // (only the placement rows are read from here on)
     if constexpr (PAIR >= 1)
         tasks2(
@@ -796,6 +808,55 @@ HD void correlate_tile(float2* Z, int RS, int rows_in, int rows_out, const float
         });
         sync();
     }
+}
+
+template <int N1, int N2, int PAIR = 0, class Sync, class Store, class Hook = NoHook>
+HD void correlate_tile(float2* Z, int RS, int rows_in, int rows_out, const float2* tw,
+                       const int* neg, const int* half, const Centre& centre, int tid, int nt,
+                       Sync sync, Store store, Hook cols_done = Hook{})
+{
+    correlate_forward<N1, N2, PAIR>(Z, RS, rows_in, tw, centre, tid, nt, sync);
+    // the columns' forward step B, the correlation spectrum and the inverse's step B on the
+    // columns of the Hermitian half, one task per pair of column groups
+    constexpr int NH = half_count<N1, N2>();
+    for (int t = tid; t < NH * N1; t += nt) {
+        const int c = t % NH, k1 = t / NH;
+        const int x = half[c], xn = neg[x];
+        if (x == xn && k1 > (N1 - k1) % N1) continue;  // done by the task of the partner group
+        if (k1 == 0)
+            spectrum_groups<N1, N2, true>(Z, RS, x, xn, k1);
+        else
+            spectrum_groups<N1, N2, false>(Z, RS, x, xn, k1);
+    }
+    sync();
+    correlate_inverse<N1, N2, PAIR>(Z, RS, rows_out, tw, neg, half, tid, nt, sync, store, cols_done);
+}
+
+// correlate_tile of one of several tiles whose correlations add up, all N x N and at the same
+// placements (chip blocks of one pair): the spectra are summed in acc (half_count N1 N2 values), and
+// only the last tile is transformed back.  tile_done() runs in every thread once the tile may be
+// overwritten (for the last one from its row rows_out + (rows_out + 1) / 2 on, as cols_done).
+template <int N1, int N2, int PAIR, class Cen, class Sync, class Store, class Hook>
+HD void correlate_sum(float2* Z, int RS, int rows_in, int rows_out, const float2* tw, const int* neg,
+                      const int* half, const Cen& centre, float2* acc, bool first, bool last, int tid, int nt,
+                      Sync sync, Store store, Hook tile_done)
+{
+    correlate_forward<N1, N2, PAIR>(Z, RS, rows_in, tw, centre, tid, nt, sync);
+    constexpr int NH = half_count<N1, N2>();
+    for (int t = tid; t < NH * N1; t += nt) {
+        const int c = t % NH, k1 = t / NH;
+        const int x = half[c], xn = neg[x];
+        if (x == xn && k1 > (N1 - k1) % N1) continue;  // done by the task of the partner group
+        if (k1 == 0)
+            spectrum_groups<N1, N2, true, true>(Z, RS, x, xn, k1, acc + t, NH * N1, first, last);
+        else
+            spectrum_groups<N1, N2, false, true>(Z, RS, x, xn, k1, acc + t, NH * N1, first, last);
+    }
+    sync();
+    if (last)
+        correlate_inverse<N1, N2, PAIR>(Z, RS, rows_out, tw, neg, half, tid, nt, sync, store, tile_done);
+    else
+        tile_done();
 }
 
 }  // namespace fft

@@ -229,6 +229,8 @@ struct SpecGeom {
     int off_inv_raw, inv_rs;  // raster statistics as copied: C rows of inv_rs floats
     int smem_staged;  // 0: no staged form for this stage
     int threads, ctas;  // of a CTA, and resident CTAs per SM
+    int late; // summed blocks: the copy during a pair's inverse waits for its end (no room beside its rows)
+    int acc;  // staged blocks: the blocks' spectra are summed (the sum at off_gam) and transformed back once
 };
 
 // float amplitude tiles of chunk-local pair b (global pair pair0 + b): at base + off[pair0 + b]
@@ -314,8 +316,16 @@ cudaError_t launch_spec_block(const SpecGeom& tile, int nb, unsigned blocks, cud
                               SpecSource src, long long pair0, long long pairs,
                               const long long* valid, const TileStat* cstat, const float2* tw,
                               float* part, double* scal);
+// the same through the copy engine, resident CTAs walking the blocks (part: C^2 floats per pair where
+// tile.acc): wmap and cmap map the window and chip sources, 2-D over the amplitude rasters with boxes
+// of stage_rs x W and (R + 6 & ~3) x R floats, or (raster 0) 3-D over the refined tiles, a pair deep
+cudaError_t launch_spec_block_staged(const SpecGeom& tile, int nb, unsigned sms, cudaStream_t st, SpecSource src,
+                                     long long pair0, long long pairs, const long long* valid,
+                                     const TileStat* cstat, const float2* tw, float* part, double* scal,
+                                     unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster);
 int spec_reduce_smem(int C);
-cudaError_t launch_spec_reduce(const SpecGeom& full, int K, unsigned blocks, cudaStream_t st,
+// kp: partial surfaces per pair
+cudaError_t launch_spec_reduce(const SpecGeom& full, int K, int kp, unsigned blocks, cudaStream_t st,
                                SpecSource src, long long pair0, long long pairs,
                                const long long* valid, const TileStat* cstat, InvSource inv,
                                const float* part, const double* scal, SpecOut out);

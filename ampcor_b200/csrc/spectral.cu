@@ -336,7 +336,8 @@ __device__ __forceinline__ pair_t pk_fma(pair_t a, pair_t b, pair_t c)
 // spec_box_stats for a staged refined window (W dense floats a row, W a multiple of 4): the same sums
 // in the same precision, two columns to a thread in packed FP32, and the box sums' first warp sum
 // carries both moments at once (one half of the warp each).  V: 2 C W floats, part: 4 nseg W
-// doubles, both in the tile's first bytes.  @@MEAS4@@
+// doubles, both in the tile's first bytes.  Clock stamps at the production geometry: 10.7K cycles a
+// pair (3.0K, 2.9K and 4.7K in its three phases) against 13.1K of spec_box_stats on the same copy.
 template <int NT>
 __device__ void staged_box_stats(const float* win, const SpecGeom& g, float sx, float* V, double* part, float* invs)
 {
@@ -793,6 +794,23 @@ __device__ __forceinline__ void tensor_to_smem(void* dst, const CUtensorMap* map
             saddr(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(saddr(bar))
         : "memory");
+}
+
+// the same of a 3-D map at (x, y, z)
+__device__ __forceinline__ void tensor3_to_smem(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            saddr(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(saddr(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void tensor3_prefetch_l2(const CUtensorMap* map, int x, int y, int z)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map)),
+                 "r"(x), "r"(y), "r"(z)
+                 : "memory");
 }
 
 __device__ __forceinline__ void tensor_prefetch_l2(const CUtensorMap* map, int x, int y)
@@ -1297,14 +1315,263 @@ spec_block_kernel(SpecSource src, long long pair0, long long pairs, const long l
     }
 }
 
+// The blocks of a stage whose tiles the copy engine can bring (a raster's windows, or refined
+// windows), staged as spec_staged_kernel stages whole windows: one resident CTA per SM walks the
+// blocks, and the next block's sub-window arrives in the tile's last bytes while this one's inverse
+// transform finishes.  ACC (tiles of up to 128 samples, whose summed spectrum fits beside them): a
+// CTA takes all blocks of a pair in turn, adds up their spectra and transforms back once, part
+// holding C^2 floats per pair; else one block at a time, C^2 floats per (pair, block).  The sums and
+// the centring are spec_block_kernel's.  Bounded waits as in spec_staged_kernel; the partial
+// numerators of pairs left out after one ran out are undefined, their maxima still placements.
+// Measured on B200, 3,844 pairs of 128 px chips: the coarse stage (four 128-sample tiles a pair) 2,136
+// us unstaged, 1,910 staged block by block, 1,534 with the spectra summed; the fine stage (four
+// 160-sample tiles, whose 104 KB spectrum fits nowhere beside them) 3,025 -> 2,603 us.
+template <int N1, int N2, bool ACC>
+__global__ void __launch_bounds__(kSpecThreads, 1)
+spec_block_staged_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
+                         int nb, const TileStat* cstat, const float2* tw_g, float* part, double* scal,
+                         unsigned int* errs, const __grid_constant__ CUtensorMap wmap,
+                         const __grid_constant__ CUtensorMap cmap, int raster)
+{
+    extern __shared__ __align__(16) unsigned char ssm[];
+    constexpr int NT = kSpecThreads, NW = NT / 32, N = N1 * N2, RS = N + 1;
+    constexpr int JN = (N + NW - 1) / NW, IN = (N + 31) / 32;
+    constexpr int PJ = 5;  // row groups of a piece read whole before it is written
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int B = g.R, S = g.W, C = g.C, SW = g.stage_rs, K = nb * nb;
+    float2* Z = reinterpret_cast<float2*>(ssm + g.off_z);
+    float2* tw = reinterpret_cast<float2*>(ssm + g.off_tw);
+    int* neg = reinterpret_cast<int*>(ssm + g.off_neg);
+    int* half = reinterpret_cast<int*>(ssm + g.off_half);
+    double* red = reinterpret_cast<double*>(ssm + g.off_red);
+    float2* acc = reinterpret_cast<float2*>(ssm + g.off_gam);
+    float* stage = reinterpret_cast<float*>(ssm + g.off_stage);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(ssm + g.off_bar);
+    int& s_err = *reinterpret_cast<int*>(ssm + g.off_bar + 8);
+    const long long cs = src.chip_stride, ws = src.win_stride;
+    const int jA = g.stage_y0 / NW;
+
+    for (int k = tid; k < N; k += NT) {
+        tw[k] = __ldg(tw_g + k);
+        neg[k] = fft::neg_pos<N1, N2>(k);
+    }
+    if (warp == 0) build_half<N1, N2>(half);
+    if (tid == 0) {
+        s_err = 0;
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    // item n of this CTA: chunk pair b and its block k; false past the end
+    auto item = [&](long long n, long long& b, int& k) {
+        const long long t = ACC ? (blockIdx.x + n / K * gridDim.x) * K + n % K : blockIdx.x + n * gridDim.x;
+        b = t / K;
+        k = (int)(t - b * K);
+        return b < pairs;
+    };
+    // first sample of a block's sub-window and chip block within the pair's window and chip
+    auto corner = [&](int k, int& i0, int& j0) {
+        i0 = k / nb * B;
+        j0 = (k - k / nb * nb) * B;
+    };
+    // thread 0: where the next item's tiles lie, found out early, and their copy (as in
+    // spec_staged_kernel)
+    bool next_ok = false;
+    int nx = 0, ny = 0, nz = 0, ncx = 0, ncy = 0;
+    auto look = [&](long long n) {
+        long long b;
+        int k, i0, j0;
+        item(n, b, k);
+        corner(k, i0, j0);
+        next_ok = valid[pair0 + b] >= 0;
+        if (!next_ok) return;
+        nx = ncx = j0;
+        ny = ncy = i0;
+        nz = (int)b;
+        if (raster) {
+            const long long wo = src.win_off[pair0 + b], co = src.chip_off[pair0 + b];
+            const int wy = (int)(wo / ws), cy = (int)(co / cs);
+            ny += wy;
+            nx += (int)(wo - (long long)wy * ws);
+            ncy += cy;
+            ncx += (int)(co - (long long)cy * cs);
+        }
+    };
+    auto issue = [&]() {
+        if (!next_ok) {
+            mbar_arrive(bar);
+            return;
+        }
+        mbar_expect_tx(bar, (unsigned)S * (unsigned)SW * 4u);
+        if (raster) {
+            tensor_to_smem(stage, &wmap, nx & ~3, ny, bar);
+            tensor_prefetch_l2(&cmap, ncx & ~3, ncy);
+        } else {
+            tensor3_to_smem(stage, &wmap, nx & ~3, ny, nz, bar);
+            tensor3_prefetch_l2(&cmap, ncx & ~3, ncy, nz);
+        }
+    };
+    long long b;
+    int k;
+    bool inflight = item(0, b, k);
+    if (tid == 0 && inflight) {
+        look(0);
+        issue();
+    }
+    uint32_t parity = 0;
+    for (long long n = 0; item(n, b, k); ++n) {
+        const long long p = pair0 + b;
+        const bool ok = valid[p] >= 0;
+        long long bn;
+        int kn, i0, j0;
+        const bool more = item(n + 1, bn, kn);
+        corner(k, i0, j0);
+        const TileStat cst = cstat[b];
+        const float mc_hi = (float)cst.mean, mc_lo = (float)(cst.mean - (double)mc_hi);
+        const bool landed = mbar_wait(bar, parity, &s_err);
+        if (__syncthreads_or(!landed)) break;
+        parity ^= 1u;
+        inflight = false;
+        if (tid == 0 && more) look(n + 1);
+        auto next = [&]() {
+            // the staged bytes are free: the next block's sub-window comes in
+            fence_async_smem();
+            __syncthreads();
+            if (more) {
+                if (tid == 0) issue();
+                inflight = true;
+            }
+        };
+        const bool late = ACC && g.late && k == K - 1;
+        auto early = [&]() {
+            if (!late) next();
+        };
+        if (!ok) {
+            next();
+            continue;
+        }
+        const float* chip = spec_chip(src, pair0, b) + i0 * cs + j0;
+        float cr[JN][IN];
+#pragma unroll
+        for (int j = 0; j < JN; ++j)
+#pragma unroll
+            for (int i = 0; i < IN; ++i) {
+                const int y = warp + NW * j, x = lane + 32 * i;
+                cr[j][i] = y < B && x < B ? (__ldg(chip + y * cs + x) - mc_hi) - mc_lo : 0.0f;
+            }
+        // sub-window sample (y, x) in the staging bytes: the box starts xo samples before it
+        const int xo = raster ? (int)((src.win_off[p] + j0) % ws & 3) : j0 & 3;
+        const float pk = stage[xo];
+        float sw = 0.0f, sw2 = 0.0f;
+        auto put = [&](int j, int i, float t) {
+            const int y = warp + NW * j, x = lane + 32 * i;
+            if (y < N && x < N) {
+                if (y < S && x < S) {
+                    const float d = t - pk;
+                    sw += d;
+                    sw2 = fmaf(d, d, sw2);
+                }
+                Z[y * RS + x] = make_float2(t, cr[j][i]);
+            }
+        };
+        auto staged = [&](int j, int i) {
+            const int y = warp + NW * j, x = lane + 32 * i;
+            return y < S && x < S ? stage[y * SW + xo + x] : 0.0f;
+        };
+        // the tile, as spec_staged_kernel writes it
+#pragma unroll
+        for (int j = 0; j < JN; ++j)
+            if (j < jA)
+#pragma unroll
+                for (int i = 0; i < IN; ++i) put(j, i, staged(j, i));
+        __syncthreads();
+#pragma unroll
+        for (int q0 = 0; q0 < JN; q0 += PJ) {
+            if (q0 + PJ <= jA) continue;
+            float v[PJ][IN];
+#pragma unroll
+            for (int q = 0; q < PJ; ++q)
+#pragma unroll
+                for (int i = 0; i < IN; ++i) v[q][i] = q0 + q < JN && q0 + q >= jA ? staged(q0 + q, i) : 0.0f;
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < PJ; ++q)
+                if (q0 + q < JN && q0 + q >= jA)
+#pragma unroll
+                    for (int i = 0; i < IN; ++i) put(q0 + q, i, v[q][i]);
+        }
+        // FP64 sums over the block (FP32 over a thread's samples of a row): sum c, sum c^2 of the
+        // centred chip block, sum t - k, sum (t - k)^2 of the sub-window
+        double a[4] = {0.0, 0.0, (double)sw, (double)sw2};
+#pragma unroll
+        for (int j = 0; j < JN; ++j)
+            if (warp + NW * j < B) {
+                float c1 = 0.0f, c2 = 0.0f;
+#pragma unroll
+                for (int i = 0; i < IN; ++i) {
+                    c1 += cr[j][i];
+                    c2 = fmaf(cr[j][i], cr[j][i], c2);
+                }
+                a[0] += (double)c1;
+                a[1] += (double)c2;
+            }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            a[q] = warp_sum(a[q]);
+            if (lane == 0) red[4 * warp + q] = a[q];
+        }
+        __syncthreads();
+        double a2 = 0.0, a3 = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) a2 += red[4 * w + 2];
+        const double cells = (double)S * (double)S;
+        const fft::Centre centre{(float)((double)pk + a2 / cells), S};
+        if (tid == 0) {
+            double a0 = 0.0, a1 = 0.0;
+            for (int w = 0; w < NW; ++w) {
+                a0 += red[4 * w];
+                a1 += red[4 * w + 1];
+                a3 += red[4 * w + 3];
+            }
+            const double st = fmax(a3 - a2 * a2 / cells, 0.0) + 1e-5 * a3;
+            double* to = scal + 2 * (b * K + k);
+            to[0] = (double)centre.sx * a0;
+            to[1] = sqrt(a1 * st);
+        }
+        const float scale = (float)(1.0 / (4.0 * (double)N * (double)N));
+        float* out = part + (ACC ? b : b * K + k) * C * C;
+        auto store = [&](int u, int v, float2 val) {
+            if (v < C) out[u * C + v] = val.x * scale;
+        };
+        if constexpr (ACC)
+            fft::correlate_sum<N1, N2, 2>(Z, RS, S, C, tw, neg, half, centre, acc, k == 0, k == K - 1, tid, NT,
+                                          BlockSync{}, store, early);
+        else
+            fft::correlate_tile<N1, N2, 0>(Z, RS, S, C, tw, neg, half, centre, tid, NT, BlockSync{}, store, early);
+        if (late) next();
+    }
+    if (s_err) {
+        if (tid == 0) {
+            atomicAdd(errs, 1u);
+            if (inflight) {
+                const long long t0 = clock64();
+                while (!mbar_try(bar, parity) && clock64() - t0 < kSpinCycles) {
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // One CTA per pair: the sum of the K partial numerators of every placement (FP64, in block order,
 // plus the centring corrections), normalised by the chip's 1/|r'| and the placement's 1/sigma_box,
 // then the direct FP32 recomputation where the transform's bound is loose (spec_surface) and the
-// stage's outputs, as in spec_kernel.  g: the whole stage (R, W, C).  Shared memory: the
+// stage's outputs, as in spec_kernel.  kp: partial surfaces per pair, K, or 1 where the spectra of
+// the blocks were summed.  g: the whole stage (R, W, C).  Shared memory: the
 // placement statistics and the surface (C^2 floats each) and a reduction scratch.
 __global__ void __launch_bounds__(kThreads, 1)
 spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
-                   int K, const TileStat* cstat, InvSource inv, const float* part, const double* scal,
+                   int K, int kp, const TileStat* cstat, InvSource inv, const float* part, const double* scal,
                    SpecOut out)
 {
     extern __shared__ __align__(16) unsigned char ssm[];
@@ -1341,10 +1608,10 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
     float bv = -INFINITY;
     int bi = INT_MAX;
     int flagged = 0;
-    const float* pp = part + (long long)blockIdx.x * K * CC;
+    const float* pp = part + (long long)blockIdx.x * kp * CC;
     for (int idx = tid; idx < CC; idx += kThreads) {
         double num = corr;
-        for (int k = 0; k < K; ++k) num += (double)__ldg(pp + (long long)k * CC + idx);
+        for (int k = 0; k < kp; ++k) num += (double)__ldg(pp + (long long)k * CC + idx);
         const float inv_box = invs[idx];
         const float gv = (float)num * inv_box * inv_sigma;
         G[idx] = gv;
@@ -1577,7 +1844,13 @@ cudaError_t spec_set_smem_limits()
     if (e == cudaSuccess)          \
         e = cudaFuncSetAttribute(spec_staged_kernel<A, B, false, kSpecThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
     if (e == cudaSuccess)          \
-        e = cudaFuncSetAttribute(spec_block_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+        e = cudaFuncSetAttribute(spec_block_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
+    if constexpr (NN <= 128)       \
+        if (e == cudaSuccess)      \
+            e = cudaFuncSetAttribute(spec_block_staged_kernel<A, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
+    if constexpr (NN >= 128)       \
+        if (e == cudaSuccess)      \
+            e = cudaFuncSetAttribute(spec_block_staged_kernel<A, B, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     AMPCOR_SPEC_LENGTHS(AMPCOR_SPEC_CASE)
 #undef AMPCOR_SPEC_CASE
 #define AMPCOR_SPEC_CASE(NN, A, B, NT, CTAS) \
@@ -1640,18 +1913,43 @@ cudaError_t launch_spec_block(const SpecGeom& tile, int nb, unsigned blocks, cud
     return cudaErrorInvalidValue;
 }
 
+cudaError_t launch_spec_block_staged(const SpecGeom& tile, int nb, unsigned sms, cudaStream_t st, SpecSource src,
+                                     long long pair0, long long pairs, const long long* valid,
+                                     const TileStat* cstat, const float2* tw, float* part, double* scal,
+                                     unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster)
+{
+    if (pairs <= 0) return cudaSuccess;
+    const long long units = tile.acc ? pairs : pairs * nb * nb;
+    const unsigned blocks = (unsigned)std::min<long long>(units, std::max(1u, sms));
+    auto run = [&](auto kernel) {
+        kernel<<<blocks, kSpecThreads, tile.smem_staged, st>>>(src, pair0, pairs, valid, tile, nb, cstat, tw, part,
+                                                               scal, errs, *wmap, *cmap, raster);
+        return cudaGetLastError();
+    };
+#define AMPCOR_SPEC_CASE(NN, A, B)                                                          \
+    if (tile.N == NN) {                                                                     \
+        if constexpr (NN <= 128)                                                            \
+            if (tile.acc) return run(spec_block_staged_kernel<A, B, true>);                 \
+        if constexpr (NN >= 128)                                                            \
+            if (!tile.acc) return run(spec_block_staged_kernel<A, B, false>);               \
+    }
+    AMPCOR_SPEC_LENGTHS(AMPCOR_SPEC_CASE)
+#undef AMPCOR_SPEC_CASE
+    return cudaErrorInvalidValue;
+}
+
 int spec_reduce_smem(int C)
 {
     return 2 * ((C * C + 3) & ~3) * 4 + 256;
 }
 
-cudaError_t launch_spec_reduce(const SpecGeom& full, int K, unsigned blocks, cudaStream_t st,
+cudaError_t launch_spec_reduce(const SpecGeom& full, int K, int kp, unsigned blocks, cudaStream_t st,
                                SpecSource src, long long pair0, long long pairs,
                                const long long* valid, const TileStat* cstat, InvSource inv,
                                const float* part, const double* scal, SpecOut out)
 {
     spec_reduce_kernel<<<blocks, kThreads, spec_reduce_smem(full.C), st>>>(src, pair0, pairs, valid, full, K,
-                                                                           cstat, inv, part, scal, out);
+                                                                           kp, cstat, inv, part, scal, out);
     return cudaGetLastError();
 }
 
