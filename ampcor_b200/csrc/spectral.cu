@@ -1591,9 +1591,11 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
     double* red = reinterpret_cast<double*>(G + ((CC + 3) & ~3));
     const float* inv_b = inv.off ? inv.base + inv.off[p] : inv.base + (long long)blockIdx.x * CC;
     const long long is = inv.off ? inv.stride : C;
-    for (int idx = tid; idx < CC; idx += kThreads) {
-        const int u = idx / C, v = idx - u * C;
-        invs[idx] = __ldg(inv_b + u * is + v);
+    {
+        const int warp = tid >> 5, lane = tid & 31;
+        for (int u = warp; u < C; u += kWarps)
+#pragma unroll 4
+            for (int v = lane; v < C; v += 32) cp_async4(invs + u * C + v, inv_b + u * is + v);
     }
     const double* sc = scal + 2 * (long long)blockIdx.x * K;
     double corr = 0.0, errs = 0.0;
@@ -1604,21 +1606,46 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
     const TileStat cst = cstat[blockIdx.x];
     const float inv_sigma = (float)cst.inv_norm;
     const float ebox = kSpecErr * (float)errs * inv_sigma;
+    cp_async_wait_all();
     __syncthreads();
     float bv = -INFINITY;
     int bi = INT_MAX;
     int flagged = 0;
     const float* pp = part + (long long)blockIdx.x * kp * CC;
-    for (int idx = tid; idx < CC; idx += kThreads) {
-        double num = corr;
-        for (int k = 0; k < kp; ++k) num += (double)__ldg(pp + (long long)k * CC + idx);
-        const float inv_box = invs[idx];
-        const float gv = (float)num * inv_box * inv_sigma;
-        G[idx] = gv;
-        if (ebox * inv_box > kSpecTol)
-            flagged = 1;
-        else
-            better(bv, bi, gv, idx);
+    // a batch of placements and blocks in flight per thread (one load after the other, 33 placements of
+    // four blocks a thread, kept a +-64 px search waiting: 246 -> 182 us for 900 pairs)
+    constexpr int kPlace = 4, kBlocks = 4;
+    for (int idx0 = tid; idx0 < CC; idx0 += kPlace * kThreads) {
+        double num[kPlace];
+#pragma unroll
+        for (int q = 0; q < kPlace; ++q) num[q] = corr;
+        for (int k0 = 0; k0 < kp; k0 += kBlocks) {
+            float v[kPlace][kBlocks];
+#pragma unroll
+            for (int q = 0; q < kPlace; ++q)
+#pragma unroll
+                for (int k = 0; k < kBlocks; ++k)
+                    v[q][k] = idx0 + q * kThreads < CC && k0 + k < kp
+                                  ? __ldg(pp + (long long)(k0 + k) * CC + idx0 + q * kThreads)
+                                  : 0.0f;
+#pragma unroll
+            for (int q = 0; q < kPlace; ++q)
+#pragma unroll
+                for (int k = 0; k < kBlocks; ++k)
+                    if (k0 + k < kp) num[q] += (double)v[q][k];
+        }
+#pragma unroll
+        for (int q = 0; q < kPlace; ++q) {
+            const int idx = idx0 + q * kThreads;
+            if (idx >= CC) break;
+            const float inv_box = invs[idx];
+            const float gv = (float)num[q] * inv_box * inv_sigma;
+            G[idx] = gv;
+            if (ebox * inv_box > kSpecTol)
+                flagged = 1;
+            else
+                better(bv, bi, gv, idx);
+        }
     }
     __syncthreads();
     const float* chip = spec_chip(src, pair0, blockIdx.x);

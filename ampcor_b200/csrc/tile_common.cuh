@@ -142,24 +142,46 @@ __device__ void window_stats_xs(const float* win, int S, int W, int R, int C, in
     double* V2 = vbuf + SR * (W + 1);
     double s1 = 0.0, s2 = 0.0;
     if (tid < W) {
-        for (int i = 0; i < R; ++i) {
-            const double t = win[i * S + tid * XS];
-            s1 += t;
-            s2 += t * t;
+        // (a batch of loads in flight: 256 rows of a refined window, one after the other, were most of
+        // spec_tile_stats_kernel's time)
+        constexpr int kBatch = 16;
+        for (int i0 = 0; i0 < R; i0 += kBatch) {
+            float v[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) v[k] = win[min(i0 + k, R - 1) * S + tid * XS];
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k)
+                if (i0 + k < R) {
+                    const double t = v[k];
+                    s1 += t;
+                    s2 += t * t;
+                }
         }
     }
     const double cells = (double)R * (double)R;
     for (int u0 = 0; u0 < C; u0 += SR) {
         const int nrows = min(SR, C - u0);
         if (tid < W) {
-            for (int r = 0; r < nrows; ++r) {
-                const int u = u0 + r;
-                V1[r * (W + 1) + tid] = s1;
-                V2[r * (W + 1) + tid] = s2;
-                if (u + 1 < C) {
-                    const double a = win[(u + R) * S + tid * XS], b = win[u * S + tid * XS];
-                    s1 += a - b;
-                    s2 += a * a - b * b;
+            constexpr int kBatch = 8;
+            for (int r0 = 0; r0 < nrows; r0 += kBatch) {
+                float va[kBatch], vb[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    const int u = max(min(u0 + r0 + k, C - 2), 0);
+                    va[k] = win[min(u + R, W - 1) * S + tid * XS];
+                    vb[k] = win[u * S + tid * XS];
+                }
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    const int r = r0 + k, u = u0 + r;
+                    if (r >= nrows) break;
+                    V1[r * (W + 1) + tid] = s1;
+                    V2[r * (W + 1) + tid] = s2;
+                    if (u + 1 < C) {
+                        const double a = va[k], b = vb[k];
+                        s1 += a - b;
+                        s2 += a * a - b * b;
+                    }
                 }
             }
         }
