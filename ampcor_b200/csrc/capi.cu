@@ -613,6 +613,7 @@ struct ampcor_handle {
     size_t chunk = 0;      // pairs per chunk
     size_t chunk_cap = 0;  // pairs the scratch holds: the chunk, or all of a smaller job
     size_t chunk_override = 0;
+    bool chunk_short = false;  // the default chunk's scratch did not fit: one wave instead
     long long refined_stride = 0;
     // host-path staging
     void* d_ref_raster = nullptr;
@@ -742,12 +743,27 @@ int ensure_pairs(ampcor_handle* h, size_t pairs)
     return AMPCOR_OK;
 }
 
+// partial numerators, their scalars (blocks) and placement statistics (cells) of a pair in the blocked
+// stages
+void blocked_scratch(const ampcor_handle* h, size_t& parts, size_t& blocks, size_t& cells)
+{
+    parts = blocks = cells = 0;
+    if (h->form != kFormSpectral) return;
+    for (const auto& s : {std::make_pair(&h->bc, (size_t)h->C), std::make_pair(&h->bf, (size_t)h->Cf)}) {
+        if (!s.first->on) continue;
+        blocks = std::max(blocks, (size_t)s.first->K);
+        parts = std::max(parts, (size_t)s.first->K * s.second * s.second);
+        cells = std::max(cells, s.second * s.second);
+    }
+}
+
+constexpr size_t kChunkWave = 148 * 4;  // pairs: four to a multiprocessor
+
 // The chunk of pairs whose refined amplitudes are resident at once, unless configured or set by
-// AMPCOR_CHUNK: as many waves of 592 pairs (four to a multiprocessor) as keep the scratch of a pair
-// (refined amplitudes and surface) within half a gigabyte in all, at least one.  Each chunk costs
-// five launches whose last waves leave multiprocessors idle, and reading the refined tiles from HBM
-// instead of L2 costs less than that: 23,625 pairs of 32 px chips in 40 chunks of 592 take 5.38 ms,
-// in 3 chunks 4.07 ms; the scratch of a worker is what bounds the chunk.
+// AMPCOR_CHUNK: as many waves as keep the scratch of all their pairs within a gigabyte, at least
+// one.  Each chunk costs five launches whose last waves leave multiprocessors idle, and reading the
+// refined tiles from HBM instead of L2 costs less than that: 23,625 pairs of 32 px chips in 40
+// chunks of 592 take 5.38 ms, in 3 chunks 4.07 ms; the scratch of a worker is what bounds the chunk.
 size_t default_chunk(const ampcor_handle* h)
 {
     const char* env = std::getenv("AMPCOR_CHUNK");
@@ -755,9 +771,13 @@ size_t default_chunk(const ampcor_handle* h)
         long v = std::strtol(env, nullptr, 10);
         if (v > 0) return (size_t)v;
     }
-    const size_t pair = ((size_t)h->Rf * h->Rf + (size_t)h->Wf * h->Wf + (size_t)h->Cf * h->Cf) * sizeof(float);
-    const size_t wave = 148 * 4;
-    return std::max<size_t>(1, (size_t)512 * 1024 * 1024 / (pair * wave)) * wave;
+    if (h->chunk_short) return kChunkWave;
+    size_t parts, blocks, cells;
+    blocked_scratch(h, parts, blocks, cells);
+    const size_t tiles = (size_t)h->Rf * h->Rf + (size_t)h->Wf * h->Wf + (size_t)h->Cf * h->Cf;
+    const size_t stats = h->form == kFormTensor ? (size_t)h->C * h->C + (size_t)h->Cf * h->Cf : 0;
+    const size_t pair = (tiles + stats + parts + cells) * sizeof(float) + blocks * 2 * sizeof(double);
+    return std::max<size_t>(1, ((size_t)1 << 30) / (pair * kChunkWave)) * kChunkWave;
 }
 
 void free_chunk_scratch(ampcor_handle* h)
@@ -788,13 +808,9 @@ int scratch_fail(ampcor_handle* h, const std::string& what)
     return fail(h, AMPCOR_E_NOMEM, what);
 }
 
-// the scratch of a job of `pairs` pairs: a chunk's, or less where the job is smaller
-int ensure_refined(ampcor_handle* h, size_t pairs)
+// the scratch of n pairs
+int alloc_chunk_scratch(ampcor_handle* h, size_t n)
 {
-    h->chunk = h->chunk_override ? h->chunk_override : default_chunk(h);
-    const size_t n = std::min(h->chunk, std::max<size_t>(pairs, 1));
-    if (h->d_refined && h->chunk_cap >= n) return AMPCOR_OK;
-    free_chunk_scratch(h);
     h->refined_stride = (long long)h->Rf * h->Rf + (long long)h->Wf * h->Wf;
     // 16 floats of slack: staged copies round rows out to 16-byte boundaries
     cudaError_t e = cudaMalloc(&h->d_refined, (n * h->refined_stride + 16) * sizeof(float));
@@ -813,17 +829,31 @@ int ensure_refined(ampcor_handle* h, size_t pairs)
         return scratch_fail(h, "allocating refined-surface scratch");
     if (h->form == kFormSpectral && cudaMalloc(&h->d_tstat, 3 * n * sizeof(TileStat)) != cudaSuccess)
         return scratch_fail(h, "allocating tile statistics");
-    if (h->form == kFormSpectral && (h->bc.on || h->bf.on)) {
-        const size_t K = (size_t)std::max(h->bc.on ? h->bc.K : 0, h->bf.on ? h->bf.K : 0);
-        const size_t parts = std::max(h->bc.on ? (size_t)h->bc.K * h->C * h->C : 0,
-                                      h->bf.on ? (size_t)h->bf.K * h->Cf * h->Cf : 0);
-        const size_t cells = std::max(h->bc.on ? (size_t)h->C * h->C : 0, h->bf.on ? (size_t)h->Cf * h->Cf : 0);
-        if (cudaMalloc(&h->d_inv_blk, n * cells * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&h->d_part, n * parts * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&h->d_scal, n * K * 2 * sizeof(double)) != cudaSuccess)
-            return scratch_fail(h, "allocating blocked-correlation scratch");
-    }
+    size_t parts, blocks, cells;
+    blocked_scratch(h, parts, blocks, cells);
+    if (blocks && (cudaMalloc(&h->d_inv_blk, n * cells * sizeof(float)) != cudaSuccess ||
+                   cudaMalloc(&h->d_part, n * parts * sizeof(float)) != cudaSuccess ||
+                   cudaMalloc(&h->d_scal, n * blocks * 2 * sizeof(double)) != cudaSuccess))
+        return scratch_fail(h, "allocating blocked-correlation scratch");
     return AMPCOR_OK;
+}
+
+// The scratch of a job whose pairs the worker is sized for (ensure_pairs): a chunk's, or less where
+// the worker's largest job is smaller, so that a smaller job does not leave a later one short.  A
+// default chunk of several waves that the device cannot hold beside the caller's data gives way
+// to one wave, for good: no later call tries again.
+int ensure_refined(ampcor_handle* h)
+{
+    const bool chosen = h->chunk_override || std::getenv("AMPCOR_CHUNK");
+    for (;;) {
+        h->chunk = h->chunk_override ? h->chunk_override : default_chunk(h);
+        const size_t n = std::min(h->chunk, std::max<size_t>(h->cap, 1));
+        if (h->d_refined && h->chunk_cap >= n) return AMPCOR_OK;
+        free_chunk_scratch(h);
+        const int rc = alloc_chunk_scratch(h, n);
+        if (rc != AMPCOR_E_NOMEM || chosen || n <= kChunkWave) return rc;
+        h->chunk_short = true;
+    }
 }
 
 
@@ -863,7 +893,7 @@ int run_plain(ampcor_handle* h, const PairSource& src, long long pairs, float2* 
               PairDiag* diag, float* coarse_surfaces, float* refined_surfaces, cudaStream_t st)
 {
     if (pairs == 0) return AMPCOR_OK;
-    int rc = ensure_refined(h, (size_t)pairs);
+    int rc = ensure_refined(h);
     if (rc) return rc;
     cudaEvent_t a = mark(h, st);
     coarse_kernel<<<(unsigned)pairs, kThreads, h->gc.smem_bytes, st>>>(
@@ -922,7 +952,7 @@ int run_tensor(ampcor_handle* h, const PairSource& src, long long pairs, float2*
                PairDiag* diag, float* coarse_surfaces, float* refined_surfaces, cudaStream_t st)
 {
     if (pairs == 0) return AMPCOR_OK;
-    int rc = ensure_refined(h, (size_t)pairs);
+    int rc = ensure_refined(h);
     if (rc) return rc;
     if ((rc = ensure_fine_out(h, (size_t)pairs))) return rc;
     const RealTiles rt{h->d_refined, h->refined_stride, 0, (long long)h->Rf * h->Rf};
@@ -1026,7 +1056,7 @@ bool tiles_map(CUtensorMap& m, const float* base, int n, long long pairs, long l
 
 int spec_rasters(ampcor_handle* h, const PairSource& src, long long pairs, SpecRasters& r)
 {
-    int rc = ensure_refined(h, (size_t)pairs);
+    int rc = ensure_refined(h);
     if (rc) return rc;
     if ((rc = ensure_fine_out(h, (size_t)pairs))) return rc;
     r.shared = src.ref_base == src.tgt_base;
