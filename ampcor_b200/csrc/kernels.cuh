@@ -176,10 +176,11 @@ __global__ void tc_fine_kernel(RealTiles t, long long pair0, long long pairs, Tc
                                const float* inv, const long long* ref_off, FineOut* fout,
                                float* gam, float* surfaces, unsigned int* err);
 
-// the zoom of the refined surfaces (zoom_kernel): teams of kZoomTeam threads, a pair each, at most
-// kZoomTeams to a CTA, kZoomCols columns of the zoomed surface at a time
+// the zoom of the refined surfaces (zoom_kernel): teams of kZoomTeam threads (or three times as many),
+// a pair each, at most kZoomTeams (3) to a CTA, kZoomCols columns of the zoomed surface at a time
 constexpr int kZoomTeam = 96;
 constexpr int kZoomTeams = 8;
+constexpr int zoom_teams(int groups) { return groups == 1 ? kZoomTeams : 3; }
 constexpr int kZoomCols = 36;
 
 struct ZoomGeomCols {

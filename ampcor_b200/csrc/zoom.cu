@@ -19,8 +19,8 @@
 // of the production surface remain; noise keeps everything, at the cost of the whole product, and
 // so does NaN (comparisons are written to keep it).
 //
-// What bounds it: the FP32 pipes and instruction issue.  A team of three warps walks one pair at a
-// time; the lanes of a warp are 8 rows of U x 4 rows of the other factor, a thread three of the
+// What bounds it: the FP32 pipes and instruction issue.  A team of three warps (nine where
+// a multiprocessor has few pairs) walks one pair at a time; the lanes of a warp are 8 rows of U x 4 rows of the other factor, a thread three of the
 // former against three of the latter: 18 packed FMAs per six 128-bit shared loads of one
 // wavefront each (four rows a thread leave a third of the lanes idle over the 66 sampled rows: 364
 // against 317 us below).  The teams of a CTA (one CTA per SM) share U and nothing else, so one
@@ -39,12 +39,12 @@ namespace ampcor_b200 {
 
 namespace {
 
-constexpr int kTeam = kZoomTeam;  // threads of a team
 constexpr int kCols = kZoomCols;
 
+template <int TEAM>
 __device__ __forceinline__ void team_sync(int team)
 {
-    asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeam) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(TEAM) : "memory");
 }
 
 // acc += a * b on two packed floats
@@ -60,7 +60,8 @@ __device__ __forceinline__ float halves(unsigned long long v)
 
 constexpr int kNR = 3, kNC = 3;      // rows of U and of the other factor per thread
 constexpr int kRows = 8 * kNR;       // rows a warp forms at a time: its lanes are 8 rows x 4 columns
-constexpr int kStep = kTeam / 32 * kRows;
+constexpr int kGroup = kZoomTeam / 32;  // warps of a group: they share out the rows
+constexpr int kStep = kGroup * kRows;
 static_assert(kCols % (4 * kNC) == 0, "a batch is whole blocks of columns");
 
 // out[i][k] = row ra[i] of U times row rb + 4 k of b (rows of kp4 float4, zero past Cf); kp4 is odd,
@@ -103,8 +104,8 @@ __device__ __forceinline__ void dots(const float* U, const int (&ra)[kNR], const
 struct ZoomTeam {
     float* G;             // g_rows rows of kp4 float4, zero past Cf
     float* T;             // kCols kept columns of T, kp4 float4 each
-    float* val;           // J: the norms of T's sampled columns, then the maxima of the sampled rows
-    float* red;           // 16
+    float* val;           // J a group: the norms of T's sampled columns, then the maxima of the sampled rows
+    float* red;           // a slot per warp, four times (16 or 32 in all), the last one after them
     unsigned* cols;       // Z: the kept columns, index | row of U << 16
     unsigned* rows;       // Z: the kept rows, the same
 };
@@ -135,6 +136,7 @@ __device__ __forceinline__ int kept_intervals(const float* val, const ZoomGeomCo
 }
 
 // the maximum over a team of (value, index), ends with a barrier; every thread gets it
+template <int TEAM>
 __device__ __forceinline__ void team_argmax(float& bv, int& bi, float* red, int team, int tid)
 {
 #pragma unroll
@@ -143,25 +145,29 @@ __device__ __forceinline__ void team_argmax(float& bv, int& bi, float* red, int 
         const int oi = __shfl_xor_sync(kFull, bi, o);
         better(bv, bi, ov, oi);
     }
+    constexpr int kWarpsT = TEAM / 32;
     if ((tid & 31) == 0) {
         red[tid >> 5] = bv;
-        reinterpret_cast<int*>(red)[4 + (tid >> 5)] = bi;
+        reinterpret_cast<int*>(red)[kWarpsT + (tid >> 5)] = bi;
     }
-    team_sync(team);
+    team_sync<TEAM>(team);
 #pragma unroll
-    for (int w = 0; w < kTeam / 32; ++w) better(bv, bi, red[w], reinterpret_cast<int*>(red)[4 + w]);
-    team_sync(team);
+    for (int w = 0; w < kWarpsT; ++w) better(bv, bi, red[w], reinterpret_cast<int*>(red)[kWarpsT + w]);
+    team_sync<TEAM>(team);
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(kZoomTeams * kZoomTeam, 1)
+// GROUPS groups of three warps to a team: they share out the columns of a product
+template <int GROUPS>
+__global__ void __launch_bounds__(zoom_teams(GROUPS) * GROUPS * kZoomTeam, 1)
 zoom_kernel(const float* gam, long long pair0, long long pairs, const long long* ref_off, ZoomGeomCols g,
             const float* u_g, const CoarseOut* coarse, const float* coarse_peak, const FineOut* fout, int margin,
             int refine_factor, int refine_margin, int ref_compat, float2* offsets, PairDiag* diag,
             unsigned int* err_out, int stall)
 {
     extern __shared__ __align__(16) unsigned char zsm[];
+    constexpr int kTeam = GROUPS * kZoomTeam, kWarpsT = kTeam / 32, kTotal = 4 * kWarpsT;
     const int team = threadIdx.x / kTeam, tid = threadIdx.x - team * kTeam, teams = blockDim.x / kTeam;
     const int Cf = g.Cf, Z = g.Z, kp4 = g.kp4;
     float* U = reinterpret_cast<float*>(zsm);
@@ -170,10 +176,12 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
     t.G = reinterpret_cast<float*>(own);
     t.T = t.G + g.g_rows * 4 * kp4;
     t.val = t.T + kCols * 4 * kp4;
-    t.red = t.val + (g.J + 3) / 4 * 4;
-    t.cols = reinterpret_cast<unsigned*>(t.red + 16);
+    const int Jv = (g.J + 3) / 4 * 4;
+    t.red = t.val + GROUPS * Jv;
+    t.cols = reinterpret_cast<unsigned*>(t.red + (kTotal + 4) / 4 * 4);
     t.rows = t.cols + (Z + 3) / 4 * 4;
     const int lane = tid & 31, warp = tid >> 5, rl = lane >> 2, cl = lane & 3;
+    const int grp = warp / kGroup, wrow = (warp - grp * kGroup) * kRows;  // this warp's share: columns, rows
     // element tid of a row-major array of Cf columns, and the one kTeam further on
     const int ta0 = tid / Cf, tq0 = tid - ta0 * Cf, da = kTeam / Cf, dq = kTeam - da * Cf;
     auto walk = [&](int& a, int& q) {
@@ -220,7 +228,7 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
         float g1 = 0.0f, g2 = 0.0f;
         {
             // (row, column) of this thread's samples walk along by kTeam; a batch of loads in flight
-            constexpr int kLoads = 12;
+            constexpr int kLoads = 12 / GROUPS;
             int a = ta0, q = tq0;
             for (int i0 = tid; i0 < Cf * Cf; i0 += kLoads * kTeam) {
                 float gv[kLoads];
@@ -244,14 +252,14 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
         }
         if (lane == 0) {
             t.red[warp] = g1;
-            t.red[4 + warp] = g2;
+            t.red[kWarpsT + warp] = g2;
         }
-        team_sync(team);
+        team_sync<kTeam>(team);
         g1 = g2 = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kTeam / 32; ++w) {
+        for (int w = 0; w < kWarpsT; ++w) {
             g1 += t.red[w];
-            g2 += t.red[4 + w];
+            g2 += t.red[kWarpsT + w];
         }
         // the constant c, and |G - c| from above (the slack covers the FP32 sums)
         const float c = g1 / (float)(Cf * Cf);
@@ -259,7 +267,7 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
 
         // T at every s-th column: the largest entry, the norm of every column
         float best = -INFINITY;
-        for (int j0 = warp * kRows; j0 < g.J; j0 += kStep) {
+        for (int j0 = wrow; j0 < g.J; j0 += kStep) {
             int q[kNR];
             float nn[kNR];
 #pragma unroll
@@ -267,7 +275,7 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
                 q[i] = min(j0 + rl + 8 * i, g.J - 1);
                 nn[i] = 0.0f;
             }
-            for (int a = 0; a < Cf; a += 4 * kNC) {
+            for (int a = 4 * kNC * grp; a < Cf; a += 4 * kNC * GROUPS) {
                 float v[kNR][kNC];
                 dots(U, q, t.G, a + cl, kp4, v);
 #pragma unroll
@@ -284,27 +292,36 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
             for (int i = 0; i < kNR; ++i) {
                 nn[i] += __shfl_xor_sync(kFull, nn[i], 1);
                 nn[i] += __shfl_xor_sync(kFull, nn[i], 2);
-                if (cl == i && j0 + rl + 8 * i < g.J) t.val[j0 + rl + 8 * i] = sqrtf(nn[i]);
+                if (cl == i && j0 + rl + 8 * i < g.J) t.val[grp * Jv + j0 + rl + 8 * i] = GROUPS == 1 ? sqrtf(nn[i]) : nn[i];
             }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(kFull, best, o));
-        if (lane == 0) t.red[8 + warp] = best;
-        team_sync(team);
+        if (lane == 0) t.red[2 * kWarpsT + warp] = best;
+        team_sync<kTeam>(team);
+        if constexpr (GROUPS > 1) {
+            for (int j = tid; j < g.J; j += kTeam) {
+                float n2 = 0.0f;
+#pragma unroll
+                for (int i = 0; i < GROUPS; ++i) n2 += t.val[i * Jv + j];
+                t.val[j] = sqrtf(n2);
+            }
+            team_sync<kTeam>(team);
+        }
         float top = 0.0f;  // the largest norm
         for (int j = lane; j < g.J; j += 32) top = fmaxf(top, t.val[j]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(kFull, top, o));
 #pragma unroll
-        for (int w = 0; w < kTeam / 32; ++w) best = fmaxf(best, t.red[8 + w]);
+        for (int w = 0; w < kWarpsT; ++w) best = fmaxf(best, t.red[2 * kWarpsT + w]);
         const float slack = 1e-4f * (gn + fabsf(c)) + 1e-6f;
         // (warp 0 writes the list, its length goes through the reduction slots)
         if (warp == 0) {
             const int n = kept_intervals(t.val, g, c + g.curv * gn + slack, best, true, t.cols);
-            if (lane == 0) reinterpret_cast<int*>(t.red)[12] = n;
+            if (lane == 0) reinterpret_cast<int*>(t.red)[kTotal] = n;
         }
-        team_sync(team);
-        const int total = reinterpret_cast<int*>(t.red)[12];
+        team_sync<kTeam>(team);
+        const int total = reinterpret_cast<int*>(t.red)[kTotal];
         const float rise = g.curv * (top + g.curv * gn) + slack;  // of a kept column between two rows
 
         float bv = -INFINITY;
@@ -314,7 +331,7 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
         auto cells = [&](const int (&ra)[kNR], const int (&pa)[kNR], int c0, int nb, float (&rm)[kNR]) {
 #pragma unroll
             for (int i = 0; i < kNR; ++i) rm[i] = -INFINITY;
-            for (int s = 0; s < nb; s += 4 * kNC) {
+            for (int s = 4 * kNC * grp; s < nb; s += 4 * kNC * GROUPS) {
                 float v[kNR][kNC];
                 dots(U, ra, t.T, s + cl, kp4, v);
 #pragma unroll
@@ -351,9 +368,9 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
                 for (int r = 0; r < 3; ++r)
                     if (a + r * nt < Cf) t.T[q * 4 * kp4 + a + r * nt] = halves(acc[r]);
             }
-            team_sync(team);
+            team_sync<kTeam>(team);
             // every s-th row
-            for (int j0 = warp * kRows; j0 < g.J; j0 += kStep) {
+            for (int j0 = wrow; j0 < g.J; j0 += kStep) {
                 int ra[kNR], pa[kNR];
                 float rm[kNR];
 #pragma unroll
@@ -366,10 +383,19 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
                 for (int i = 0; i < kNR; ++i) {
                     rm[i] = fmaxf(rm[i], __shfl_xor_sync(kFull, rm[i], 1));
                     rm[i] = fmaxf(rm[i], __shfl_xor_sync(kFull, rm[i], 2));
-                    if (cl == i && j0 + rl + 8 * i < g.J) t.val[j0 + rl + 8 * i] = rm[i];
+                    if (cl == i && j0 + rl + 8 * i < g.J) t.val[grp * Jv + j0 + rl + 8 * i] = rm[i];
                 }
             }
-            team_sync(team);
+            team_sync<kTeam>(team);
+            if constexpr (GROUPS > 1) {
+                for (int j = tid; j < g.J; j += kTeam) {
+                    float m = t.val[j];
+#pragma unroll
+                    for (int i = 1; i < GROUPS; ++i) m = fmaxf(m, t.val[i * Jv + j]);
+                    t.val[j] = m;
+                }
+                team_sync<kTeam>(team);
+            }
             // the rows between them that can hold more than the largest cell seen
             if (warp == 0) {
                 float seen = best;
@@ -377,11 +403,11 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) seen = fmaxf(seen, __shfl_xor_sync(kFull, seen, o));
                 const int n = kept_intervals(t.val, g, rise, seen, false, t.rows);
-                if (lane == 0) reinterpret_cast<int*>(t.red)[12] = n;
+                if (lane == 0) reinterpret_cast<int*>(t.red)[kTotal] = n;
             }
-            team_sync(team);
-            const int nr = reinterpret_cast<int*>(t.red)[12];
-            for (int r0 = warp * kRows; r0 < nr; r0 += kStep) {
+            team_sync<kTeam>(team);
+            const int nr = reinterpret_cast<int*>(t.red)[kTotal];
+            for (int r0 = wrow; r0 < nr; r0 += kStep) {
                 int ra[kNR], pa[kNR];
                 float rm[kNR];
 #pragma unroll
@@ -392,9 +418,9 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
                 }
                 cells(ra, pa, c0, nb, rm);
             }
-            team_sync(team);
+            team_sync<kTeam>(team);
         }
-        team_argmax(bv, bi, t.red, team, tid);
+        team_argmax<kTeam>(bv, bi, t.red, team, tid);
         if (tid == 0) {
             const CoarseOut co = coarse[p];
             const FineOut fo = fout[p];
@@ -421,7 +447,9 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
 cudaError_t zoom_set_smem_limits()
 {
     const int limit = 227 * 1024;
-    return cudaFuncSetAttribute(zoom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    cudaError_t e = cudaFuncSetAttribute(zoom_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(zoom_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    return e;
 }
 
 cudaError_t launch_zoom_kernel(unsigned sms, cudaStream_t st, const float* gam, long long pair0, unsigned n,
@@ -431,11 +459,24 @@ cudaError_t launch_zoom_kernel(unsigned sms, cudaStream_t st, const float* gam, 
                                PairDiag* diag, unsigned int* err_out, int stall)
 {
     // as many teams to a CTA as keep every multiprocessor busy
-    const unsigned teams = std::min<unsigned>((unsigned)g.teams, (n + sms - 1) / sms);
-    const unsigned blocks = std::min<unsigned>((n + teams - 1) / teams, sms);
-    zoom_kernel<<<blocks, teams * kZoomTeam, g.off_team + teams * g.team_bytes, st>>>(
-        gam, pair0, n, ref_off, g, u, coarse, coarse_peak, fout, margin, refine_factor, refine_margin, ref_compat,
-        offsets, diag, err_out, stall);
+    const unsigned each = (n + sms - 1) / sms;
+    auto launch = [&](auto* kernel, ZoomGeomCols gg, unsigned fit, int threads) {
+        const unsigned teams = std::min(fit, each), blocks = std::min<unsigned>((n + teams - 1) / teams, sms);
+        kernel<<<blocks, teams * threads, gg.off_team + teams * gg.team_bytes, st>>>(
+            gam, pair0, n, ref_off, gg, u, coarse, coarse_peak, fout, margin, refine_factor, refine_margin,
+            ref_compat, offsets, diag, err_out, stall);
+    };
+    // Three groups to a team where a multiprocessor has few pairs: a pair's chain of products is what such
+    // a call waits for.  225 surfaces of 33 x 33 at z = 8: 24.2 -> 20.5 us, of noise 127 -> 92 (z = 16: 32.4 ->
+    // 24.5, 310 -> 201); 444 surfaces, three to a multiprocessor, 25.9 -> 22.6, but 17 x 17 samples have
+    // too few rows for that: 14.3 -> 16.3.
+    ZoomGeomCols wide = g;
+    wide.team_bytes += 2 * ((g.J + 3) / 4 * 4) * 4 + 96;
+    const unsigned fit = (unsigned)std::min<long>(g.J > 48 ? zoom_teams(3) : 2, (227L * 1024 - g.off_team) / wide.team_bytes);
+    if (each <= fit)
+        launch(zoom_kernel<3>, wide, fit, 3 * kZoomTeam);
+    else
+        launch(zoom_kernel<1>, g, (unsigned)g.teams, kZoomTeam);
     return cudaGetLastError();
 }
 

@@ -54,3 +54,26 @@ def test_zoom_maximum(m, z, kind):
     np.testing.assert_array_equal(off[:, 0], d["top"] - 16 + d["fine_p"] / np.float32(2 * z))
     np.testing.assert_array_equal(off[:, 1], d["left"] - 16 + d["fine_q"] / np.float32(2 * z))
     worker.close()
+
+
+@pytest.mark.parametrize("kind", ["peak", "noise"])
+# one, two, three and four pairs to a multiprocessor: teams of nine warps, then of three
+@pytest.mark.parametrize("m,z", [(4, 4), (8, 8), (8, 16)])
+def test_zoom_teams_agree(m, z, kind):
+    ref, tgt = rasters(kind)
+    ulhc = np.array([[y + 16, x + 16, y, x] for y in range(0, 236, 59) for x in range(0, 236, 47)], np.int32)
+    P, dev = len(ulhc), torch.device("cuda:0")
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    got = []
+    for n in (P, 2 * sms, 2 * sms + 1, 3 * sms, 3 * sms + 1):
+        many = np.ascontiguousarray(np.resize(ulhc, (n, 4)))
+        worker = Worker(n, (32, 32), (64, 64), refine_factor=2, refine_margin=m, zoom_factor=z)
+        diag = torch.zeros((n, DIAG_DTYPE.itemsize), dtype=torch.uint8, device=dev)
+        worker.correlate(torch.from_numpy(ref).to(dev), torch.from_numpy(tgt).to(dev), torch.from_numpy(many).to(dev),
+                         diag=diag)
+        d = diag.cpu().numpy()
+        np.testing.assert_array_equal(d, d[np.arange(n) % P])
+        got.append(d[:P])
+        worker.close()
+    for d in got[1:]:
+        np.testing.assert_array_equal(d, got[0])
