@@ -20,7 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 HOST_CC = "/usr/bin/gcc"
 
-CUDA_SOURCES = ["kernels.cu", "tc_ncc.cu", "zoom.cu", "spectral.cu", "refine_fft.cu", "capi.cu"]
+CUDA_SOURCES = ["kernels.cu", "tc_ncc.cu", "zoom.cu", "raster_stats.cu", "spectral.cu", "refine_fft.cu", "capi.cu"]
 CUDA_HEADERS = ["kernels.cuh", "tile_common.cuh", "fft.cuh", "tcgen05.cuh", os.path.join("..", "..", "include", "ampcor_b200.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

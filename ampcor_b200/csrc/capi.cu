@@ -657,8 +657,6 @@ struct ampcor_handle {
     // box statistics of the secondary raster (FP64 column sums, 1/sigma of every box)
     float* d_amp = nullptr;
     size_t amp_cap = 0;
-    double* d_vsum = nullptr;
-    size_t vsum_cap = 0;
     float* d_inv_raster = nullptr;
     size_t inv_raster_cap = 0;
     // tensor-core form
@@ -996,7 +994,7 @@ struct SpecRasters {
     bool shared = false;        // one raster holds chips and windows
     bool raster_stats = false;  // coarse box statistics once per raster, else inside the kernel
     long long rows = 0;         // box rows of the secondary raster (tgt_lines - R + 1)
-    size_t cells = 0;           // rows * stride
+    int block_rows = 0;         // of the box statistics
     InvSource inv_c{nullptr, nullptr, 0};
 };
 
@@ -1074,9 +1072,8 @@ int spec_rasters(ampcor_handle* h, const PairSource& src, long long pairs, SpecR
     r.raster_stats = src.tgt_lines > 0 && r.rows > 0 && src.tgt_stride <= 12288;
     r.inv_c = InvSource{nullptr, nullptr, 0};
     if (r.raster_stats) {
-        r.cells = (size_t)r.rows * (size_t)src.tgt_stride;
-        if ((rc = grow(h, h->d_vsum, h->vsum_cap, 2 * r.cells, "box statistics")) ||
-            (rc = grow(h, h->d_inv_raster, h->inv_raster_cap, r.cells + 16, "box statistics")))
+        r.block_rows = box_block_rows(r.rows, src.tgt_stride, h->R, (unsigned)std::max(1, h->sms));
+        if ((rc = grow(h, h->d_inv_raster, h->inv_raster_cap, (size_t)r.rows * (size_t)src.tgt_stride + 16, "box statistics")))
             return rc;
         r.inv_c = InvSource{h->d_inv_raster, src.tgt_off, src.tgt_stride};
     }
@@ -1090,31 +1087,21 @@ int spec_band(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lon
               long long ref_hi, long long tgt_lo, long long tgt_hi, long long box_lo, long long box_hi,
               cudaStream_t st)
 {
-    auto detect = [&](const float2* x, long long n, float* y) {
-        const long long blocks = std::min<long long>((n + 1023) / 1024, 148 * 16);
-        if (n > 0) detect_kernel<<<(unsigned)std::max<long long>(blocks, 1), 256, 0, st>>>(x, n, y);
-        return n > 0 ? 1 : 0;
-    };
     cudaEvent_t a0 = mark(h, st);
-    int kernels = 0;
+    int kernels = 1;
     if (r.shared) {
         const long long lo = std::min(ref_lo, tgt_lo), hi = std::max(ref_hi, tgt_hi);
-        kernels += detect(src.ref_base + lo, hi - lo, r.amp_ref + lo);
+        CK(h, launch_detect(st, src.ref_base + lo, std::max(0LL, hi - lo), r.amp_ref + lo, nullptr, 0, nullptr),
+           "launching the detection kernel");
     } else {
-        kernels += detect(src.ref_base + ref_lo, ref_hi - ref_lo, r.amp_ref + ref_lo);
-        kernels += detect(src.tgt_base + tgt_lo, tgt_hi - tgt_lo, r.amp_tgt + tgt_lo);
+        CK(h, launch_detect(st, src.ref_base + ref_lo, std::max(0LL, ref_hi - ref_lo), r.amp_ref + ref_lo,
+                            src.tgt_base + tgt_lo, std::max(0LL, tgt_hi - tgt_lo), r.amp_tgt + tgt_lo),
+           "launching the detection kernel");
     }
-    CK(h, cudaGetLastError(), "launching the detection kernel");
     if (r.raster_stats && box_hi > box_lo) {
-        const long long vlo = box_lo / kVBlock * kVBlock;
-        const dim3 vg((unsigned)((src.tgt_stride + 255) / 256), (unsigned)((box_hi - vlo + kVBlock - 1) / kVBlock));
-        box_vsum_kernel<<<vg, 256, 0, st>>>(r.amp_tgt, src.tgt_stride, h->R, vlo, box_hi, h->d_vsum,
-                                            h->d_vsum + r.cells);
-        const int psmem = (int)((2 * (src.tgt_stride + 1) + 2 * kWarps) * sizeof(double));
-        box_inv_kernel<<<(unsigned)(box_hi - box_lo), kThreads, psmem, st>>>(
-            h->d_vsum, h->d_vsum + r.cells, box_lo, box_hi, src.tgt_stride, h->R, h->d_inv_raster);
-        CK(h, cudaGetLastError(), "launching the box statistics kernels");
-        kernels += 2;
+        CK(h, launch_box_stats(st, r.amp_tgt, src.tgt_stride, h->R, r.block_rows, box_lo, box_hi, h->d_inv_raster),
+           "launching the box statistics kernel");
+        ++kernels;
     }
     keep(h, 3, a0, mark(h, st), kernels);
     return AMPCOR_OK;
@@ -1450,7 +1437,7 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         (e = cudaFuncSetAttribute(tc_fine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kMaxSmem)) != cudaSuccess ||
         (e = zoom_set_smem_limits()) != cudaSuccess ||
-        (e = refine_half_set_smem_limits()) != cudaSuccess || (e = spec_set_smem_limits()) != cudaSuccess)
+        (e = refine_half_set_smem_limits()) != cudaSuccess || (e = raster_set_smem_limits()) != cudaSuccess || (e = spec_set_smem_limits()) != cudaSuccess)
         return cuda_create_fail(e, "configuring kernel shared memory");
 
     const std::vector<float> ct = taps_table(h->R, h->f, 1, h->ic.taps_len);
@@ -1516,7 +1503,6 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_tw_f);
     cudaFree(h->d_tw_refine);
     cudaFree(h->d_amp);
-    cudaFree(h->d_vsum);
     cudaFree(h->d_inv_raster);
     cudaFree(h->d_tstat);
     cudaFree(h->d_inv_blk);

@@ -13,8 +13,7 @@
 // windows overlap, so every sample is shared by many pairs) and the correlation kernel takes float
 // amplitudes through asynchronous copies.  The placement statistics (1/sigma of every window box)
 // come from the window while it sits in shared memory (spec_box_stats), or, for the coarse stage
-// of windows that tile a raster, from FP64 sums over the whole raster (box_vsum_kernel,
-// box_inv_kernel).
+// of windows that tile a raster, from FP64 sums over the whole raster (raster_stats.cu).
 //
 // Accuracy.  The window is centred on its mean before the transform (sum r' = 0, so the
 // numerators keep their value) and the twiddles are correctly rounded, which keeps the transform
@@ -1675,143 +1674,6 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
 
 }  // namespace
 
-__global__ void detect_kernel(const float2* __restrict__ src, long long n, float* __restrict__ dst)
-{
-    const long long step = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
-        float2 z[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const long long j = i + k * step;
-            z[k] = j < n ? __ldg(src + j) : make_float2(0.0f, 0.0f);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const long long j = i + k * step;
-            if (j < n) dst[j] = amp_of(z[k]);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256)
-box_vsum_kernel(const float* __restrict__ a, long long samples, int R, long long row_lo,
-                long long row_hi, double* __restrict__ v1, double* __restrict__ v2)
-{
-    const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long y0 = row_lo + (long long)blockIdx.y * kVBlock;
-    if (x >= samples || y0 >= row_hi) return;
-    const long long y1 = y0 + kVBlock < row_hi ? y0 + kVBlock : row_hi;
-    const float* col = a + x;
-    double a1[4] = {0.0, 0.0, 0.0, 0.0}, a2[4] = {0.0, 0.0, 0.0, 0.0};
-    int i = 0;
-    for (; i + 4 <= R; i += 4) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const double tv = __ldg(col + (y0 + i + k) * samples);
-            a1[k] += tv;
-            a2[k] += tv * tv;
-        }
-    }
-    for (; i < R; ++i) {
-        const double tv = __ldg(col + (y0 + i) * samples);
-        a1[0] += tv;
-        a2[0] += tv * tv;
-    }
-    double s1 = (a1[0] + a1[1]) + (a1[2] + a1[3]);
-    double s2 = (a2[0] + a2[1]) + (a2[2] + a2[3]);
-    for (long long y = y0; y < y1; ++y) {
-        v1[y * samples + x] = s1;
-        v2[y * samples + x] = s2;
-        if (y + 1 < y1) {
-            const double p = __ldg(col + (y + R) * samples), q = __ldg(col + y * samples);
-            s1 += p - q;
-            s2 += p * p - q * q;
-        }
-    }
-}
-
-// one CTA per box row: FP64 exclusive prefix sums of the row's column sums (in chunks of four per
-// thread, a fixed order), then the box of every x from two prefix differences; two CTAs per SM,
-// so that one row's loads overlap another's scan
-__global__ void __launch_bounds__(kThreads, 2)
-box_inv_kernel(const double* __restrict__ v1, const double* __restrict__ v2, long long row_lo,
-               long long row_hi, long long samples, int R, float* __restrict__ inv)
-{
-    extern __shared__ __align__(16) double psm[];
-    const long long y = row_lo + blockIdx.x;
-    if (y >= row_hi) return;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double* P1 = psm;
-    double* P2 = psm + samples + 1;
-    double* red = P2 + samples + 1;  // 2 x kWarps
-    const double* r1 = v1 + y * samples;
-    const double* r2 = v2 + y * samples;
-    double carry1 = 0.0, carry2 = 0.0;
-    constexpr int kPer = 4;  // consecutive samples per thread and chunk
-    for (long long c0 = 0; c0 < samples; c0 += kThreads * kPer) {
-        const long long b0 = c0 + (long long)tid * kPer;
-        double l1[kPer], l2[kPer], s1 = 0.0, s2 = 0.0;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const long long i = b0 + k;
-            const double p = i < samples ? __ldg(r1 + i) : 0.0;
-            const double q = i < samples ? __ldg(r2 + i) : 0.0;
-            l1[k] = s1;
-            l2[k] = s2;
-            s1 += p;
-            s2 += q;
-        }
-        // exclusive scan of the thread totals: within the warp, then across warps
-        double i1 = s1, i2 = s2;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double u1 = __shfl_up_sync(kFull, i1, o), u2 = __shfl_up_sync(kFull, i2, o);
-            if (lane >= o) {
-                i1 += u1;
-                i2 += u2;
-            }
-        }
-        if (lane == 31) {
-            red[warp] = i1;
-            red[kWarps + warp] = i2;
-        }
-        __syncthreads();
-        double w1 = 0.0, w2 = 0.0, t1 = 0.0, t2 = 0.0;
-        for (int w = 0; w < kWarps; ++w) {
-            if (w < warp) {
-                w1 += red[w];
-                w2 += red[kWarps + w];
-            }
-            t1 += red[w];
-            t2 += red[kWarps + w];
-        }
-        const double o1 = carry1 + w1 + (i1 - s1), o2 = carry2 + w2 + (i2 - s2);
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const long long i = b0 + k;
-            if (i < samples) {
-                P1[i] = o1 + l1[k];
-                P2[i] = o2 + l2[k];
-            }
-        }
-        carry1 += t1;
-        carry2 += t2;
-        __syncthreads();
-    }
-    if (tid == 0) {
-        P1[samples] = carry1;
-        P2[samples] = carry2;
-    }
-    __syncthreads();
-    const double cells = (double)R * (double)R;
-    for (long long x = tid; x + R <= samples; x += kThreads) {
-        const double b1 = P1[x + R] - P1[x];
-        const double b2 = P2[x + R] - P2[x];
-        const float var = (float)(b2 - b1 * b1 / cells);
-        inv[y * samples + x] = var > 0.0f ? __frsqrt_rn(var) : 0.0f;
-    }
-}
-
 bool spec_radices(int n, int& n1, int& n2)
 {
 #define AMPCOR_SPEC_CASE(NN, A, B) \
@@ -1862,7 +1724,7 @@ bool spec_shared(int n, int& threads, int& ctas)
 cudaError_t spec_set_smem_limits()
 {
     const int limit = 227 * 1024;
-    cudaError_t e = cudaFuncSetAttribute(box_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    cudaError_t e = cudaSuccess;
 #define AMPCOR_SPEC_CASE(NN, A, B) \
     if (e == cudaSuccess)          \
         e = cudaFuncSetAttribute(spec_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \

@@ -415,10 +415,10 @@ def run_b200(args):
             .get(worker.form, "coarse_kernel"),
             "fine_correlation": {"tensor": "tc_fine_kernel", "spectral": "spec_staged_kernel (fine)"}
             .get(worker.form, "fine_kernel"),
-            "refinement": {"spectral": "spec_refine_kernel (chip + window)"}.get(worker.form, "refine_kernel"),
-            "coarse_statistics": {"spectral": "detect_kernel + box_vsum_kernel + box_inv_kernel (per raster)"}
+            "refinement": {"spectral": "refine_half_kernel (chip + window)"}.get(worker.form, "refine_kernel"),
+            "coarse_statistics": {"spectral": "detect_kernel + box_stats_kernel (per raster)"}
             .get(worker.form, "window_stats_cplx_kernel"),
-            "fine_statistics": {"spectral": "spec_chip_stats_kernel + spec_tile_stats_kernel (blocked fine stage)"}
+            "fine_statistics": {"spectral": "spec_tile_stats_kernel (blocked fine stage)"}
             .get(worker.form, "window_stats_real_kernel"),
             "zoom": "zoom_kernel",
         }
@@ -458,8 +458,8 @@ def run_b200(args):
             fft = {
                 "coarse_correlation": (W + nc + nc // 2 + 1 + (C + 1) // 2) * fft_flops(nc),
                 "fine_correlation": (Wf + nf + nf // 2 + 1 + (Cf + 1) // 2) * fft_flops(nf),
-                "refinement": sum(n * fft_flops(n) + n * fft_flops(f * n) + f * n * fft_flops(n)
-                                  + f * n * fft_flops(f * n) for n in (R, E)),
+                # half-sample shifts of 3 n lines, each a transform there and back
+                "refinement": sum(6 * n * fft_flops(n) for n in (R, E)),
             }
             for k, per_pair in fft.items():
                 if k in kernels:
