@@ -440,7 +440,8 @@ __device__ void zoom_argmax(const float* G, float* T, const float* taps, const Z
 __global__ void pair_offsets_kernel(const int* ulhc, long long pairs, long long ref_lines,
                                     long long ref_samples, long long tgt_lines,
                                     long long tgt_samples, int R, int W, long long* ref_off,
-                                    long long* tgt_off, unsigned int* bad)
+                                    long long* tgt_off, unsigned int* bad, long long amp_ref_stride,
+                                    long long amp_tgt_stride, long long* amp_ref_off, long long* amp_tgt_off)
 {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= pairs) return;
@@ -450,6 +451,10 @@ __global__ void pair_offsets_kernel(const int* ulhc, long long pairs, long long 
                     tl >= 0 && ts >= 0 && tl + W <= tgt_lines && ts + W <= tgt_samples;
     ref_off[p] = ok ? rl * ref_samples + rs : -1;
     tgt_off[p] = ok ? tl * tgt_samples + ts : -1;
+    if (amp_ref_off) {
+        amp_ref_off[p] = ok ? rl * amp_ref_stride + rs : -1;
+        amp_tgt_off[p] = ok ? tl * amp_tgt_stride + ts : -1;
+    }
     if (!ok) atomicAdd(bad, 1u);
 }
 

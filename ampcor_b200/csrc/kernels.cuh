@@ -82,6 +82,11 @@ struct PairSource {
     long long ref_count;  // samples behind ref_base (the raster or the arena)
     long long tgt_count;
     long long tgt_lines;  // lines of the secondary raster (tgt_count / tgt_stride); 0 for the arena
+    // where the amplitude rasters have longer lines than the rasters: their strides, and the tiles'
+    // offsets in them (else nullptr)
+    long long amp_ref_stride = 0, amp_tgt_stride = 0;
+    const long long* amp_ref_off = nullptr;
+    const long long* amp_tgt_off = nullptr;
 };
 
 // coarse result of one pair
@@ -142,7 +147,9 @@ struct FineOut {
 __global__ void pair_offsets_kernel(const int* ulhc, long long pairs, long long ref_lines,
                                     long long ref_samples, long long tgt_lines,
                                     long long tgt_samples, int R, int W, long long* ref_off,
-                                    long long* tgt_off, unsigned int* bad);
+                                    long long* tgt_off, unsigned int* bad,
+                                    long long amp_ref_stride, long long amp_tgt_stride, long long* amp_ref_off,
+                                    long long* amp_tgt_off);
 
 __global__ void arena_offsets_kernel(long long pairs, long long ref_cells, long long tgt_cells,
                                      long long* ref_off, long long* tgt_off);
@@ -262,13 +269,20 @@ struct SpecOut {
 // |z| of the n samples of a complex array and of the n2 of another
 cudaError_t launch_detect(cudaStream_t st, const float2* src, long long n, float* dst, const float2* src2,
                           long long n2, float* dst2);
+// the same of two rasters' first `lines` lines, line for line into longer ones (pitch)
+struct DetectLines {
+    const float2* src;
+    float* dst;
+    long long lines, samples, pitch;
+};
+cudaError_t launch_detect_lines(cudaStream_t st, const DetectLines& a, const DetectLines& b);
 // 1/sqrt(var), from FP64 sums, of the R x R box at every (y, x) of an amplitude raster, x <= samples - R, for
 // box rows [row_lo, row_hi) (box row y covers raster rows y .. y + R - 1).  The sums start anew at
 // every block_rows-th row (box_block_rows: by the size of the raster), so that a band computes its
 // rows exactly as the whole raster would.
 int box_block_rows(long long rows, long long samples, int R, unsigned sms);
-cudaError_t launch_box_stats(cudaStream_t st, const float* a, long long samples, int R, int block_rows,
-                             long long row_lo, long long row_hi, float* inv);
+cudaError_t launch_box_stats(cudaStream_t st, const float* a, long long samples, long long pitch, int R,
+                             int block_rows, long long row_lo, long long row_hi, float* inv);
 cudaError_t raster_set_smem_limits();
 
 // where a spectral correlation finds 1/sigma_box of placement (u, v) of chunk-local pair b:

@@ -62,6 +62,28 @@ detect_kernel(const float2* __restrict__ src, long long n, float* __restrict__ d
     }
 }
 
+// the same line for line into longer lines, a CTA per line
+__global__ void __launch_bounds__(256, kDetectCtas)
+detect_lines_kernel(DetectLines a, DetectLines b, int blocks)
+{
+    const bool second = (int)blockIdx.x >= blocks;
+    const DetectLines d = second ? b : a;
+    const int first = (int)blockIdx.x - (second ? blocks : 0), step = second ? (int)gridDim.x - blocks : blocks;
+    for (long long y = first; y < d.lines; y += step) {
+        const float2* src = d.src + y * d.samples;
+        float* dst = d.dst + y * d.pitch;
+        long long x = threadIdx.x;
+        for (; x + 768 < d.samples; x += 1024) {
+            float2 z[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) z[k] = __ldg(src + x + 256 * k);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dst[x + 256 * k] = amp_of(z[k]);
+        }
+        for (; x < d.samples; x += 256) dst[x] = amp_of(__ldg(src + x));
+    }
+}
+
 // element i of a padded row of FP64 sums: 16 neighbours sit in different banks, and so do the first of
 // 16 lanes' NT / 32 neighbours (a slot left out every 8 instead costs half of the wavefronts' rate)
 __device__ __forceinline__ int padded(int i) { return i + (i >> 4); }
@@ -71,7 +93,7 @@ constexpr int kBoxRow = NT + NT / 16 + 1;  // slots of a row
 
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT)
-box_stats_kernel(const float* __restrict__ a, int samples, int R, int block_rows, int row_lo, int row_hi,
+box_stats_kernel(const float* __restrict__ a, int samples, int pitch, int R, int block_rows, int row_lo, int row_hi,
                  float* __restrict__ inv)
 {
     constexpr int kRow = kBoxRow<NT>, kPer = NT / 32;
@@ -82,15 +104,15 @@ box_stats_kernel(const float* __restrict__ a, int samples, int R, int block_rows
     const int y0 = (row_lo / block_rows + blockIdx.y) * block_rows;
     const int y1 = min(y0 + block_rows, row_hi);
     // (threads past the raster's last column sum that column again: no box uses it)
-    const float* leave = a + (long long)y0 * samples + min(x, samples - 1);  // row y of this column
+    const float* leave = a + (long long)y0 * pitch + min(x, samples - 1);  // row y of this column
     const float* enter = leave;                                              // and row y + R
     double s1 = 0.0, s2 = 0.0;
     auto add = [&](auto rows) {
         constexpr int kN = decltype(rows)::value;
         float v[kN];
 #pragma unroll
-        for (int k = 0; k < kN; ++k) v[k] = __ldg(enter + k * samples);
-        enter += kN * samples;
+        for (int k = 0; k < kN; ++k) v[k] = __ldg(enter + k * pitch);
+        enter += kN * pitch;
         double c1[2] = {0.0, 0.0}, c2[2] = {0.0, 0.0};
 #pragma unroll
         for (int k = 0; k < kN; ++k) {
@@ -105,26 +127,26 @@ box_stats_kernel(const float* __restrict__ a, int samples, int R, int block_rows
     for (; i + 16 <= R; i += 16) add(std::integral_constant<int, 16>{});
     for (; i < R; ++i) add(std::integral_constant<int, 1>{});
     const double per_cell = 1.0 / ((double)R * (double)R);
-    float* out = inv + (long long)y0 * samples + x;
+    float* out = inv + (long long)y0 * pitch + x;
     const bool box = tid < cols && x + R <= samples;
     for (int y = y0; y < y1; y += kBoxRows) {
         float up[kBoxRows], dn[kBoxRows];
         if (y + kBoxRows < y1) {
 #pragma unroll
             for (int r = 0; r < kBoxRows; ++r) {
-                up[r] = __ldg(leave + r * samples);
-                dn[r] = __ldg(enter + r * samples);
+                up[r] = __ldg(leave + r * pitch);
+                dn[r] = __ldg(enter + r * pitch);
             }
         } else {
 #pragma unroll
             for (int r = 0; r < kBoxRows; ++r) {
                 const bool in = y + r + 1 < y1;
-                up[r] = in ? __ldg(leave + r * samples) : 0.0f;
-                dn[r] = in ? __ldg(enter + r * samples) : 0.0f;
+                up[r] = in ? __ldg(leave + r * pitch) : 0.0f;
+                dn[r] = in ? __ldg(enter + r * pitch) : 0.0f;
             }
         }
-        leave += kBoxRows * samples;
-        enter += kBoxRows * samples;
+        leave += kBoxRows * pitch;
+        enter += kBoxRows * pitch;
         double* mine = sums + padded(tid);
 #pragma unroll
         for (int r = 0; r < kBoxRows; ++r) {
@@ -165,10 +187,10 @@ box_stats_kernel(const float* __restrict__ a, int samples, int R, int block_rows
             for (int r = 0; r < kBoxRows; ++r) {
                 const double b1 = hi[r * kRow] - lo[r * kRow], b2 = hi[(kBoxRows + r) * kRow] - lo[(kBoxRows + r) * kRow];
                 const float var = (float)(b2 - b1 * b1 * per_cell);
-                if (r >= first && r < last) out[r * samples] = var > 0.0f ? __frsqrt_rn(var) : 0.0f;
+                if (r >= first && r < last) out[r * pitch] = var > 0.0f ? __frsqrt_rn(var) : 0.0f;
             }
         }
-        out += kBoxRows * samples;
+        out += kBoxRows * pitch;
         __syncthreads();
     }
 }
@@ -201,6 +223,17 @@ cudaError_t launch_detect(cudaStream_t st, const float2* src, long long n, float
     return cudaGetLastError();
 }
 
+cudaError_t launch_detect_lines(cudaStream_t st, const DetectLines& a, const DetectLines& b)
+{
+    const long long la = std::max(a.lines, 0LL), lb = std::max(b.lines, 0LL);
+    const long long all = std::min<long long>(la + lb, 148LL * kDetectCtas);
+    if (all <= 0) return cudaSuccess;
+    long long blocks = (all * la + (la + lb) / 2) / (la + lb);
+    blocks = lb == 0 ? all : la == 0 ? 0 : std::min(std::max(blocks, 1LL), all - 1);
+    detect_lines_kernel<<<(unsigned)all, 256, 0, st>>>(a, b, (int)blocks);
+    return cudaGetLastError();
+}
+
 // columns of a CTA: at least twice the box
 static int box_threads(int R) { return R <= 96 ? 256 : R <= 256 ? 512 : 1024; }
 
@@ -212,19 +245,19 @@ int box_block_rows(long long rows, long long samples, int R, unsigned sms)
     return block;
 }
 
-cudaError_t launch_box_stats(cudaStream_t st, const float* a, long long samples, int R, int block_rows,
-                             long long row_lo, long long row_hi, float* inv)
+cudaError_t launch_box_stats(cudaStream_t st, const float* a, long long samples, long long pitch, int R,
+                             int block_rows, long long row_lo, long long row_hi, float* inv)
 {
     const int nt = box_threads(R);
     const long long cols = nt + 1 - R, first = row_lo / block_rows;
     if (samples < R || row_hi <= row_lo) return cudaSuccess;
     const dim3 grid((unsigned)((samples - R + cols) / cols), (unsigned)((row_hi + block_rows - 1) / block_rows - first));
     if (nt == 256)
-        box_stats_kernel<256><<<grid, 256, box_smem<256>(), st>>>(a, (int)samples, R, block_rows, (int)row_lo, (int)row_hi, inv);
+        box_stats_kernel<256><<<grid, 256, box_smem<256>(), st>>>(a, (int)samples, (int)pitch, R, block_rows, (int)row_lo, (int)row_hi, inv);
     else if (nt == 512)
-        box_stats_kernel<512><<<grid, 512, box_smem<512>(), st>>>(a, (int)samples, R, block_rows, (int)row_lo, (int)row_hi, inv);
+        box_stats_kernel<512><<<grid, 512, box_smem<512>(), st>>>(a, (int)samples, (int)pitch, R, block_rows, (int)row_lo, (int)row_hi, inv);
     else
-        box_stats_kernel<1024><<<grid, 1024, box_smem<1024>(), st>>>(a, (int)samples, R, block_rows, (int)row_lo, (int)row_hi, inv);
+        box_stats_kernel<1024><<<grid, 1024, box_smem<1024>(), st>>>(a, (int)samples, (int)pitch, R, block_rows, (int)row_lo, (int)row_hi, inv);
     return cudaGetLastError();
 }
 
