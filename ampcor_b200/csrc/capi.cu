@@ -431,6 +431,25 @@ bool plan_spec_block_staged(int K, SpecGeom& g)
     return N >= 128 && g.smem_staged <= limit;
 }
 
+// A coarse window beyond one tile may split its placements instead of its chip: four sub-windows of
+// R + Cq - 1 samples, Cq of C placements a side (the second ones from placement C - Cq on, a multiple of 4 so that
+// tensor copies start on 16 bytes), each an ordinary staged correlation with its own maximum.  That
+// pays where four such tiles are smaller than the K tiles of the chip's blocks: 64 px chips and
+// +-64 px are four tiles of 128 samples against four of 160 and a reduction, 900 pairs 1,094 -> 526 us
+// (the job 1,551 -> 988); 128 px chips and +-32 px would be four of 160 against four of 128.
+bool plan_spec_parts(int R, int W, const SpecBlocks& b, int& Cq, SpecGeom& g)
+{
+    std::string e;
+    const int C = W - R + 1, s = C / 2 / 4 * 4;
+    Cq = C - s;
+    SpecGeom several;
+    if (s < 1 || !plan_spec(R, R + Cq - 1, g, e) || 4L * g.N * g.N >= (long)b.K * b.tile.N * b.tile.N ||
+        4L * Cq * Cq > (long)b.K * C * C || !plan_spec_staged(R, R + Cq - 1, false, kSpecThreads, g))
+        return false;
+    if (plan_spec_shared(R, R + Cq - 1, false, several)) g = several;
+    return true;
+}
+
 bool plan_spec_blocked(int R, int W, SpecBlocks& b, std::string& err)
 {
     b = SpecBlocks{};
@@ -650,6 +669,13 @@ struct ampcor_handle {
     // blocked spectral stages (coarse, fine): placement statistics, partial numerators and their
     // scalars, all per chunk
     SpecBlocks bc{}, bf{};
+    // the coarse stage of a raster's windows in four parts of part_c x part_c placements (plan_spec_parts)
+    bool parts_on = false;
+    int part_c = 0;
+    SpecGeom spp_st{};
+    float* d_tw_p = nullptr;
+    CoarseOut* d_parts = nullptr;  // 4 cap
+    float* d_part_peaks = nullptr;
     float* d_inv_blk = nullptr;
     float* d_part = nullptr;
     double* d_scal = nullptr;
@@ -719,6 +745,8 @@ int grow(ampcor_handle* h, T*& ptr, size_t& cap, size_t n, const char* what)
 int ensure_pairs(ampcor_handle* h, size_t pairs)
 {
     if (h->cap >= pairs && h->d_ref_off) return AMPCOR_OK;
+    cudaFree(h->d_parts);
+    cudaFree(h->d_part_peaks);
     cudaFree(h->d_ref_off);
     cudaFree(h->d_tgt_off);
     cudaFree(h->d_amp_ref_off);
@@ -728,6 +756,8 @@ int ensure_pairs(ampcor_handle* h, size_t pairs)
     cudaFree(h->d_offsets);
     cudaFree(h->d_diag);
     h->d_ref_off = h->d_tgt_off = h->d_amp_ref_off = h->d_amp_tgt_off = nullptr;
+    h->d_parts = nullptr;
+    h->d_part_peaks = nullptr;
     h->d_coarse = nullptr;
     h->d_coarse_peak = nullptr;
     h->d_offsets = nullptr;
@@ -738,6 +768,8 @@ int ensure_pairs(ampcor_handle* h, size_t pairs)
         cudaMalloc(&h->d_tgt_off, n * sizeof(long long)) != cudaSuccess ||
         cudaMalloc(&h->d_amp_ref_off, n * sizeof(long long)) != cudaSuccess ||
         cudaMalloc(&h->d_amp_tgt_off, n * sizeof(long long)) != cudaSuccess ||
+        (h->parts_on && (cudaMalloc(&h->d_parts, 4 * n * sizeof(CoarseOut)) != cudaSuccess ||
+                         cudaMalloc(&h->d_part_peaks, 4 * n * sizeof(float)) != cudaSuccess)) ||
         cudaMalloc(&h->d_coarse, n * sizeof(CoarseOut)) != cudaSuccess ||
         cudaMalloc(&h->d_coarse_peak, n * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&h->d_offsets, n * sizeof(float2)) != cudaSuccess ||
@@ -1031,13 +1063,14 @@ EncodeTiledFn encode_tiled()
 // a 2-D map of a float raster (lines x samples) whose boxes are bx x by floats (bx a multiple of
 // 4); false where the driver has no tensor maps or the raster breaks the copy engine's alignment
 // rules (a 16-byte aligned base, lines a multiple of 16 bytes)
-bool raster_map(CUtensorMap& m, const float* base, long long lines, long long samples, int bx, int by)
+bool raster_map(CUtensorMap& m, const float* base, long long lines, long long samples, int bx, int by,
+                long long from = 0)
 {
     const EncodeTiledFn fn = encode_tiled();
     if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || (samples & 3) || lines < 1 || bx % 4 || bx < 4 ||
         bx > 256 || by < 1 || by > 256)
         return false;
-    const cuuint64_t dim[2] = {(cuuint64_t)samples, (cuuint64_t)lines};
+    const cuuint64_t dim[2] = {(cuuint64_t)(samples - from), (cuuint64_t)lines};
     const cuuint64_t stride[1] = {(cuuint64_t)samples * 4};
     const cuuint32_t box[2] = {(cuuint32_t)bx, (cuuint32_t)by};
     const cuuint32_t es[2] = {1, 1};
@@ -1181,6 +1214,19 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
                                  h->refined_stride, h->bf.tile_st.stage_rs, h->bf.tile_st.W) &&
                        tiles_map(bcf, h->d_refined, h->Rf, (long long)h->chunk_cap, h->refined_stride,
                                  (h->bf.B + 6) & ~3, h->bf.B);
+    // the coarse stage in four parts: the maps of each part's windows and statistics start at its first
+    // placement
+    CUtensorMap pw[4]{}, pi[4]{}, pc{};
+    const int part_s = h->parts_on ? h->C - h->part_c : 0, part_w = h->R + h->part_c - 1;
+    bool parts_st = h->parts_on && r.inv_c.base && src.tgt_stride > 0 && src.ref_stride > 0 &&
+                    raster_map(pc, r.amp_ref, src.ref_count / src.ref_stride, r.ref_pitch, (h->R + 6) & ~3, h->R);
+    auto part_at = [&](int k) { return (k >> 1) * part_s * r.tgt_pitch + (k & 1) * part_s; };
+    for (int k = 0; parts_st && k < 4; ++k) {
+        const int y = (k >> 1) * part_s, x = (k & 1) * part_s;
+        parts_st = src.tgt_lines > y && r.tgt_pitch > x &&
+                   raster_map(pw[k], r.amp_tgt + part_at(k), src.tgt_lines - y, r.tgt_pitch, h->spp_st.stage_rs, part_w, x) &&
+                   raster_map(pi[k], r.inv_c.base + part_at(k), r.rows - y, r.tgt_pitch, h->spp_st.inv_rs, h->part_c, x);
+    }
     for (long long c0 = p0; c0 < p1; c0 += (long long)h->chunk) {
         const unsigned n = (unsigned)std::min<long long>((long long)h->chunk, p1 - c0);
         TileStat* const st_raw = h->d_tstat;               // the chips
@@ -1205,7 +1251,24 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
             b = b1;
         }
         const SpecOut co{0, h->m, h->d_coarse, h->d_coarse_peak, nullptr, nullptr, coarse_surfaces};
-        if (h->bc.on) {
+        if (parts_st) {
+            const long long cells = (long long)h->part_c * h->part_c, cap = (long long)h->cap;
+            for (int k = 0; k < 4; ++k) {
+                SpecSource ps = cs;
+                ps.win += part_at(k);
+                // (the kernel indexes surfaces by the pair: the chunk's start in the scratch)
+                float* surf = coarse_surfaces ? h->d_part + (k * (long long)n - c0) * cells : nullptr;
+                const SpecOut po{0, h->m, h->d_parts + k * cap, h->d_part_peaks + k * cap, nullptr, nullptr, surf};
+                CK(h, launch_spec_staged(h->spp_st, (unsigned)h->sms, st, ps, c0, n, src.ref_off,
+                                         InvSource{r.inv_c.base + part_at(k), r.inv_c.off, r.inv_c.stride},
+                                         reinterpret_cast<const float2*>(h->d_tw_p), po, st_raw, nullptr, h->d_tc_err,
+                                         &pw[k], &pc, &pi[k], h->inject_timeouts > 0 ? 1 : 0),
+                   "launching a part of the coarse correlation");
+            }
+            CK(h, launch_join_parts(st, h->d_parts, h->d_part_peaks, cap, c0, n, src.ref_off, h->C, h->part_c, h->m, h->W,
+                                    h->E, h->d_coarse, h->d_coarse_peak, h->d_part, coarse_surfaces),
+               "launching the join of the coarse parts");
+        } else if (h->bc.on) {
             InvSource ic = r.inv_c;
             if (!ic.base) {
                 CK(h, launch_spec_tile_stats(n, st, cs, c0, n, src.ref_off, h->R, h->W, h->d_inv_blk),
@@ -1239,7 +1302,7 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
                    "launching the spectral coarse correlation");
         }
         cudaEvent_t c = mark(h, st);
-        keep(h, 0, b, c, h->bc.on ? 2 : 1);
+        keep(h, 0, b, c, parts_st ? 5 : h->bc.on ? 2 : 1);
         if (h->refine_fft) {
             CK(h, launch_refine_half(h->E, n, st, src.tgt_base, src.tgt_off, src.tgt_stride, h->d_coarse, c0, n,
                                      src.ref_off, tab + 2 * h->R, h->d_refined, h->refined_stride,
@@ -1422,6 +1485,7 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         const bool fine_ok = coarse_ok && (direct_f || plan_spec_blocked(h->Rf, h->Wf, h->bf, serr));
         h->spectral_ok = fine_ok && (h->refine_fft || interp_ok);
         if (direct_c || !h->spectral_ok) h->bc = SpecBlocks{};
+        h->parts_on = staged_on && h->bc.on && plan_spec_parts(h->R, h->W, h->bc, h->part_c, h->spp_st);
         if (direct_f || !h->spectral_ok) h->bf = SpecBlocks{};
         if (!h->spectral_ok && serr.empty()) serr = "no refinement of these tiles is compiled";
         if (!h->plain_ok && !h->spectral_ok) {
@@ -1498,6 +1562,8 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         (e = upload(h->d_tw_c, spec_twiddle_table(std::max(h->bc.on ? h->bc.tile.N : h->spc.N, 1)))) != cudaSuccess ||
         (e = upload(h->d_tw_f, spec_twiddle_table(std::max(h->bf.on ? h->bf.tile.N : h->spf.N, 1)))) != cudaSuccess)
         return cuda_create_fail(e, "uploading interpolation taps");
+    if (h->parts_on && (e = upload(h->d_tw_p, spec_twiddle_table(h->spp_st.N))) != cudaSuccess)
+        return cuda_create_fail(e, "uploading twiddles");
     if (h->refine_fft) {
         std::vector<float> tw;
         for (int n : {h->R, h->E}) {
@@ -1526,6 +1592,8 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_zoom_taps);
     cudaFree(h->d_zoom_u);
     cudaFree(h->d_arena);
+    cudaFree(h->d_parts);
+    cudaFree(h->d_part_peaks);
     cudaFree(h->d_ref_off);
     cudaFree(h->d_tgt_off);
     cudaFree(h->d_amp_ref_off);
@@ -1548,6 +1616,7 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_tw_c);
     cudaFree(h->d_tw_f);
     cudaFree(h->d_tw_refine);
+    cudaFree(h->d_tw_p);
     cudaFree(h->d_amp);
     cudaFree(h->d_inv_raster);
     cudaFree(h->d_tstat);

@@ -285,6 +285,13 @@ cudaError_t launch_box_stats(cudaStream_t st, const float* a, long long samples,
                              int block_rows, long long row_lo, long long row_hi, float* inv);
 cudaError_t raster_set_smem_limits();
 
+// The coarse result of n pairs whose placements were correlated in four parts of Cq x Cq, the second ones
+// from placement C - Cq on: part k of pair p at parts[k stride + p] and peaks[k stride + p], its surface (where
+// surfaces are wanted) at part_surfaces + (k n + p - pair0) Cq^2.
+cudaError_t launch_join_parts(cudaStream_t st, const CoarseOut* parts, const float* peaks, long long stride,
+                              long long pair0, unsigned n, const long long* valid, int C, int Cq, int m, int W, int E,
+                              CoarseOut* coarse, float* coarse_peak, const float* part_surfaces, float* surfaces);
+
 // where a spectral correlation finds 1/sigma_box of placement (u, v) of chunk-local pair b:
 // base + off[pair0 + b] + u stride + v when off is given, else base + b C^2 + u C + v
 struct InvSource {

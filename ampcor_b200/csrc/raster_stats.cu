@@ -261,4 +261,45 @@ cudaError_t launch_box_stats(cudaStream_t st, const float* a, long long samples,
     return cudaGetLastError();
 }
 
+static __global__ void __launch_bounds__(128)
+join_parts_kernel(const CoarseOut* parts, const float* peaks, long long stride, long long pair0, unsigned n,
+                  const long long* valid, int C, int Cq, int m, int W, int E, CoarseOut* coarse, float* coarse_peak,
+                  const float* part_surfaces, float* surfaces)
+{
+    const long long p = pair0 + blockIdx.x;
+    if (valid[p] < 0) return;
+    const int s = C - Cq;
+    if (threadIdx.x == 0) {
+        // the first maximum in row-major order over all placements (a part without one reports a cell outside)
+        float bv = -INFINITY;
+        int bi = INT_MAX;
+        for (int k = 0; k < 4; ++k) {
+            const CoarseOut c = parts[k * stride + p];
+            if ((unsigned)c.u < (unsigned)Cq && (unsigned)c.v < (unsigned)Cq)
+                better(bv, bi, peaks[k * stride + p], (c.u + (k >> 1) * s) * C + c.v + (k & 1) * s);
+        }
+        const int u = bi / C, v = bi - u * C;
+        // nudge.cu:107-140
+        const int left = min(max(v - m, 0), W - E), top = min(max(u - m, 0), W - E);
+        coarse[p] = CoarseOut{u, v, top, left};
+        coarse_peak[p] = bv;
+    }
+    if (surfaces) {
+        for (int i = threadIdx.x; i < C * C; i += 128) {
+            const int u = i / C, v = i - u * C, k = (u >= Cq ? 2 : 0) + (v >= Cq ? 1 : 0);
+            surfaces[p * C * C + i] = part_surfaces[((long long)k * n + blockIdx.x) * Cq * Cq +
+                                                    (u - (k >> 1) * s) * Cq + v - (k & 1) * s];
+        }
+    }
+}
+
+cudaError_t launch_join_parts(cudaStream_t st, const CoarseOut* parts, const float* peaks, long long stride,
+                              long long pair0, unsigned n, const long long* valid, int C, int Cq, int m, int W, int E,
+                              CoarseOut* coarse, float* coarse_peak, const float* part_surfaces, float* surfaces)
+{
+    join_parts_kernel<<<n, 128, 0, st>>>(parts, peaks, stride, pair0, n, valid, C, Cq, m, W, E, coarse, coarse_peak,
+                                         part_surfaces, surfaces);
+    return cudaGetLastError();
+}
+
 }  // namespace ampcor_b200
