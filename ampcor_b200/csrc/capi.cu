@@ -634,7 +634,8 @@ struct ampcor_handle {
     size_t chunk = 0;      // pairs per chunk
     size_t chunk_cap = 0;  // pairs the scratch holds: the chunk, or all of a smaller job
     size_t chunk_override = 0;
-    bool chunk_short = false;  // the default chunk's scratch did not fit: one wave instead
+    bool chunk_short = false;  // the default chunk's scratch had no room: one wave instead
+    bool captured = false;     // a graph may hold the addresses of the worker's buffers
     long long refined_stride = 0;
     // host-path staging
     void* d_ref_raster = nullptr;
@@ -726,6 +727,29 @@ int cuda_fail(ampcor_handle* h, cudaError_t e, const char* what)
         if (e_ != cudaSuccess) return cuda_fail(h, e_, what); \
     } while (0)
 
+void free_chunk_scratch(ampcor_handle* h);
+bool default_chunk_waves(const ampcor_handle* h);
+
+// Device memory of a worker.  A default chunk of several waves is held for speed alone: where something
+// else finds no room it gives way to one wave, for good (ensure_refined), unless a captured graph may
+// still use it.  A failure leaves no runtime error behind for the next launch to trip over.
+template <typename T>
+cudaError_t device_alloc(ampcor_handle* h, T*& ptr, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(&ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && default_chunk_waves(h) && !h->captured) {
+        cudaGetLastError();
+        free_chunk_scratch(h);
+        h->chunk_short = true;
+        e = cudaMalloc(&ptr, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        ptr = nullptr;
+    }
+    return e;
+}
+
 template <typename T>
 int grow(ampcor_handle* h, T*& ptr, size_t& cap, size_t n, const char* what)
 {
@@ -733,11 +757,9 @@ int grow(ampcor_handle* h, T*& ptr, size_t& cap, size_t n, const char* what)
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc((void**)&ptr, std::max<size_t>(n, 1) * sizeof(T));
-    if (e != cudaSuccess) {
-        ptr = nullptr;
+    cudaError_t e = device_alloc(h, ptr, std::max<size_t>(n, 1) * sizeof(T));
+    if (e != cudaSuccess)
         return fail(h, AMPCOR_E_NOMEM, std::string("allocating ") + what + ": " + cudaGetErrorName(e));
-    }
     cap = n;
     return AMPCOR_OK;
 }
@@ -764,16 +786,16 @@ int ensure_pairs(ampcor_handle* h, size_t pairs)
     h->d_diag = nullptr;
     h->cap = 0;
     const size_t n = std::max<size_t>(pairs, 1);
-    if (cudaMalloc(&h->d_ref_off, n * sizeof(long long)) != cudaSuccess ||
-        cudaMalloc(&h->d_tgt_off, n * sizeof(long long)) != cudaSuccess ||
-        cudaMalloc(&h->d_amp_ref_off, n * sizeof(long long)) != cudaSuccess ||
-        cudaMalloc(&h->d_amp_tgt_off, n * sizeof(long long)) != cudaSuccess ||
-        (h->parts_on && (cudaMalloc(&h->d_parts, 4 * n * sizeof(CoarseOut)) != cudaSuccess ||
-                         cudaMalloc(&h->d_part_peaks, 4 * n * sizeof(float)) != cudaSuccess)) ||
-        cudaMalloc(&h->d_coarse, n * sizeof(CoarseOut)) != cudaSuccess ||
-        cudaMalloc(&h->d_coarse_peak, n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&h->d_offsets, n * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&h->d_diag, n * sizeof(PairDiag)) != cudaSuccess)
+    if (device_alloc(h, h->d_ref_off, n * sizeof(long long)) != cudaSuccess ||
+        device_alloc(h, h->d_tgt_off, n * sizeof(long long)) != cudaSuccess ||
+        device_alloc(h, h->d_amp_ref_off, n * sizeof(long long)) != cudaSuccess ||
+        device_alloc(h, h->d_amp_tgt_off, n * sizeof(long long)) != cudaSuccess ||
+        (h->parts_on && (device_alloc(h, h->d_parts, 4 * n * sizeof(CoarseOut)) != cudaSuccess ||
+                         device_alloc(h, h->d_part_peaks, 4 * n * sizeof(float)) != cudaSuccess)) ||
+        device_alloc(h, h->d_coarse, n * sizeof(CoarseOut)) != cudaSuccess ||
+        device_alloc(h, h->d_coarse_peak, n * sizeof(float)) != cudaSuccess ||
+        device_alloc(h, h->d_offsets, n * sizeof(float2)) != cudaSuccess ||
+        device_alloc(h, h->d_diag, n * sizeof(PairDiag)) != cudaSuccess)
         return fail(h, AMPCOR_E_NOMEM, "allocating per-pair device buffers");
     h->cap = n;
     return AMPCOR_OK;
@@ -795,6 +817,17 @@ void blocked_scratch(const ampcor_handle* h, size_t& parts, size_t& blocks, size
 
 constexpr size_t kChunkWave = 148 * 4;  // pairs: four to a multiprocessor
 
+// bytes of chunk scratch per pair
+size_t pair_scratch(const ampcor_handle* h)
+{
+    size_t parts, blocks, cells;
+    blocked_scratch(h, parts, blocks, cells);
+    const size_t tiles = (size_t)h->Rf * h->Rf + (size_t)h->Wf * h->Wf + (size_t)h->Cf * h->Cf;
+    const size_t stats = h->form == kFormTensor ? (size_t)h->C * h->C + (size_t)h->Cf * h->Cf : 0;
+    return (tiles + stats + parts + cells) * sizeof(float) + blocks * 2 * sizeof(double) +
+           (h->form == kFormSpectral ? 3 * sizeof(TileStat) : 0);
+}
+
 // The chunk of pairs whose refined amplitudes are resident at once, unless configured or set by
 // AMPCOR_CHUNK: as many waves as keep the scratch of all their pairs within a gigabyte, at least
 // one.  Each chunk costs five launches whose last waves leave multiprocessors idle, and reading the
@@ -808,12 +841,13 @@ size_t default_chunk(const ampcor_handle* h)
         if (v > 0) return (size_t)v;
     }
     if (h->chunk_short) return kChunkWave;
-    size_t parts, blocks, cells;
-    blocked_scratch(h, parts, blocks, cells);
-    const size_t tiles = (size_t)h->Rf * h->Rf + (size_t)h->Wf * h->Wf + (size_t)h->Cf * h->Cf;
-    const size_t stats = h->form == kFormTensor ? (size_t)h->C * h->C + (size_t)h->Cf * h->Cf : 0;
-    const size_t pair = (tiles + stats + parts + cells) * sizeof(float) + blocks * 2 * sizeof(double);
-    return std::max<size_t>(1, ((size_t)1 << 30) / (pair * kChunkWave)) * kChunkWave;
+    return std::max<size_t>(1, ((size_t)1 << 30) / (pair_scratch(h) * kChunkWave)) * kChunkWave;
+}
+
+// whether the scratch held is that of a default chunk of several waves
+bool default_chunk_waves(const ampcor_handle* h)
+{
+    return h->chunk_cap > kChunkWave && !h->chunk_override && !std::getenv("AMPCOR_CHUNK");
 }
 
 void free_chunk_scratch(ampcor_handle* h)
@@ -876,8 +910,10 @@ int alloc_chunk_scratch(ampcor_handle* h, size_t n)
 
 // The scratch of a job whose pairs the worker is sized for (ensure_pairs): a chunk's, or less where
 // the worker's largest job is smaller, so that a smaller job does not leave a later one short.  A
-// default chunk of several waves that the device cannot hold beside the caller's data gives way
-// to one wave, for good: no later call tries again.
+// default chunk of several waves takes at most an eighth of the device memory that is free, so that
+// a worker leaves room to the caller and to other workers; where it finds less, or the device holds it
+// back all the same, one wave does, for good: no later call tries again.  Called after a job's other
+// buffers, which a job cannot do without, have been allocated.
 int ensure_refined(ampcor_handle* h)
 {
     const bool chosen = h->chunk_override || std::getenv("AMPCOR_CHUNK");
@@ -886,12 +922,18 @@ int ensure_refined(ampcor_handle* h)
         const size_t n = std::min(h->chunk, std::max<size_t>(h->cap, 1));
         if (h->d_refined && h->chunk_cap >= n) return AMPCOR_OK;
         free_chunk_scratch(h);
+        size_t room = 0, all = 0;
+        if (!chosen && n > kChunkWave &&
+            (cudaMemGetInfo(&room, &all) != cudaSuccess || n * pair_scratch(h) > room / 8)) {
+            cudaGetLastError();
+            h->chunk_short = true;
+            continue;
+        }
         const int rc = alloc_chunk_scratch(h, n);
         if (rc != AMPCOR_E_NOMEM || chosen || n <= kChunkWave) return rc;
         h->chunk_short = true;
     }
 }
-
 
 int ensure_fine_out(ampcor_handle* h, size_t pairs)
 {
@@ -899,7 +941,7 @@ int ensure_fine_out(ampcor_handle* h, size_t pairs)
     cudaFree(h->d_fine_out);
     h->d_fine_out = nullptr;
     h->fine_cap = 0;
-    if (cudaMalloc(&h->d_fine_out, std::max<size_t>(pairs, 1) * sizeof(FineOut)) != cudaSuccess)
+    if (device_alloc(h, h->d_fine_out, std::max<size_t>(pairs, 1) * sizeof(FineOut)) != cudaSuccess)
         return fail(h, AMPCOR_E_NOMEM, "allocating refined maxima");
     h->fine_cap = std::max<size_t>(pairs, 1);
     return AMPCOR_OK;
@@ -988,9 +1030,8 @@ int run_tensor(ampcor_handle* h, const PairSource& src, long long pairs, float2*
                PairDiag* diag, float* coarse_surfaces, float* refined_surfaces, cudaStream_t st)
 {
     if (pairs == 0) return AMPCOR_OK;
-    int rc = ensure_refined(h);
-    if (rc) return rc;
-    if ((rc = ensure_fine_out(h, (size_t)pairs))) return rc;
+    int rc = ensure_fine_out(h, (size_t)pairs);
+    if (rc || (rc = ensure_refined(h))) return rc;
     const RealTiles rt{h->d_refined, h->refined_stride, 0, (long long)h->Rf * h->Rf};
     for (long long c0 = 0; c0 < pairs; c0 += (long long)h->chunk) {
         const unsigned n = (unsigned)std::min<long long>((long long)h->chunk, pairs - c0);
@@ -1111,9 +1152,8 @@ void pad_lines(ampcor_handle* h, PairSource& src)
 
 int spec_rasters(ampcor_handle* h, const PairSource& src, long long pairs, SpecRasters& r)
 {
-    int rc = ensure_refined(h);
+    int rc = ensure_fine_out(h, (size_t)pairs);
     if (rc) return rc;
-    if ((rc = ensure_fine_out(h, (size_t)pairs))) return rc;
     r.shared = src.ref_base == src.tgt_base;
     r.padded = src.amp_ref_off != nullptr;
     r.ref_pitch = r.padded ? src.amp_ref_stride : src.ref_stride;
@@ -1142,7 +1182,7 @@ int spec_rasters(ampcor_handle* h, const PairSource& src, long long pairs, SpecR
             return rc;
         r.inv_c = InvSource{h->d_inv_raster, r.tgt_off, r.tgt_pitch};
     }
-    return AMPCOR_OK;
+    return ensure_refined(h);
 }
 
 // amplitudes of samples [ref_lo, ref_hi) of the reference source and [tgt_lo, tgt_hi) of the
@@ -1380,6 +1420,9 @@ int run_spectral(ampcor_handle* h, const PairSource& src, long long pairs, float
 int run_pipeline(ampcor_handle* h, const PairSource& src, long long pairs, float2* offsets,
                  PairDiag* diag, float* coarse_surfaces, float* refined_surfaces, cudaStream_t st)
 {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+    if (capture != cudaStreamCaptureStatusNone) h->captured = true;
     int rc;
     switch (h->form) {
         case kFormSpectral:
@@ -1683,7 +1726,7 @@ int ampcor_adjust(ampcor_handle* h, const float** offsets)
     if (rc) return rc;
     CK(h, cudaSetDevice(h->prm.device), "cudaSetDevice");
     const size_t cells = (size_t)h->R * h->R + (size_t)h->W * h->W;
-    if (!h->d_arena) CK(h, cudaMalloc(&h->d_arena, std::max<size_t>(P * cells, 1) * sizeof(float2)), "allocating the device arena");
+    if (!h->d_arena) CK(h, device_alloc(h, h->d_arena, std::max<size_t>(P * cells, 1) * sizeof(float2)), "allocating the device arena");
     if (!h->h_offsets) CK(h, cudaMallocHost(&h->h_offsets, std::max<size_t>(2 * P, 1) * sizeof(float)), "allocating the offset field");
     if ((rc = ensure_pairs(h, P))) return rc;
     cudaStream_t st = h->stream;
@@ -1873,14 +1916,14 @@ int ampcor_correlate_host(ampcor_handle* h, const ampcor_job* j)
         cudaFree(h->d_ref_raster);
         h->d_ref_raster = nullptr;
         h->raster_bytes_ref = 0;
-        CK(h, cudaMalloc(&h->d_ref_raster, rb), "allocating the reference raster");
+        CK(h, device_alloc(h, h->d_ref_raster, rb), "allocating the reference raster");
         h->raster_bytes_ref = rb;
     }
     if (h->raster_bytes_tgt < tb) {
         cudaFree(h->d_tgt_raster);
         h->d_tgt_raster = nullptr;
         h->raster_bytes_tgt = 0;
-        CK(h, cudaMalloc(&h->d_tgt_raster, tb), "allocating the secondary raster");
+        CK(h, device_alloc(h, h->d_tgt_raster, tb), "allocating the secondary raster");
         h->raster_bytes_tgt = tb;
     }
     if ((rc = grow(h, h->d_ulhc, h->ulhc_cap, 4 * j->pairs, "pair corners"))) return rc;
