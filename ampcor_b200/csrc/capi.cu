@@ -1438,6 +1438,17 @@ int run_pipeline(ampcor_handle* h, const PairSource& src, long long pairs, float
     return rc;
 }
 
+// the expired waits that were read into h_status are an error, and count once
+int expired_waits(ampcor_handle* h, cudaStream_t st)
+{
+    const unsigned int n = h->h_status[1];
+    if (!n) return AMPCOR_OK;
+    CK(h, cudaMemsetAsync(h->d_tc_err, 0, sizeof(unsigned int), st), "resetting the error counter");
+    CK(h, cudaStreamSynchronize(st), "resetting the error counter");
+    return fail(h, AMPCOR_E_CUDA,
+                std::to_string(n) + " tile pair(s) or resident blocks timed out in a bounded device wait");
+}
+
 cudaStream_t pick(ampcor_handle* h, void* stream)
 {
     return stream ? (cudaStream_t)stream : h->stream;
@@ -1742,7 +1753,11 @@ int ampcor_adjust(ampcor_handle* h, const float** offsets)
         CK(h, cudaMemcpyAsync(h->h_offsets, h->d_offsets, 2 * P * sizeof(float), cudaMemcpyDeviceToHost, st),
            "harvesting the offset field");
     }
+    // (the expired waits only: adding tiles leaves no pair out of bounds)
+    CK(h, cudaMemcpyAsync(h->h_status + 1, h->d_tc_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, st),
+       "reading the error counter");
     CK(h, cudaStreamSynchronize(st), "running the correlation pipeline");
+    if ((rc = expired_waits(h, st))) return rc;
     *offsets = h->h_offsets;
     return AMPCOR_OK;
 }
@@ -1802,13 +1817,8 @@ int ampcor_synchronize(ampcor_handle* h, void* stream)
     CK(h, cudaMemcpyAsync(h->h_status, h->d_bad, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st),
        "reading the error counters");
     CK(h, cudaStreamSynchronize(st), "running the correlation pipeline");
-    const unsigned int bad = h->h_status[0], tcerr = h->h_status[1];
-    if (tcerr) {
-        CK(h, cudaMemsetAsync(h->d_tc_err, 0, sizeof(unsigned int), st), "resetting the error counter");
-        CK(h, cudaStreamSynchronize(st), "resetting the error counter");
-        return fail(h, AMPCOR_E_CUDA, std::to_string(tcerr) +
-                           " tile pair(s) or resident blocks timed out in a bounded device wait");
-    }
+    const unsigned int bad = h->h_status[0];
+    if (const int rc = expired_waits(h, st)) return rc;
     if (bad) {
         CK(h, cudaMemsetAsync(h->d_bad, 0, sizeof(unsigned int), st), "resetting the bounds counter");
         CK(h, cudaStreamSynchronize(st), "resetting the bounds counter");
@@ -1932,8 +1942,9 @@ int ampcor_correlate_host(ampcor_handle* h, const ampcor_job* j)
     cudaStream_t st = h->stream;
     if (h->form == kFormSpectral && j->pairs >= 2 * kHostBands && !j->coarse_surfaces && !j->refined_surfaces &&
         j->ref != j->tgt) {
-        if ((rc = correlate_host_banded(h, j))) return rc;
-        return ampcor_synchronize(h, st);
+        rc = correlate_host_banded(h, j);
+        if (h->inject_timeouts > 0) --h->inject_timeouts;
+        return rc ? rc : ampcor_synchronize(h, st);
     }
     CK(h, cudaMemcpyAsync(h->d_ref_raster, j->ref, rb, cudaMemcpyHostToDevice, st), "uploading the reference raster");
     CK(h, cudaMemcpyAsync(h->d_tgt_raster, j->tgt, tb, cudaMemcpyHostToDevice, st), "uploading the secondary raster");

@@ -208,8 +208,9 @@ int ampcor_configure(ampcor_handle* handle, int form, uint64_t chunk);
    nothing completes, bounded at about a millisecond: every wait of those kernels is bounded in
    time, and an expired wait stops the kernel cleanly and is reported.  The kernels issue no work
    after it and write no offsets for those batches (a staged coarse stage leaves its pairs
-   refinement corners inside their windows), and the ampcor_synchronize() that ends each of them
-   returns AMPCOR_E_CUDA with a time-out message; the worker stays usable.  0 switches it off. */
+   refinement corners inside their windows), and the ampcor_synchronize(), ampcor_adjust() or
+   ampcor_correlate_host() that ends each of them returns AMPCOR_E_CUDA with a time-out message; the
+   worker stays usable.  0 switches it off. */
 int ampcor_inject_timeout(ampcor_handle* handle, int batches);
 
 /* The number of pairs refined per chunk. */
