@@ -1321,7 +1321,8 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
             if (bc_st)
                 CK(h, launch_spec_block_staged(h->bc.tile_st, h->bc.nb, (unsigned)h->sms, st, cs, c0, n, src.ref_off,
                                                st_raw, reinterpret_cast<const float2*>(h->d_tw_c), h->d_part,
-                                               h->d_scal, h->d_tc_err, &bwc, &bcc, 1),
+                                               h->d_scal, h->d_tc_err, &bwc, &bcc, 1,
+                                               h->inject_timeouts > 0 ? 1 : 0),
                    "launching the staged blocked coarse correlation");
             else
                 CK(h, launch_spec_block(h->bc.tile, h->bc.nb, n * (unsigned)h->bc.K, st, cs, c0, n, src.ref_off,
@@ -1376,7 +1377,8 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
             if (bf_st)
                 CK(h, launch_spec_block_staged(h->bf.tile_st, h->bf.nb, (unsigned)h->sms, st, fs, c0, n, src.ref_off,
                                                st_chip, reinterpret_cast<const float2*>(h->d_tw_f), h->d_part,
-                                               h->d_scal, h->d_tc_err, &bwf, &bcf, 0),
+                                               h->d_scal, h->d_tc_err, &bwf, &bcf, 0,
+                                               h->inject_timeouts > 0 ? 1 : 0),
                    "launching the staged blocked fine correlation");
             else
                 CK(h, launch_spec_block(h->bf.tile, h->bf.nb, n * (unsigned)h->bf.K, st, fs, c0, n, src.ref_off,

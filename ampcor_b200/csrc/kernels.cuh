@@ -339,11 +339,13 @@ cudaError_t launch_spec_block(const SpecGeom& tile, int nb, unsigned blocks, cud
                               float* part, double* scal);
 // the same through the copy engine, resident CTAs walking the blocks (part: C^2 floats per pair where
 // tile.acc): wmap and cmap map the window and chip sources, 2-D over the amplitude rasters with boxes
-// of stage_rs x W and (R + 6 & ~3) x R floats, or (raster 0) 3-D over the refined tiles, a pair deep
+// of stage_rs x W and (R + 6 & ~3) x R floats, or (raster 0) 3-D over the refined tiles, a pair deep;
+// stall as of launch_spec_staged
 cudaError_t launch_spec_block_staged(const SpecGeom& tile, int nb, unsigned sms, cudaStream_t st, SpecSource src,
                                      long long pair0, long long pairs, const long long* valid,
                                      const TileStat* cstat, const float2* tw, float* part, double* scal,
-                                     unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster);
+                                     unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster,
+                                     int stall);
 int spec_reduce_smem(int C);
 // kp: partial surfaces per pair
 cudaError_t launch_spec_reduce(const SpecGeom& full, int K, int kp, unsigned blocks, cudaStream_t st,

@@ -1330,7 +1330,7 @@ __global__ void __launch_bounds__(kSpecThreads, 1)
 spec_block_staged_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
                          int nb, const TileStat* cstat, const float2* tw_g, float* part, double* scal,
                          unsigned int* errs, const __grid_constant__ CUtensorMap wmap,
-                         const __grid_constant__ CUtensorMap cmap, int raster)
+                         const __grid_constant__ CUtensorMap cmap, int raster, int stall)
 {
     extern __shared__ __align__(16) unsigned char ssm[];
     constexpr int NT = kSpecThreads, NW = NT / 32, N = N1 * N2, RS = N + 1;
@@ -1358,9 +1358,16 @@ spec_block_staged_kernel(SpecSource src, long long pair0, long long pairs, const
     if (tid == 0) {
         s_err = 0;
         mbar_init(bar, 1);
+        mbar_init(bar + 2, 1);  // completed by nothing: the wait of a failure-detection test
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    // a failure-detection test, as in spec_staged_kernel: the CTA skips its blocks
+    if (stall) {
+        mbar_wait(bar + 2, 0u, &s_err, kStallCycles);
+        __syncthreads();
+    }
+    const bool run = !stall || !s_err;
     // item n of this CTA: chunk pair b and its block k; false past the end
     auto item = [&](long long n, long long& b, int& k) {
         const long long t = ACC ? (blockIdx.x + n / K * gridDim.x) * K + n % K : blockIdx.x + n * gridDim.x;
@@ -1412,13 +1419,13 @@ spec_block_staged_kernel(SpecSource src, long long pair0, long long pairs, const
     };
     long long b;
     int k;
-    bool inflight = item(0, b, k);
+    bool inflight = run && item(0, b, k);
     if (tid == 0 && inflight) {
         look(0);
         issue();
     }
     uint32_t parity = 0;
-    for (long long n = 0; item(n, b, k); ++n) {
+    for (long long n = 0; run && item(n, b, k); ++n) {
         const long long p = pair0 + b;
         const bool ok = valid[p] >= 0;
         long long bn;
@@ -1805,14 +1812,14 @@ cudaError_t launch_spec_block(const SpecGeom& tile, int nb, unsigned blocks, cud
 cudaError_t launch_spec_block_staged(const SpecGeom& tile, int nb, unsigned sms, cudaStream_t st, SpecSource src,
                                      long long pair0, long long pairs, const long long* valid,
                                      const TileStat* cstat, const float2* tw, float* part, double* scal,
-                                     unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster)
+                                     unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster, int stall)
 {
     if (pairs <= 0) return cudaSuccess;
     const long long units = tile.acc ? pairs : pairs * nb * nb;
     const unsigned blocks = (unsigned)std::min<long long>(units, std::max(1u, sms));
     auto run = [&](auto kernel) {
         kernel<<<blocks, kSpecThreads, tile.smem_staged, st>>>(src, pair0, pairs, valid, tile, nb, cstat, tw, part,
-                                                               scal, errs, *wmap, *cmap, raster);
+                                                               scal, errs, *wmap, *cmap, raster, stall);
         return cudaGetLastError();
     };
 #define AMPCOR_SPEC_CASE(NN, A, B)                                                          \

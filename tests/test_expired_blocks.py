@@ -1,4 +1,4 @@
-"""Expired waits of a 128 px chip's job in the calls that wait by themselves (needs a
+"""Expired waits of the staged blocked kernels and of the calls that wait by themselves (needs a
 B200): a 128 px chip's stages time out on a barrier that nothing completes, before any copy is
 issued, in a raster job, the pair-by-pair interface and a banded host job; the call reports it, and
 the same worker's next call gives the offsets of the one before."""
@@ -57,4 +57,19 @@ def test_expired_wait_is_reported(name, pairs):
             run(worker, ulhc)
         assert "AMPCOR_E_CUDA" in str(e.value) and "timed out" in str(e.value)
         np.testing.assert_array_equal(run(worker, ulhc), want)
+    worker.close()
+
+
+def test_the_blocked_kernels_time_out_themselves():
+    """More waits run out than the zoom and the other staged kernels of a batch have CTAs."""
+    ulhc = corners(40)
+    worker = Worker(40, (R, R), (W, W), refine_factor=2, refine_margin=8, zoom_factor=8)
+    worker.inject_timeout(1)
+    with pytest.raises(Error) as e:
+        calls()["raster"](worker, ulhc)
+    expired = int(str(e.value).split(": ", 1)[1].split()[0])
+    # coarse: a CTA per pair (summed blocks); fine: a CTA per block and multiprocessor; the zoom: a CTA
+    # per pair at most
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert 40 + min(4 * 40, sms) < expired <= 40 + min(4 * 40, sms) + 40
     worker.close()
