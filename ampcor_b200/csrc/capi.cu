@@ -2036,14 +2036,9 @@ int ampcor_configure(ampcor_handle* h, int form, uint64_t chunk)
     }
     const bool switching = form != -1 && form != h->form;
     if (form != -1) h->form = form;
-    if (chunk && chunk != h->chunk) {
-        // the chunk scratch is sized on first use
-        free_chunk_scratch(h);
-        h->chunk_override = (size_t)chunk;
-    } else if (switching && h->d_refined) {
-        // a form switch needs the chunk scratch of the new form
-        free_chunk_scratch(h);
-    }
+    // the chunk scratch is sized on first use, and by the form
+    if ((chunk && chunk != h->chunk) || (switching && h->d_refined)) free_chunk_scratch(h);
+    if (chunk) h->chunk_override = (size_t)chunk;
     return AMPCOR_OK;
 }
 
