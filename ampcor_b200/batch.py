@@ -120,7 +120,7 @@ class UnevenBatch:
 
                 forms = ("plain",) if plain else ("spectral", "tensor", "plain")
                 self.tuning[j.geometry] = run_tune(w, j.ref, j.tgt, u, forms=forms,
-                                                   chunks=(296, 592, 1184), reps=1,
+                                                   chunks={296, 592, 1184, w.chunk}, reps=1,
                                                    use_cache=False)
             self.workers[j.geometry] = w
         self.graph = None
