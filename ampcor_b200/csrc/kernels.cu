@@ -506,16 +506,8 @@ coarse_kernel(PairSource src, long long pair0, long long pairs, NccGeom g, int m
     int bi;
     surface_argmax(gam, g.C * g.C, smem + g.off_red, bv, bi);
     if (threadIdx.x == 0) {
-        // nudge.cu:107-140 (argument roles from nudge.cu:57: old = W, new = R + 2m)
         const int u = bi / g.C, v = bi - u * g.C;
-        const int E = g.R + 2 * m;
-        int left = v - m;
-        if (left < 0) left = 0;
-        if (left + E > g.W) left = g.W - E;
-        int top = u - m;
-        if (top < 0) top = 0;
-        if (top + E > g.W) top = g.W - E;
-        out[p] = CoarseOut{u, v, top, left};
+        out[p] = nudged(u, v, g.R, g.W, m);
         coarse_peak[p] = bv;
     }
 }

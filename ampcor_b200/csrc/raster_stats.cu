@@ -279,9 +279,7 @@ join_parts_kernel(const CoarseOut* parts, const float* peaks, long long stride, 
                 better(bv, bi, peaks[k * stride + p], (c.u + (k >> 1) * s) * C + c.v + (k & 1) * s);
         }
         const int u = bi / C, v = bi - u * C;
-        // nudge.cu:107-140
-        const int left = min(max(v - m, 0), W - E), top = min(max(u - m, 0), W - E);
-        coarse[p] = CoarseOut{u, v, top, left};
+        coarse[p] = nudged(u, v, E - 2 * m, W, m);
         coarse_peak[p] = bv;
     }
     if (surfaces) {

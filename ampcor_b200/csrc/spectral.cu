@@ -559,16 +559,7 @@ __device__ void spec_result(const SpecOut& out, long long p, int R, int W, int C
 {
     const int u = bi / C, v = bi - u * C;
     if (out.stage == 0) {
-        // nudge.cu:107-140 (argument roles from nudge.cu:57: old = W, new = R + 2m)
-        const int m = out.m;
-        const int E = R + 2 * m;
-        int left = v - m;
-        if (left < 0) left = 0;
-        if (left + E > W) left = W - E;
-        int top = u - m;
-        if (top < 0) top = 0;
-        if (top + E > W) top = W - E;
-        out.coarse[p] = CoarseOut{u, v, top, left};
+        out.coarse[p] = nudged(u, v, R, W, out.m);
         out.coarse_peak[p] = bv;
     } else {
         out.fine[p] = FineOut{u, v, bv, 0.0f};
@@ -1660,23 +1651,7 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
     float* gam = out.stage == 1 ? out.gam + (long long)blockIdx.x * CC : nullptr;
     spec_surface<kThreads>(G, red, g, invs, inv_sigma, cst.mean, ebox, chip, src.chip_stride, win,
                            src.win_stride, gam, surf, bv, bi, flagged);
-    if (tid == 0) {
-        const int u = bi / C, v = bi - u * C;
-        if (out.stage == 0) {
-            // nudge.cu:107-140 (argument roles from nudge.cu:57: old = W, new = R + 2m)
-            const int E = R + 2 * out.m;
-            int left = v - out.m;
-            if (left < 0) left = 0;
-            if (left + E > W) left = W - E;
-            int top = u - out.m;
-            if (top < 0) top = 0;
-            if (top + E > W) top = W - E;
-            out.coarse[p] = CoarseOut{u, v, top, left};
-            out.coarse_peak[p] = bv;
-        } else {
-            out.fine[p] = FineOut{u, v, bv, 0.0f};
-        }
-    }
+    if (tid == 0) spec_result(out, p, R, W, C, bv, bi);
 }
 
 }  // namespace

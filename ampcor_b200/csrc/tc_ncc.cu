@@ -460,16 +460,8 @@ tc_coarse_kernel(PairSource src, long long pair0, long long pairs, TcGeom g, con
     const SurfaceMax sm = tc_surface(tl, g, inv + (long long)blockIdx.x * g.C * g.C, false, nullptr,
                                      surfaces ? surfaces + (size_t)p * g.C * g.C : nullptr, err);
     if (threadIdx.x == 0) {
-        // nudge.cu:107-140
         const int u = sm.i / g.C, v = sm.i - u * g.C;
-        const int E = g.R + 2 * m;
-        int left = v - m;
-        if (left < 0) left = 0;
-        if (left + E > g.W) left = g.W - E;
-        int top = u - m;
-        if (top < 0) top = 0;
-        if (top + E > g.W) top = g.W - E;
-        out[p] = CoarseOut{u, v, top, left};
+        out[p] = nudged(u, v, g.R, g.W, m);
         coarse_peak[p] = sm.v;
     }
 }
