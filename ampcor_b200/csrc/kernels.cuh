@@ -95,6 +95,16 @@ struct CoarseOut {
     int top, left;     // nudged corner of the refinement neighbourhood inside the window
 };
 
+// The coarse cell (u, v) and the corner of its refinement neighbourhood, nudged into the window
+// (nudge.cu:107-140; argument roles from nudge.cu:57: old = W, new = R + 2m).  A surface without a
+// maximum (NaN) hands in a cell far outside: its corner still lies inside.
+__host__ __device__ inline CoarseOut nudged(int u, int v, int R, int W, int m)
+{
+    const int room = W - (R + 2 * m);
+    auto corner = [&](int x) { return x < m ? 0 : x - m > room ? room : x - m; };
+    return CoarseOut{u, v, corner(u), corner(v)};
+}
+
 // optional per-pair diagnostics (matches ampcor_pair_diag in the public header)
 struct PairDiag {
     int coarse_u, coarse_v;

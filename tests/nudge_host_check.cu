@@ -4,7 +4,7 @@
 #include <climits>
 #include <cstdio>
 
-#include "tile_common.cuh"
+#include "kernels.cuh"
 
 using namespace ampcor_b200;
 
