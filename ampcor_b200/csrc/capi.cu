@@ -1274,17 +1274,19 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         TileStat* const st_win = st_chip + h->chunk_cap;       // the refined windows
         const float2* tab = reinterpret_cast<const float2*>(h->d_tw_refine);
         const bool deramp = (h->prm.flags & AMPCOR_FLAG_DERAMP) != 0;
-        // the chips' refinement needs no coarse result, and gives the coarse stage their statistics
+        const double flat = h->bf.on ? 0.0 : kFlatChip;
         cudaEvent_t b = mark(h, st);
         if (h->refine_fft) {
             CK(h, launch_refine_half(h->R, n, st, src.ref_base, src.ref_off, src.ref_stride, nullptr, c0, n,
-                                     src.ref_off, tab, h->d_refined, h->refined_stride, 0, deramp, st_raw, st_chip),
+                                     src.ref_off, tab, h->d_refined, h->refined_stride, 0, deramp, flat, st_chip),
                "launching the chip refinement");
             cudaEvent_t b1 = mark(h, st);
             keep(h, 1, b, b1);
             b = b1;
-        } else {
-            CK(h, launch_spec_chip_stats(n, st, cs, c0, n, src.ref_off, h->R, st_raw),
+        }
+        // (chips of one tile, or of parts, are summed by the correlation itself)
+        if (h->bc.on && !parts_st) {
+            CK(h, launch_spec_chip_stats(n, st, cs, c0, n, src.ref_off, h->R, 0.0, st_raw),
                "launching the chip statistics");
             cudaEvent_t b1 = mark(h, st);
             keep(h, 3, b, b1);
@@ -1301,7 +1303,7 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
                 const SpecOut po{0, h->m, h->d_parts + k * cap, h->d_part_peaks + k * cap, nullptr, nullptr, surf};
                 CK(h, launch_spec_staged(h->spp_st, (unsigned)h->sms, st, ps, c0, n, src.ref_off,
                                          InvSource{r.inv_c.base + part_at(k), r.inv_c.off, r.inv_c.stride},
-                                         reinterpret_cast<const float2*>(h->d_tw_p), po, st_raw, nullptr, h->d_tc_err,
+                                         reinterpret_cast<const float2*>(h->d_tw_p), po, nullptr, nullptr, h->d_tc_err,
                                          &pw[k], &pc, &pi[k], h->inject_timeouts > 0 ? 1 : 0),
                    "launching a part of the coarse correlation");
             }
@@ -1334,7 +1336,7 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         } else {
             if (coarse_st)
                 CK(h, launch_spec_staged(h->spc_st, (unsigned)h->sms, st, cs, c0, n, src.ref_off, r.inv_c,
-                                         reinterpret_cast<const float2*>(h->d_tw_c), co, st_raw, nullptr, h->d_tc_err,
+                                         reinterpret_cast<const float2*>(h->d_tw_c), co, nullptr, nullptr, h->d_tc_err,
                                          &wmap, &cmap, &imap, h->inject_timeouts > 0 ? 1 : 0),
                    "launching the staged coarse correlation");
             else
@@ -1347,7 +1349,7 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         if (h->refine_fft) {
             CK(h, launch_refine_half(h->E, n, st, src.tgt_base, src.tgt_off, src.tgt_stride, h->d_coarse, c0, n,
                                      src.ref_off, tab + 2 * h->R, h->d_refined, h->refined_stride,
-                                     (long long)h->Rf * h->Rf, deramp, nullptr, st_win),
+                                     (long long)h->Rf * h->Rf, deramp, 0.0, h->bf.on ? nullptr : st_win),
                "launching the window refinement");
         } else {
             refine_kernel<<<n, kThreads, h->refine_smem, st>>>(src, c0, n, h->d_coarse, h->ic, h->iw,
@@ -1358,10 +1360,9 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         cudaEvent_t e = mark(h, st);
         keep(h, 1, c, e);
         if (!h->refine_fft) {
-            const SpecSource wins{fs.win, fs.win_stride, nullptr, fs.win_step, fs.win, fs.win_stride, nullptr, fs.win_step};
-            CK(h, launch_spec_chip_stats(n, st, fs, c0, n, src.ref_off, h->Rf, st_chip),
+            CK(h, launch_spec_chip_stats(n, st, fs, c0, n, src.ref_off, h->Rf, flat, st_chip),
                "launching the refined chip statistics");
-            CK(h, launch_spec_chip_stats(n, st, wins, c0, n, src.ref_off, h->Wf, st_win),
+            CK(h, launch_spec_window_stats(n, st, fs, c0, n, src.ref_off, h->Wf, st_win),
                "launching the refined window statistics");
             cudaEvent_t e1 = mark(h, st);
             keep(h, 4, e, e1, 2);

@@ -310,13 +310,16 @@ struct InvSource {
     long long stride;
 };
 
-// FP64 statistics of an amplitude tile: its mean, 1/|t - mean| (0 for a tile flat to its own
-// rounding) and |t - mean|
+// statistics of an amplitude tile, FP64: its mean; of a chip, 1/|r - mean| (0 for a constant one);
+// of a window, |t - mean| from above (it only scales the transform's error bound)
 struct TileStat {
     double mean;
     double inv_norm;
     double norm;
 };
+// the share of a chip's sum of squares up to which its deviations are its amplitudes' rounding: a
+// refined chip that one tile correlates counts as constant up to here
+constexpr double kFlatChip = 1e-14;
 
 // the transform lengths that are compiled, with their radices
 bool spec_radices(int n, int& n1, int& n2);
@@ -328,18 +331,21 @@ cudaError_t spec_set_smem_limits();
 // phases over N of the frequencies at the transform's positions.
 bool refine_half_radices(int n, int& n1, int& n2);
 cudaError_t refine_half_set_smem_limits();
-// Statistics of the tiles, one per chunk-local pair: raw (unless null) of the amplitudes as they are,
-// fine of the upsampled ones.
+// stat (unless null): the statistics of the upsampled tiles, one per chunk-local pair; a chip's from
+// FP64 sums of every amplitude (chip_stat with `flat`).
 cudaError_t launch_refine_half(int n, unsigned blocks, cudaStream_t st, const float2* base, const long long* off,
                                long long stride, const CoarseOut* coarse, long long pair0, long long pairs,
                                const long long* valid, const float2* tab, float* refined, long long refined_stride,
-                               long long out_off, bool deramp, TileStat* raw, TileStat* fine);
+                               long long out_off, bool deramp, double flat, TileStat* stat);
 
 // blocked spectral correlation (windows too large for one tile; see spectral.cu): per chunk of
 // pairs the chip statistics, the placement statistics when no raster gives them, the partial
 // numerators of every (pair, chip block) and their per-pair reduction to the stage's outputs
+// (the chips of src, R x R samples, or its windows, R x R too)
 cudaError_t launch_spec_chip_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                   long long pairs, const long long* valid, int R, TileStat* out);
+                                   long long pairs, const long long* valid, int R, double flat, TileStat* out);
+cudaError_t launch_spec_window_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
+                                     long long pairs, const long long* valid, int R, TileStat* out);
 int spec_tile_stats_rows(int W, int C, int& smem);
 cudaError_t launch_spec_tile_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
                                    long long pairs, const long long* valid, int R, int W, float* inv);
@@ -371,7 +377,7 @@ bool spec_shared(int n, int& threads, int& ctas);
 // counted in errs.  Refined tiles: wmap and cmap null, no statistics given.  Raster windows:
 // wmap, cmap and imap 2-D maps of the secondary and reference amplitude rasters and of the
 // secondary's box statistics (inv) with boxes of stage_rs x W, (R + 6 & ~3) x R and inv_rs x C
-// floats.  cstat (and wstat for refined tiles): the statistics of the chips (and windows).  stall:
+// floats.  cstat and wstat, for refined tiles: the statistics of the chips and windows.  stall:
 // the failure-detection test's wait on a barrier that nothing completes.
 cudaError_t launch_spec_staged(const SpecGeom& g, unsigned sms, cudaStream_t st, SpecSource src,
                                long long pair0, long long pairs, const long long* valid, InvSource inv,

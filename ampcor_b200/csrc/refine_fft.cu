@@ -20,6 +20,7 @@
 // us with packed sums and strips of 32 rows, 1,561 us with the tiles' statistics on the way out (which
 // save the correlation kernels more); 3,844 pairs of 128 and 144 samples 3,235 -> 1,912 us.
 #include <algorithm>
+#include <type_traits>
 
 #include "fft.cuh"
 #include "kernels.cuh"
@@ -57,11 +58,11 @@ struct HalfGeom {
 
 // one tile of every pair of a chunk: the chip (coarse == nullptr) or the nudged window.  tab: the
 // N twiddles exp(-2 pi i m / N), then P in the order of the transform's positions.
-template <int N1, int N2, int NT, int SR, int CTAS, bool DERAMP>
+template <int N1, int N2, int NT, int SR, int CTAS, bool DERAMP, bool CHIP>
 __global__ void __launch_bounds__(NT, CTAS)
 refine_half_kernel(const float2* base, const long long* off, long long stride, const CoarseOut* coarse,
                    long long pair0, long long pairs, const long long* valid, const float2* tab, float* refined,
-                   long long refined_stride, long long out_off, TileStat* raw, TileStat* fine)
+                   long long refined_stride, long long out_off, double flat, TileStat* stat)
 {
     using G = HalfGeom<N1, N2, NT, SR, CTAS>;
     constexpr int N = G::N, F = 2 * N, RS = G::RS;
@@ -76,7 +77,7 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
     float2* ph = tw + N;
     double* red = reinterpret_cast<double*>(ph + N);
     const float2* src = base + off[p];
-    if (coarse) {
+    if constexpr (!CHIP) {
         const CoarseOut co = coarse[p];
         src += co.top * stride + co.left;
     }
@@ -127,12 +128,14 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
         mu = make_float2((float)(ta / ((double)N * N)), (float)(tb / ((double)N * N)));
     }
 
-    // The amplitudes' sums and sums of squares, of the tile itself (even) and of the rest: FP32 per
-    // thread about one of the tile's own amplitudes, FP64 from there on, so that a strong steady
-    // return costs no digits of their variance
-    const float pivot = amplitude(X[(tid % N) * RS + (7 * tid) % N]);
-    float e1 = 0.0f, e2 = 0.0f, r1 = 0.0f, r2 = 0.0f;
-    int lines = 0;  // tasks done: N1 outputs of each kind per task
+    // The sums and sums of squares of the upsampled amplitudes.  A chip's make its correlations'
+    // mean and norm: FP64 for every amplitude.  A window's mean only conditions the transform and its
+    // norm only scales the error bound: FP32 per thread about one of the tile's own amplitudes (so that
+    // a strong steady return costs no digits of their variance), FP64 from there on.
+    using Sum = std::conditional_t<CHIP, double, float>;
+    const Sum pivot = CHIP ? 0.0f : amplitude(X[(tid % N) * RS + (7 * tid) % N]);
+    Sum r1 = 0, r2 = 0;
+    int lines = 0;  // tasks done: 2 N1 outputs per task
     // Output rows 2 y + odd: row y of the tile (less m, with add back on: the tile as it was loaded
     // gives its own amplitudes exactly) and S of it, a strip at a time
     auto rows = [&](int odd, float2 m, float2 add) {
@@ -167,16 +170,11 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
                     const float2 z = make_float2(amplitude(make_float2(e.x + add.x, e.y + add.y)),
                                                  amplitude(make_float2(v.x + mu.x, v.y + mu.y)));
                     o[n] = z;
-                    const float de = z.x - pivot, dv = z.y - pivot;
-                    if (odd == 0) {
-                        e1 += de;
-                        e2 = fmaf(de, de, e2);
-                    } else {
-                        r1 += de;
-                        r2 = fmaf(de, de, r2);
-                    }
+                    const Sum de = CHIP ? (Sum)z.x : z.x - pivot, dv = CHIP ? (Sum)z.y : z.y - pivot;
+                    r1 += de;
+                    r2 = fma(de, de, r2);
                     r1 += dv;
-                    r2 = fmaf(dv, dv, r2);
+                    r2 = fma(dv, dv, r2);
                 });
                 ++lines;
             }
@@ -192,26 +190,27 @@ refine_half_kernel(const float2* base, const long long* off, long long stride, c
     __syncthreads();
     for (int t = tid; t < N * N2; t += NT) fft::inv_a<N1, N2>(X + t % N, RS, t / N, tw);
     __syncthreads();
-    const int even = lines * N1;  // outputs of the tile itself, and as many beside them
     rows(1, zero, mu);
-    const double pv = pivot, ne = even, nr = lines * 2 * N1 - even;
-    double sum[4] = {ne * pv + (double)e1, (double)e2 + pv * (2.0 * (double)e1 + ne * pv),
-                     nr * pv + (double)r1, (double)r2 + pv * (2.0 * (double)r1 + nr * pv)};
+    if (!stat) return;
+    const double pv = pivot, nr = lines * 2 * N1;
+    double sum[3] = {nr * pv + (double)r1, (double)r2 + pv * (2.0 * (double)r1 + nr * pv), (double)r2};
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < 3; ++q) {
         sum[q] = warp_sum(sum[q]);
         if (lane == 0) red[4 * warp + q] = sum[q];
     }
     __syncthreads();
-    if (tid < 2) {
-        // thread 0: the tile itself, thread 1: all four phases
-        double s1 = 0.0, s2 = 0.0;
+    if (tid == 0) {
+        double s1 = 0.0, s2 = 0.0, about = 0.0;
         for (int w = 0; w < NT / 32; ++w) {
-            s1 += red[4 * w] + (tid ? red[4 * w + 2] : 0.0);
-            s2 += red[4 * w + 1] + (tid ? red[4 * w + 3] : 0.0);
+            s1 += red[4 * w];
+            s2 += red[4 * w + 1];
+            about += red[4 * w + 2];
         }
-        TileStat* to = tid ? fine : raw;
-        if (to) to[blockIdx.x] = tile_stat(s1, s2, tid ? (double)F * F : (double)N * N);
+        // (a window's slack: the FP32 rounding of a thread's sum of squares, at most 100 terms for the
+        // windows of up to 80 samples whose norm is used, 6e-6 relative)
+        const double n = (double)F * F;
+        stat[blockIdx.x] = CHIP ? chip_stat(0.0, s1, s2, n, flat) : window_stat(0.0, s1, s2, n, 1e-5 * about);
     }
 }
 
@@ -249,9 +248,12 @@ bool refine_half_radices(int n, int& n1, int& n2)
 cudaError_t refine_half_set_smem_limits()
 {
     cudaError_t e = cudaSuccess;
-#define AMPCOR_REFINE_CASE(NN, A, B, NT, SR, CTAS)                                                              \
-    for (auto* k : {refine_half_kernel<A, B, NT, SR, CTAS, false>, refine_half_kernel<A, B, NT, SR, CTAS, true>}) \
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
+#define AMPCOR_REFINE_CASE(NN, A, B, NT, SR, CTAS)                                                            \
+    for (auto* k : {refine_half_kernel<A, B, NT, SR, CTAS, false, false>,                                     \
+                    refine_half_kernel<A, B, NT, SR, CTAS, true, false>,                                      \
+                    refine_half_kernel<A, B, NT, SR, CTAS, false, true>,                                      \
+                    refine_half_kernel<A, B, NT, SR, CTAS, true, true>})                                      \
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,        \
                                                        HalfGeom<A, B, NT, SR, CTAS>::smem);
     AMPCOR_REFINE_TILES(AMPCOR_REFINE_CASE)
 #undef AMPCOR_REFINE_CASE
@@ -261,14 +263,17 @@ cudaError_t refine_half_set_smem_limits()
 cudaError_t launch_refine_half(int n, unsigned blocks, cudaStream_t st, const float2* base, const long long* off,
                                long long stride, const CoarseOut* coarse, long long pair0, long long pairs,
                                const long long* valid, const float2* tab, float* refined, long long refined_stride,
-                               long long out_off, bool deramp, TileStat* raw, TileStat* fine)
+                               long long out_off, bool deramp, double flat, TileStat* stat)
 {
 #define AMPCOR_REFINE_CASE(NN, A, B, NT, SR, CTAS)                                                             \
     if (n == NN) {                                                                                             \
-        (deramp ? refine_half_kernel<A, B, NT, SR, CTAS, true> : refine_half_kernel<A, B, NT, SR, CTAS, false>) \
-            <<<blocks, NT, HalfGeom<A, B, NT, SR, CTAS>::smem, st>>>(base, off, stride, coarse, pair0, pairs,  \
-                                                                     valid, tab, refined, refined_stride, out_off, \
-                                                                     raw, fine);                              \
+        auto* kernel = coarse ? deramp ? refine_half_kernel<A, B, NT, SR, CTAS, true, false>                   \
+                                       : refine_half_kernel<A, B, NT, SR, CTAS, false, false>                  \
+                              : deramp ? refine_half_kernel<A, B, NT, SR, CTAS, true, true>                    \
+                                       : refine_half_kernel<A, B, NT, SR, CTAS, false, true>;                  \
+        kernel<<<blocks, NT, HalfGeom<A, B, NT, SR, CTAS>::smem, st>>>(base, off, stride, coarse, pair0, pairs, \
+                                                                       valid, tab, refined, refined_stride,    \
+                                                                       out_off, flat, stat);                   \
         return cudaGetLastError();                                                                             \
     }
     AMPCOR_REFINE_TILES(AMPCOR_REFINE_CASE)

@@ -748,8 +748,9 @@ spec_kernel(SpecSource src, long long pair0, long long pairs, const long long* v
 // blockIdx.x + gridDim.x, ...: once a pair's inverse column pass is done (from then on its
 // correlation touches only the tile's first rows) the bulk-copy engine brings the next pair's
 // window (W x W dense floats, one cp.async.bulk completing on an mbarrier) into the tile's last
-// bytes, and the chip's bytes are sent toward L2.  The statistics of the chips and of the refined
-// windows come from the refinement, which forms them on the way out.  A pair then starts with its
+// bytes, and the chip's bytes are sent toward L2.  The statistics of the refined chips and windows
+// come from the refinement, which forms them on the way out; a raster's chip is summed here, from the
+// amplitudes that are correlated.  A pair starts with its
 // window in shared memory: the placement statistics of a refined window read from the staged copy
 // (the tile's first bytes are their scratch), then one pass that writes the window and the chip
 // (loaded from L2 meanwhile) into the tile; the first transform pass takes the window's mean (and
@@ -912,12 +913,12 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         const bool ok = valid[p] >= 0;
         const float* chip = spec_chip(src, pair0, b);
         const float* win = spec_win(src, pair0, b);
-        // the chip's mean (as two floats) and 1/|r'|; a refined window's mean and |t'|
-        const double mean_c = cstat[b].mean;
-        const float mc_hi = (float)mean_c, mc_lo = (float)(mean_c - (double)mc_hi);
-        const float inv_sigma = (float)cstat[b].inv_norm;
-        float sx = 0.0f, norm_w = 0.0f;
+        // refined tiles: the chip's mean and 1/|r'|, the window's mean and |t'|
+        double mean_c = 0.0;
+        float inv_sigma = 0.0f, sx = 0.0f, norm_w = 0.0f;
         if constexpr (!RASTER) {
+            mean_c = cstat[b].mean;
+            inv_sigma = (float)cstat[b].inv_norm;
             sx = (float)wstat[b].mean;
             norm_w = (float)wstat[b].norm;
         }
@@ -962,7 +963,24 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             // the raster's placement statistics, copied with the window, into their C x C layout
             for (int u = warp; u < C; u += NW)
                 for (int v = lane; v < C; v += 32) invs[u * C + v] = inv_raw[u * g.inv_rs + xo + v];
+            // the chip's FP64 mean (spec_kernel's first sweep)
+            double c1 = 0.0;
+#pragma unroll
+            for (int j = 0; j < JN; ++j)
+                if (warp + NW * j < R)
+#pragma unroll
+                    for (int i = 0; i < IN; ++i)
+                        if (32 * i < R) c1 += (double)cr[j][i];
+            c1 = warp_sum(c1);
+            if (lane == 0) red[warp] = c1;
+            __syncthreads();
+            double t1 = 0.0;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) t1 += red[w];
+            mean_c = t1 / ((double)R * (double)R);
+            __syncthreads();
         }
+        const float mc_hi = (float)mean_c, mc_lo = (float)(mean_c - (double)mc_hi);
         auto wat = [&](int y, int x) {
             if constexpr (RASTER)
                 return stage[y * SW + xo + x];
@@ -976,19 +994,23 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
             staged_box_stats<NT>(stage, g, sx, Zf, reinterpret_cast<double*>(Zf + ((2 * C * W + 3) & ~3)), invs);
 
         // window (real parts) and chip (imaginary parts; its bytes were sent toward L2 with the
-        // window) into the tile, zeros around them.  Raster windows: the chip goes in zero-mean, and
-        // the window's sums of t - k and (t - k)^2 about a pivot k (its first sample) are taken on
-        // the way, as spec_kernel takes them (in another order).  Refined tiles: the first transform
-        // pass takes the chip's mean off.
+        // window) into the tile, zeros around them.  Raster windows: the chip goes in zero-mean and
+        // |r'|^2 is summed from the very values that go in, as spec_kernel sums it; the window's sums of
+        // t - k and (t - k)^2 about a pivot k (its first sample) are taken on the way, as spec_kernel
+        // takes them (in another order).  Refined tiles: the first transform pass takes the chip's
+        // mean off.
         const float pk = wat(0, 0);
         if constexpr (!RASTER) load_chip();
-        float sw = 0.0f, sw2 = 0.0f;
+        float sw = 0.0f, sw2 = 0.0f, sc2 = 0.0f;
         auto put = [&](int j, int i, float t) {
             const int y = warp + NW * j, x = lane + 32 * i;
             if (y < N && x < N) {
                 float c = cr[j][i];
                 if constexpr (RASTER) {
-                    if (y < R && x < R) c = (c - mc_hi) - mc_lo;
+                    if (y < R && x < R) {
+                        c = (c - mc_hi) - mc_lo;
+                        sc2 = fmaf(c, c, sc2);
+                    }
                     if (y < W && x < W) {
                         const float d = t - pk;
                         sw += d;
@@ -1028,18 +1050,21 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
         }
         fft::Centre centre{sx, W};
         if constexpr (RASTER) {
-            const double d1 = warp_sum((double)sw), d2 = warp_sum((double)sw2);
+            const double d0 = warp_sum((double)sc2), d1 = warp_sum((double)sw), d2 = warp_sum((double)sw2);
             if (lane == 0) {
-                red[2 * warp] = d1;
-                red[2 * warp + 1] = d2;
+                red[3 * warp] = d0;
+                red[3 * warp + 1] = d1;
+                red[3 * warp + 2] = d2;
             }
             __syncthreads();
-            double s1 = 0.0, s2 = 0.0;
+            double ss = 0.0, s1 = 0.0, s2 = 0.0;
 #pragma unroll
             for (int w = 0; w < NW; ++w) {
-                s1 += red[2 * w];
-                s2 += red[2 * w + 1];
+                ss += red[3 * w];
+                s1 += red[3 * w + 1];
+                s2 += red[3 * w + 2];
             }
+            inv_sigma = ss > 0.0 ? (float)(1.0 / sqrt(ss)) : 0.0f;
             const double cells = (double)W * (double)W;
             centre.sx = (float)((double)pk + s1 / cells);
             norm_w = sqrtf((float)(fmax(s2 - s1 * s1 / cells, 0.0) + 1e-5 * s2));
@@ -1080,7 +1105,7 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
 
         float* surf = out.surfaces ? out.surfaces + (size_t)p * C * C : nullptr;
         float* gam = out.stage == 1 ? out.gam + b * C * C : nullptr;
-        spec_surface<NT>(G, red, g, invs, inv_sigma, (double)mc_hi + (double)mc_lo, ebox, chip, cs, win, ws, gam, surf, bv, bi,
+        spec_surface<NT>(G, red, g, invs, inv_sigma, mean_c, ebox, chip, cs, win, ws, gam, surf, bv, bi,
                                    flagged);
         if (tid == 0) spec_result(out, p, R, W, C, bv, bi);
     }
@@ -1135,10 +1160,12 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
 // sum c (t - s_k), and the pair's numerator is the sum over blocks plus sum_k s_k sum_k c, c the
 // centred chip values the block placed in its tile.
 
-// one CTA of 256 threads per pair: FP64 mean and 1/|r - mean| of the R x R chip
+// one CTA of 256 threads per pair: the FP64 statistics of the R x R chip, or (window) window, from sums
+// about its first sample (the differences and their squares are exact, so that a strong steady return
+// costs their sums no digits)
 __global__ void __launch_bounds__(256)
-spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, int R,
-                       TileStat* out)
+spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, int R, bool window,
+                       double flat, TileStat* out)
 {
     __shared__ double red[16];
     if (blockIdx.x >= pairs) return;
@@ -1148,12 +1175,13 @@ spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const l
         if (tid == 0) out[blockIdx.x] = TileStat{0.0, 0.0, 0.0};
         return;
     }
-    const float* chip = spec_chip(src, pair0, blockIdx.x);
-    const long long cs = src.chip_stride;
+    const float* chip = window ? spec_win(src, pair0, blockIdx.x) : spec_chip(src, pair0, blockIdx.x);
+    const long long cs = window ? src.win_stride : src.chip_stride;
+    const double pivot = __ldg(chip);
     double s1 = 0.0, s2 = 0.0;
     for (int y = warp; y < R; y += 8)
         for (int x = lane; x < R; x += 32) {
-            const double v = __ldg(chip + y * cs + x);
+            const double v = (double)__ldg(chip + y * cs + x) - pivot;
             s1 += v;
             s2 += v * v;
         }
@@ -1170,7 +1198,9 @@ spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const l
             a += red[2 * w];
             b += red[2 * w + 1];
         }
-        out[blockIdx.x] = tile_stat(a, b, (double)R * (double)R);
+        // (a window's slack: the rounding of up to 2^16 FP64 terms)
+        const double n = (double)R * (double)R;
+        out[blockIdx.x] = window ? window_stat(pivot, a, b, n, 1e-11 * b) : chip_stat(pivot, a, b, n, flat);
     }
 }
 
@@ -1497,21 +1527,20 @@ spec_block_staged_kernel(SpecSource src, long long pair0, long long pairs, const
 #pragma unroll
                     for (int i = 0; i < IN; ++i) put(q0 + q, i, v[q][i]);
         }
-        // FP64 sums over the block (FP32 over a thread's samples of a row): sum c, sum c^2 of the
-        // centred chip block, sum t - k, sum (t - k)^2 of the sub-window
+        // FP64 sums over the block: sum c, sum c^2 of the centred chip block (every sample in FP64:
+        // the level of a strong steady return multiplies the first), sum t - k, sum (t - k)^2 of the
+        // sub-window (FP32 per thread)
         double a[4] = {0.0, 0.0, (double)sw, (double)sw2};
 #pragma unroll
         for (int j = 0; j < JN; ++j)
-            if (warp + NW * j < B) {
-                float c1 = 0.0f, c2 = 0.0f;
+            if (warp + NW * j < B)
 #pragma unroll
-                for (int i = 0; i < IN; ++i) {
-                    c1 += cr[j][i];
-                    c2 = fmaf(cr[j][i], cr[j][i], c2);
-                }
-                a[0] += (double)c1;
-                a[1] += (double)c2;
-            }
+                for (int i = 0; i < IN; ++i)
+                    if (32 * i < B) {
+                        const double c = cr[j][i];
+                        a[0] += c;
+                        a[1] = fma(c, c, a[1]);
+                    }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             a[q] = warp_sum(a[q]);
@@ -1739,9 +1768,16 @@ cudaError_t spec_set_smem_limits()
 }
 
 cudaError_t launch_spec_chip_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                   long long pairs, const long long* valid, int R, TileStat* out)
+                                   long long pairs, const long long* valid, int R, double flat, TileStat* out)
 {
-    spec_chip_stats_kernel<<<blocks, 256, 0, st>>>(src, pair0, pairs, valid, R, out);
+    spec_chip_stats_kernel<<<blocks, 256, 0, st>>>(src, pair0, pairs, valid, R, false, flat, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_spec_window_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
+                                     long long pairs, const long long* valid, int R, TileStat* out)
+{
+    spec_chip_stats_kernel<<<blocks, 256, 0, st>>>(src, pair0, pairs, valid, R, true, 0.0, out);
     return cudaGetLastError();
 }
 

@@ -93,15 +93,19 @@ __device__ void block_argmax_n(float& bv, int& bi, float* redf, int* redi)
     __syncthreads();
 }
 
-// the statistics of a tile of n amplitudes from their FP64 sum and sum of squares: S2 - S1^2 / n; a
-// tile flat to within its own rounding (a constant: its deviations are exactly 0) has norm 0
-__device__ __forceinline__ TileStat tile_stat(double s1, double s2, double n)
+// The statistics of a chip of n amplitudes from the FP64 sums of r - k and (r - k)^2 about a pivot k:
+// |r - mean|^2 = S2 - S1^2 / n.  A chip whose share of the amplitudes' sum of squares that is stays at
+// or below `flat` counts as constant.
+__device__ __forceinline__ TileStat chip_stat(double k, double s1, double s2, double n, double flat)
 {
-    const double mean = s1 / n;
-    double ss = s2 - s1 * mean;
-    if (!(ss > 1e-14 * s2)) ss = 0.0;
-    const double norm = sqrt(ss);
-    return TileStat{mean, norm > 0.0 ? 1.0 / norm : 0.0, norm};
+    const double ss = s2 - s1 * (s1 / n), all = s2 + k * (2.0 * s1 + n * k);
+    return TileStat{k + s1 / n, ss > flat * all ? 1.0 / sqrt(ss) : 0.0, 0.0};
+}
+// The statistics of a window from the same sums, its norm from above: slack covers the rounding of
+// the sums.
+__device__ __forceinline__ TileStat window_stat(double k, double s1, double s2, double n, double slack)
+{
+    return TileStat{k + s1 / n, 0.0, sqrt(fmax(s2 - s1 * (s1 / n), 0.0) + slack)};
 }
 
 // exclusive prefix sum of row[0..n) written in place, with the total in row[n] (one warp)
