@@ -824,7 +824,7 @@ size_t pair_scratch(const ampcor_handle* h)
     blocked_scratch(h, parts, blocks, cells);
     const size_t tiles = (size_t)h->Rf * h->Rf + (size_t)h->Wf * h->Wf + (size_t)h->Cf * h->Cf;
     const size_t stats = h->form == kFormTensor ? (size_t)h->C * h->C + (size_t)h->Cf * h->Cf : 0;
-    return (tiles + stats + parts + cells) * sizeof(float) + blocks * 2 * sizeof(double) +
+    return (tiles + stats + parts + cells) * sizeof(float) + blocks * kBlockScalars * sizeof(double) +
            (h->form == kFormSpectral ? 3 * sizeof(TileStat) : 0);
 }
 
@@ -903,7 +903,7 @@ int alloc_chunk_scratch(ampcor_handle* h, size_t n)
     blocked_scratch(h, parts, blocks, cells);
     if (blocks && (cudaMalloc(&h->d_inv_blk, n * cells * sizeof(float)) != cudaSuccess ||
                    cudaMalloc(&h->d_part, n * parts * sizeof(float)) != cudaSuccess ||
-                   cudaMalloc(&h->d_scal, n * blocks * 2 * sizeof(double)) != cudaSuccess))
+                   cudaMalloc(&h->d_scal, n * blocks * kBlockScalars * sizeof(double)) != cudaSuccess))
         return scratch_fail(h, "allocating blocked-correlation scratch");
     return AMPCOR_OK;
 }

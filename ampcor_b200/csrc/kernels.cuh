@@ -362,6 +362,7 @@ cudaError_t launch_spec_block_staged(const SpecGeom& tile, int nb, unsigned sms,
                                      const TileStat* cstat, const float2* tw, float* part, double* scal,
                                      unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster,
                                      int stall);
+constexpr int kBlockScalars = 3;  // doubles per (pair, block) beside its partial numerators
 int spec_reduce_smem(int C);
 // kp: partial surfaces per pair
 cudaError_t launch_spec_reduce(const SpecGeom& full, int K, int kp, unsigned blocks, cudaStream_t st,

@@ -1157,8 +1157,10 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
 // a fixed order, normalises them, bounds the transform error and takes the first maximum, as
 // spec_kernel does for a tile that fits.  The chip is centred on the whole chip's mean
 // (spec_chip_stats_kernel), each sub-window on its own mean s_k: the block then computes
-// sum c (t - s_k), and the pair's numerator is the sum over blocks plus sum_k s_k sum_k c, c the
-// centred chip values the block placed in its tile.
+// sum c (t - s_k), c the centred chip values the block placed in its tile, and the pair's numerator is
+// the sum over blocks of that plus (s_k - s) sum_k c, for any s, since a whole centred chip sums to 0.
+// s is the mean of the s_k: the c do not sum to 0 but to their roundings, and a steady return's level
+// must not multiply those (128 px chips under a return of 300: off by up to 8.4e-6 with s = 0).
 
 // one CTA of 256 threads per pair: the FP64 statistics of the R x R chip, or (window) window, from sums
 // about its first sample (the differences and their squares are exact, so that a strong steady return
@@ -1222,7 +1224,7 @@ spec_tile_stats_kernel(SpecSource src, long long pair0, long long pairs, const l
 
 // The partial numerators of one chip block of one pair (CTA b K + k): g is the tile of a block
 // (g.R = B, g.W = B + C - 1, g.C = C), nb blocks per axis.  part: C^2 floats per (pair, block),
-// already scaled; scal: two doubles per (pair, block), s_k sum_k c and |c| |t - s_k|.
+// already scaled; scal: kBlockScalars doubles per (pair, block), s_k, sum_k c and |c| |t - s_k|.
 template <int N1, int N2>
 __global__ void __launch_bounds__(kSpecThreads, 1)
 spec_block_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
@@ -1330,8 +1332,10 @@ spec_block_kernel(SpecSource src, long long pair0, long long pairs, const long l
         out[idx] = Z[u * RS + v].x * scale;
     }
     if (tid == 0) {
-        scal[2 * ((long long)b * K + k)] = (double)centre.sx * a0;
-        scal[2 * ((long long)b * K + k) + 1] = sqrt(a1 * st);
+        double* to = scal + kBlockScalars * ((long long)b * K + k);
+        to[0] = (double)centre.sx;
+        to[1] = a0;
+        to[2] = sqrt(a1 * st);
     }
 }
 
@@ -1560,9 +1564,10 @@ spec_block_staged_kernel(SpecSource src, long long pair0, long long pairs, const
                 a3 += red[4 * w + 3];
             }
             const double st = fmax(a3 - a2 * a2 / cells, 0.0) + 1e-5 * a3;
-            double* to = scal + 2 * (b * K + k);
-            to[0] = (double)centre.sx * a0;
-            to[1] = sqrt(a1 * st);
+            double* to = scal + kBlockScalars * (b * K + k);
+            to[0] = (double)centre.sx;
+            to[1] = a0;
+            to[2] = sqrt(a1 * st);
         }
         const float scale = (float)(1.0 / (4.0 * (double)N * (double)N));
         float* out = part + (ACC ? b : b * K + k) * C * C;
@@ -1623,11 +1628,13 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
 #pragma unroll 4
             for (int v = lane; v < C; v += 32) cp_async4(invs + u * C + v, inv_b + u * is + v);
     }
-    const double* sc = scal + 2 * (long long)blockIdx.x * K;
-    double corr = 0.0, errs = 0.0;
+    const double* sc = scal + kBlockScalars * (long long)blockIdx.x * K;
+    double level = 0.0, corr = 0.0, errs = 0.0;
+    for (int k = 0; k < K; ++k) level += sc[kBlockScalars * k];
+    level /= (double)K;
     for (int k = 0; k < K; ++k) {
-        corr += sc[2 * k];
-        errs += sc[2 * k + 1];
+        corr += (sc[kBlockScalars * k] - level) * sc[kBlockScalars * k + 1];
+        errs += sc[kBlockScalars * k + 2];
     }
     const TileStat cst = cstat[blockIdx.x];
     const float inv_sigma = (float)cst.inv_norm;
@@ -1665,7 +1672,8 @@ spec_reduce_kernel(SpecSource src, long long pair0, long long pairs, const long 
             const int idx = idx0 + q * kThreads;
             if (idx >= CC) break;
             const float inv_box = invs[idx];
-            const float gv = (float)num[q] * inv_box * inv_sigma;
+            // (one rounding instead of three)
+            const float gv = (float)(num[q] * ((double)inv_box * cst.inv_norm));
             G[idx] = gv;
             if (ebox * inv_box > kSpecTol)
                 flagged = 1;

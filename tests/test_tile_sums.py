@@ -126,3 +126,14 @@ def test_bright_scatterers_in_the_refined_chip(R):
     best = want.flatten(1).argmax(1)[:, None]
     error = (surf.double().flatten(1).gather(1, best) - want.flatten(1).gather(1, best)).abs()
     assert error.max() < 1e-6
+
+
+@pytest.mark.parametrize("M", [24, 32, 64])
+def test_blocks_under_a_steady_return(M):
+    """The blocks of a 128 px chip (spectra summed, or block by block) keep a level of 300 out of the
+    numerators: what remains is the rounding of the amplitudes' centred values and the transform, 5e-7 as
+    of one tile."""
+    R = 128
+    ref, tgt = (a + np.float32(300.0) for a in scene(R + 2 * M + 64))
+    got, chip, win = coarse(R, M, ref, tgt, serve.grid_corners(*ref.shape, R, M, 31))
+    assert (got - ncc(chip, win)).abs().max() < 5e-7
