@@ -500,11 +500,8 @@ bool plan_zoom(int Cf, int z, ZoomGeomCols& g)
     double k2 = 0.0;
     for (int n = 1; n <= Cf / 2; ++n) k2 += 2.0 / Cf * std::pow(2.0 * M_PI * n / Cf, 4);
     g.curv = (float)(1.00001 * std::sqrt(k2) * std::pow((double)g.s / z, 2) / 8.0);
-    // G, the kept columns of T, a value per sample, the reduction slots, the kept columns and rows
     g.g_rows = (Cf + 11) / 12 * 12;
-    g.team_bytes = (int)((g.g_rows + kZoomCols) * row + round4(g.J) * 4L + 64 + 2 * round4(g.Z) * 4L);
-    g.teams = (int)std::min<long>(kZoomTeams, (limit - g.off_team) / g.team_bytes);
-    return g.teams > 0;
+    return g.off_team + 4L * zoom_team(g, 3, 1).floats <= limit;
 }
 
 double dirichlet(int N, double d);

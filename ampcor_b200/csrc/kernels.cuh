@@ -193,11 +193,9 @@ __global__ void tc_fine_kernel(RealTiles t, long long pair0, long long pairs, Tc
                                const float* inv, const long long* ref_off, FineOut* fout,
                                float* gam, float* surfaces, unsigned int* err);
 
-// the zoom of the refined surfaces (zoom_kernel): teams of kZoomTeam threads (or three times as many),
-// a pair each, at most kZoomTeams (3) to a CTA, kZoomCols columns of the zoomed surface at a time
-constexpr int kZoomTeam = 96;
+// the zoom of the refined surfaces (zoom_kernel): teams of three warps, at most kZoomTeams to a CTA, or of
+// nine, a pair each; the columns of the zoomed surface in batches of some sets of kZoomCols
 constexpr int kZoomTeams = 8;
-constexpr int zoom_teams(int groups) { return groups == 1 ? kZoomTeams : 3; }
 constexpr int kZoomCols = 36;
 
 struct ZoomGeomCols {
@@ -207,10 +205,56 @@ struct ZoomGeomCols {
     float curv;      // h^2 / 8 kappa: the rise between two samples h = s / z apart, per unit of norm
     int kp4;         // float4 per row of U, G and T: odd, so that rows a thread apart hit other banks
     int g_rows;      // rows of a team's G: Cf rounded up to whole blocks of rows
-    int teams;       // teams per CTA that fit
-    int off_team;    // shared memory: U (Z rows), then team_bytes per team
-    int team_bytes;
+    int off_team;    // shared memory: U (Z rows), then the teams' own (zoom_team)
 };
+
+// a team's shared memory, in floats from its start: G first, then the parts below
+struct ZoomTeamLayout {
+    int T;      // the batch's kept columns of T, kp4 float4 each
+    int val;    // a value per sampled row or column, Jv of them, for each set (or group of three warps)
+    int far;    // per 12 columns of the batch and 24 rows of T: the largest squared distance from c
+    int red;    // reduction slots: three per warp, the number of kept columns, that of each set's kept rows
+    int cols;   // the kept columns, index | row of U << 16
+    int rows;   // per set the kept rows, the same
+    int Jv, Zv, nab;
+    int floats;
+};
+__host__ __device__ inline ZoomTeamLayout zoom_team(const ZoomGeomCols& g, int warps, int sets)
+{
+    auto up = [](int x) { return (x + 3) & ~3; };
+    ZoomTeamLayout l;
+    l.Jv = up(g.J);
+    l.Zv = up(g.Z);
+    l.nab = (g.Cf + 23) / 24;
+    l.T = g.g_rows * 4 * g.kp4;
+    l.val = l.T + sets * kZoomCols * 4 * g.kp4;
+    l.far = l.val + (sets > warps / 3 ? sets : warps / 3) * l.Jv;
+    l.red = l.far + up(sets * kZoomCols / 12 * l.nab);
+    l.cols = l.red + up(3 * warps + 1 + sets);
+    l.rows = l.cols + l.Zv;
+    l.floats = l.rows + sets * l.Zv;
+    return l;
+}
+
+// the same of zoom_wide_kernel's one team: G first, then a value per sampled column, reduction slots, the
+// kept columns, and per warp 24 columns of T, a value per sampled row and a list of rows
+constexpr int kWideWarps = 12;
+struct ZoomWideLayout {
+    int norm, red, cols, own, warp, Jv, floats;
+};
+__host__ __device__ inline ZoomWideLayout zoom_wide(const ZoomGeomCols& g)
+{
+    auto up = [](int x) { return (x + 3) & ~3; };
+    ZoomWideLayout l;
+    l.Jv = up(g.J);
+    l.norm = g.Cf * 4 * g.kp4;
+    l.red = l.norm + l.Jv;
+    l.cols = l.red + up(3 * kWideWarps + 2);
+    l.own = l.cols + up(g.Z);
+    l.warp = 24 * 4 * g.kp4 + l.Jv + up(g.Z);
+    l.floats = l.own + kWideWarps * l.warp;
+    return l;
+}
 
 // zoom of the refined surfaces of a chunk (Cf^2 floats per chunk-local pair), first maximum and
 // offsets.  u: s Jp rows of 4 kp4 floats, the interpolation matrix, zero past Cf.  stall != 0 (a
