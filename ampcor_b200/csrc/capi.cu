@@ -621,11 +621,10 @@ struct ampcor_handle {
     float* d_coarse_peak = nullptr;
     float2* d_offsets = nullptr;
     PairDiag* d_diag = nullptr;
-    // the bounds counter and the expired-wait counter, next to each other on the device, and where
-    // the host reads both (page-locked)
+    // the bounds counter and the expired-wait counter, in page-locked host memory that the kernels
+    // count in when there is something to report: a call that waits reads them with no copy
     unsigned int* d_bad = nullptr;
     unsigned int* d_tc_err = nullptr;
-    unsigned int* h_status = nullptr;
     // refined amplitudes of one chunk of pairs
     float* d_refined = nullptr;
     size_t chunk = 0;      // pairs per chunk
@@ -1438,13 +1437,19 @@ int run_pipeline(ampcor_handle* h, const PairSource& src, long long pairs, float
     return rc;
 }
 
-// the expired waits that were read into h_status are an error, and count once
-int expired_waits(ampcor_handle* h, cudaStream_t st)
+// a counter's value once the work before has been waited for; it starts anew
+unsigned int take(unsigned int* counter)
 {
-    const unsigned int n = h->h_status[1];
+    volatile unsigned int* c = counter;
+    const unsigned int n = *c;
+    if (n) *c = 0;
+    return n;
+}
+
+int expired_waits(ampcor_handle* h)
+{
+    const unsigned int n = take(h->d_tc_err);
     if (!n) return AMPCOR_OK;
-    CK(h, cudaMemsetAsync(h->d_tc_err, 0, sizeof(unsigned int), st), "resetting the error counter");
-    CK(h, cudaStreamSynchronize(st), "resetting the error counter");
     return fail(h, AMPCOR_E_CUDA,
                 std::to_string(n) + " tile pair(s) or resident blocks timed out in a bounded device wait");
 }
@@ -1627,10 +1632,9 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
         if ((e = upload(h->d_tw_refine, tw)) != cudaSuccess)
             return cuda_create_fail(e, "uploading refinement twiddles");
     }
-    if ((e = cudaMalloc(&h->d_bad, 2 * sizeof(unsigned int))) != cudaSuccess ||
-        (e = cudaMemset(h->d_bad, 0, 2 * sizeof(unsigned int))) != cudaSuccess ||
-        (e = cudaMallocHost(&h->h_status, 2 * sizeof(unsigned int))) != cudaSuccess)
+    if ((e = cudaMallocHost(&h->d_bad, 2 * sizeof(unsigned int))) != cudaSuccess)
         return cuda_create_fail(e, "allocating the error counters");
+    h->d_bad[0] = h->d_bad[1] = 0;
     h->d_tc_err = h->d_bad + 1;
     *out = h;
     return AMPCOR_OK;
@@ -1656,7 +1660,6 @@ int ampcor_destroy(ampcor_handle* h)
     cudaFree(h->d_coarse_peak);
     cudaFree(h->d_offsets);
     cudaFree(h->d_diag);
-    cudaFree(h->d_bad);
     cudaFree(h->d_refined);
     cudaFree(h->d_ref_raster);
     cudaFree(h->d_tgt_raster);
@@ -1680,7 +1683,7 @@ int ampcor_destroy(ampcor_handle* h)
     drop_marks(h);
     if (h->h_arena) cudaFreeHost(h->h_arena);
     if (h->h_offsets) cudaFreeHost(h->h_offsets);
-    if (h->h_status) cudaFreeHost(h->h_status);
+    if (h->d_bad) cudaFreeHost(h->d_bad);
     for (cudaEvent_t e : h->band_ev)
         if (e) cudaEventDestroy(e);
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
@@ -1754,10 +1757,8 @@ int ampcor_adjust(ampcor_handle* h, const float** offsets)
            "harvesting the offset field");
     }
     // (the expired waits only: adding tiles leaves no pair out of bounds)
-    CK(h, cudaMemcpyAsync(h->h_status + 1, h->d_tc_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, st),
-       "reading the error counter");
     CK(h, cudaStreamSynchronize(st), "running the correlation pipeline");
-    if ((rc = expired_waits(h, st))) return rc;
+    if ((rc = expired_waits(h))) return rc;
     *offsets = h->h_offsets;
     return AMPCOR_OK;
 }
@@ -1812,18 +1813,10 @@ int ampcor_synchronize(ampcor_handle* h, void* stream)
     if (!h) return AMPCOR_E_ARG;
     CK(h, cudaSetDevice(h->prm.device), "cudaSetDevice");
     cudaStream_t st = pick(h, stream);
-    // one copy into page-locked memory, then the one wait (two pageable copies waited each: 8 us more
-    // of a 64-pair call)
-    CK(h, cudaMemcpyAsync(h->h_status, h->d_bad, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st),
-       "reading the error counters");
     CK(h, cudaStreamSynchronize(st), "running the correlation pipeline");
-    const unsigned int bad = h->h_status[0];
-    if (const int rc = expired_waits(h, st)) return rc;
-    if (bad) {
-        CK(h, cudaMemsetAsync(h->d_bad, 0, sizeof(unsigned int), st), "resetting the bounds counter");
-        CK(h, cudaStreamSynchronize(st), "resetting the bounds counter");
+    if (const int rc = expired_waits(h)) return rc;
+    if (const unsigned int bad = take(h->d_bad))
         return fail(h, AMPCOR_E_BOUNDS, std::to_string(bad) + " tile pair(s) leave their raster; their offsets are NaN");
-    }
     return AMPCOR_OK;
 }
 
