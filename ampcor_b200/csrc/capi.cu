@@ -380,9 +380,9 @@ bool plan_spec_tile(int B, int S, int C, SpecGeom& g)
 // Where the summed spectrum of the blocks fits beside the tile, with the staged bytes at the tile's
 // end: a block's tile is free once its spectrum is summed, only the last block's inverse still uses
 // the first rows, so that its copy waits (`late`) if those reach the staged bytes.  Otherwise block
-// by block, where the staged bytes fit beside the rows of every inverse (searches of +-64 px, 129
-// placement rows of a 160-sample tile, keep spec_block_kernel: a copy after the inverse hides
-// nothing, 963 us against 914 for 900 pairs of 64 px chips).
+// by block, where the staged bytes fit beside the rows of every inverse (128 px chips in searches of
+// +-64 px, 129 placement rows of 160-sample tiles, keep spec_block_kernel: a copy after the inverse
+// hides nothing, 963 us against 914 for the blocks of 900 64 px chips).
 bool plan_spec_block_staged(int K, SpecGeom& g)
 {
     auto up = [](long x, long a) { return (x + a - 1) / a * a; };
@@ -419,7 +419,7 @@ bool plan_spec_block_staged(int K, SpecGeom& g)
         g.off_gam = (int)off;
         return off;
     };
-    if (K > 1 && N <= 128 && tile >= bytes) {
+    if (K > 1 && N >= kSumLeast && N <= kSumMost && tile >= bytes) {
         const long at = up(tile - bytes, 128);
         g.acc = 1;
         g.late = kept > at ? 1 : 0;

@@ -406,6 +406,9 @@ cudaError_t launch_spec_block_staged(const SpecGeom& tile, int nb, unsigned sms,
                                      const TileStat* cstat, const float2* tw, float* part, double* scal,
                                      unsigned int* errs, const CUtensorMap* wmap, const CUtensorMap* cmap, int raster,
                                      int stall);
+// tile lengths whose blocks' spectra are summed: the sum fits beside the tile up to 128 samples, and no
+// accepted window beyond one tile has blocks of fewer than 81 samples a side
+constexpr int kSumLeast = 96, kSumMost = 128;
 constexpr int kBlockScalars = 3;  // doubles per (pair, block) beside its partial numerators
 int spec_reduce_smem(int C);
 // kp: partial surfaces per pair

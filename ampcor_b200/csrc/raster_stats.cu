@@ -205,10 +205,7 @@ constexpr int box_smem()
 
 cudaError_t raster_set_smem_limits()
 {
-    cudaError_t e = cudaFuncSetAttribute(box_stats_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, box_smem<512>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(box_stats_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, box_smem<1024>());
-    return e;
+    return cudaFuncSetAttribute(box_stats_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, box_smem<512>());
 }
 
 cudaError_t launch_detect(cudaStream_t st, const float2* src, long long n, float* dst, const float2* src2,
@@ -234,8 +231,8 @@ cudaError_t launch_detect_lines(cudaStream_t st, const DetectLines& a, const Det
     return cudaGetLastError();
 }
 
-// columns of a CTA: at least twice the box
-static int box_threads(int R) { return R <= 96 ? 256 : R <= 256 ? 512 : 1024; }
+// columns of a CTA: at least twice the box (no chip of the spectral form has more than 160 samples a side)
+static int box_threads(int R) { return R <= 96 ? 256 : 512; }
 
 int box_block_rows(long long rows, long long samples, int R, unsigned sms)
 {
@@ -250,14 +247,13 @@ cudaError_t launch_box_stats(cudaStream_t st, const float* a, long long samples,
 {
     const int nt = box_threads(R);
     const long long cols = nt + 1 - R, first = row_lo / block_rows;
+    if (R > 256) return cudaErrorInvalidValue;
     if (samples < R || row_hi <= row_lo) return cudaSuccess;
     const dim3 grid((unsigned)((samples - R + cols) / cols), (unsigned)((row_hi + block_rows - 1) / block_rows - first));
     if (nt == 256)
         box_stats_kernel<256><<<grid, 256, box_smem<256>(), st>>>(a, (int)samples, (int)pitch, R, block_rows, (int)row_lo, (int)row_hi, inv);
-    else if (nt == 512)
-        box_stats_kernel<512><<<grid, 512, box_smem<512>(), st>>>(a, (int)samples, (int)pitch, R, block_rows, (int)row_lo, (int)row_hi, inv);
     else
-        box_stats_kernel<1024><<<grid, 1024, box_smem<1024>(), st>>>(a, (int)samples, (int)pitch, R, block_rows, (int)row_lo, (int)row_hi, inv);
+        box_stats_kernel<512><<<grid, 512, box_smem<512>(), st>>>(a, (int)samples, (int)pitch, R, block_rows, (int)row_lo, (int)row_hi, inv);
     return cudaGetLastError();
 }
 

@@ -7,11 +7,11 @@
 // So no 2 N-point transform is needed: of the four phases of the 2 N x 2 N result one is the tile
 // itself, and the others are S along the rows, S down the columns, and both.  S takes three
 // in-place passes over a line (fft.cuh): the transform's step A; its step B, P and the inverse's
-// step B in registers (`shift_middle`); the inverse's step A.  An upsampled tile costs 6 N lines of
-// S (N rows, N columns, N rows again) against N + N + N 2 N-point + 2 N 2 N-point transforms of
-// the padded form (a third of the arithmetic, half the passes), and needs the N x N tile and a
-// strip of rows in shared memory instead of a 2 N x N one, so that two to four CTAs share an SM
-// and the 96-160 sample tiles need no buffer in global memory.
+// step B in registers (`shift_middle`); the inverse's step A.  An upsampled tile costs 3 N lines of
+// S (N rows, N columns, N rows again), 6 N transforms of N points, against 2 N of N points and 3 N of
+// 2 N points in the padded form, and needs the N x N tile and a strip of rows in shared memory instead
+// of a 2 N x N one, so that two to eight CTAs share an SM for tiles up to 96 samples and the larger ones
+// need no buffer in global memory.
 //
 // What bounds it: instruction issue, with shared-memory wavefronts next (ncu, 80-sample tiles: 62 %
 // of issue slots, the FMA pipes 42 %, 10.7K wavefronts of 21K cycles a tile; 15 % of the time goes

@@ -1753,7 +1753,7 @@ cudaError_t spec_set_smem_limits()
         e = cudaFuncSetAttribute(spec_staged_kernel<A, B, false, kSpecThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
     if (e == cudaSuccess)          \
         e = cudaFuncSetAttribute(spec_block_kernel<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
-    if constexpr (NN <= 128)       \
+    if constexpr (NN >= kSumLeast && NN <= kSumMost) \
         if (e == cudaSuccess)      \
             e = cudaFuncSetAttribute(spec_block_staged_kernel<A, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit); \
     if constexpr (NN >= 128)       \
@@ -1843,7 +1843,7 @@ cudaError_t launch_spec_block_staged(const SpecGeom& tile, int nb, unsigned sms,
     };
 #define AMPCOR_SPEC_CASE(NN, A, B)                                                          \
     if (tile.N == NN) {                                                                     \
-        if constexpr (NN <= 128)                                                            \
+        if constexpr (NN >= kSumLeast && NN <= kSumMost)                                    \
             if (tile.acc) return run(spec_block_staged_kernel<A, B, true>);                 \
         if constexpr (NN >= 128)                                                            \
             if (!tile.acc) return run(spec_block_staged_kernel<A, B, false>);               \
