@@ -977,9 +977,9 @@ int run_plain(ampcor_handle* h, const PairSource& src, long long pairs, float2* 
     for (long long c0 = 0; c0 < pairs; c0 += (long long)h->chunk) {
         const long long n = std::min<long long>((long long)h->chunk, pairs - c0);
         a = mark(h, st);
-        refine_kernel<<<(unsigned)n, kThreads, h->refine_smem, st>>>(
+        refine_kernel<false><<<(unsigned)n, kThreads, h->refine_smem, st>>>(
             src, c0, n, h->d_coarse, h->ic, h->iw, h->d_chip_taps, h->d_win_taps, h->d_refined,
-            h->refined_stride, (h->prm.flags & AMPCOR_FLAG_DERAMP) ? 1 : 0);
+            h->refined_stride, (h->prm.flags & AMPCOR_FLAG_DERAMP) ? 1 : 0, 0.0, nullptr, nullptr);
         CK(h, cudaGetLastError(), "launching the refinement kernel");
         cudaEvent_t b = mark(h, st);
         keep(h, 1, a, b);
@@ -1040,9 +1040,11 @@ int run_tensor(ampcor_handle* h, const PairSource& src, long long pairs, float2*
                                                             coarse_surfaces, h->d_tc_err);
         cudaEvent_t c = mark(h, st);
         keep(h, 0, b, c);
-        refine_kernel<<<n, kThreads, h->refine_smem, st>>>(src, c0, n, h->d_coarse, h->ic, h->iw,
+        refine_kernel<false><<<n, kThreads, h->refine_smem, st>>>(src, c0, n, h->d_coarse, h->ic, h->iw,
                                                            h->d_chip_taps, h->d_win_taps,
-                                                           h->d_refined, h->refined_stride, (h->prm.flags & AMPCOR_FLAG_DERAMP) ? 1 : 0);
+                                                           h->d_refined, h->refined_stride,
+                                                           (h->prm.flags & AMPCOR_FLAG_DERAMP) ? 1 : 0, 0.0, nullptr,
+                                                           nullptr);
         cudaEvent_t d = mark(h, st);
         keep(h, 1, c, d);
         window_stats_real_kernel<<<n, kThreads, h->gsf.smem_bytes, st>>>(rt, n, h->gsf, h->d_inv_f);
@@ -1282,7 +1284,7 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
         }
         // (chips of one tile, or of parts, are summed by the correlation itself)
         if (h->bc.on && !parts_st) {
-            CK(h, launch_spec_chip_stats(n, st, cs, c0, n, src.ref_off, h->R, 0.0, st_raw),
+            CK(h, launch_spec_chip_stats(n, st, cs, c0, n, src.ref_off, h->R, st_raw),
                "launching the chip statistics");
             cudaEvent_t b1 = mark(h, st);
             keep(h, 3, b, b1);
@@ -1348,22 +1350,14 @@ int spec_pairs(ampcor_handle* h, const PairSource& src, const SpecRasters& r, lo
                                      (long long)h->Rf * h->Rf, deramp, 0.0, h->bf.on ? nullptr : st_win),
                "launching the window refinement");
         } else {
-            refine_kernel<<<n, kThreads, h->refine_smem, st>>>(src, c0, n, h->d_coarse, h->ic, h->iw,
-                                                               h->d_chip_taps, h->d_win_taps,
-                                                               h->d_refined, h->refined_stride, (h->prm.flags & AMPCOR_FLAG_DERAMP) ? 1 : 0);
+            refine_kernel<true><<<n, kThreads, h->refine_smem, st>>>(src, c0, n, h->d_coarse, h->ic, h->iw,
+                                                                     h->d_chip_taps, h->d_win_taps,
+                                                                     h->d_refined, h->refined_stride, deramp ? 1 : 0,
+                                                                     flat, st_chip, st_win);
             CK(h, cudaGetLastError(), "launching the refinement kernel");
         }
         cudaEvent_t e = mark(h, st);
         keep(h, 1, c, e);
-        if (!h->refine_fft) {
-            CK(h, launch_spec_chip_stats(n, st, fs, c0, n, src.ref_off, h->Rf, flat, st_chip),
-               "launching the refined chip statistics");
-            CK(h, launch_spec_window_stats(n, st, fs, c0, n, src.ref_off, h->Wf, st_win),
-               "launching the refined window statistics");
-            cudaEvent_t e1 = mark(h, st);
-            keep(h, 4, e, e1, 2);
-            e = e1;
-        }
         const SpecOut fo{1, 0, nullptr, nullptr, h->d_fine_out, h->d_gam, refined_surfaces};
         if (h->bf.on) {
             CK(h, launch_spec_tile_stats(n, st, fs, c0, n, src.ref_off, h->Rf, h->Wf, h->d_inv_blk),
@@ -1593,7 +1587,9 @@ int ampcor_create(const ampcor_params* p, ampcor_handle** out)
                                   kMaxSmem)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(fine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kMaxSmem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (e = cudaFuncSetAttribute(refine_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kMaxSmem)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(refine_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kMaxSmem)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(window_stats_cplx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kMaxSmem)) != cudaSuccess ||
@@ -2230,7 +2226,7 @@ extern "C" int ampcor_correlate_noalloc(const ampcor_params* p, const ampcor_job
     const int kMaxSmem = 227 * 1024;
     if ((e = cudaFuncSetAttribute(coarse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)) != cudaSuccess ||
         (e = cudaFuncSetAttribute(fine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)) != cudaSuccess ||
-        (e = cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)) != cudaSuccess)
+        (e = cudaFuncSetAttribute(refine_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)) != cudaSuccess)
         return noalloc_fail(errbuf, errlen, AMPCOR_E_CUDA, "configuring kernel shared memory", e);
     // an empty batch only loads the device code and looks up the array (a start-up call)
     if (j->pairs == 0) return AMPCOR_OK;
@@ -2259,9 +2255,10 @@ extern "C" int ampcor_correlate_noalloc(const ampcor_params* p, const ampcor_job
     const int refine_smem = std::max(ic.smem_bytes, iw.smem_bytes);
     for (long long c0 = 0; c0 < P; c0 += chunk) {
         const long long n = std::min(chunk, P - c0);
-        refine_kernel<<<(unsigned)n, kThreads, refine_smem, st>>>(src, c0, n, coarse, ic, iw, taps,
+        refine_kernel<false><<<(unsigned)n, kThreads, refine_smem, st>>>(src, c0, n, coarse, ic, iw, taps,
                                                                   taps + chip_taps, refined, refined_stride,
-                                                                  (p->flags & AMPCOR_FLAG_DERAMP) ? 1 : 0);
+                                                                  (p->flags & AMPCOR_FLAG_DERAMP) ? 1 : 0, 0.0,
+                                                                  nullptr, nullptr);
         fine_kernel<<<(unsigned)n, kThreads, gf.smem_bytes, st>>>(
             refined, refined_stride, c0, n, ref_off, gf, zg, taps + chip_taps + win_taps, coarse, peak, M, f,
             m, (p->flags & AMPCOR_FLAG_REF_COMPAT) ? 1 : 0, reinterpret_cast<float2*>(j->offsets),

@@ -19,6 +19,8 @@
 // butterfly sums them.  Shared-memory row strides are odd so that both lane layouts are free of
 // bank conflicts.  Partial sums are combined in a fixed order, so every result is bitwise
 // independent of what else runs on the device.
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "tile_common.cuh"
 
@@ -267,9 +269,19 @@ __device__ __forceinline__ void interp_ring(const float* __restrict__ tp,
 }
 
 // upsample the complex N x N tile at src by f and write the amplitudes (F x F, dense) to out
-__device__ void interp_tile(const float2* __restrict__ src, long long src_stride,
-                            const InterpGeom& ig, const float* __restrict__ taps_g, float* smem,
-                            float* __restrict__ out, int deramp)
+// (the kinds of sums of the interpolated amplitudes: none; a chip's, FP64 for every amplitude; a window's,
+// FP32 per thread about the thread's first amplitude, FP64 from there on, as refine_half_kernel takes them)
+enum { kNoSums, kChipSums, kWindowSums };
+
+// what the sums come to: sum, sum of squares, and sum of squares about the pivots
+struct TileSums {
+    double s1, s2, about;
+};
+
+template <int SUMS>
+__device__ TileSums interp_tile(const float2* __restrict__ src, long long src_stride,
+                                const InterpGeom& ig, const float* __restrict__ taps_g, float* smem,
+                                float* __restrict__ out, int deramp)
 {
     float2* X = reinterpret_cast<float2*>(smem + ig.off_x);
     float2* Y = reinterpret_cast<float2*>(smem + ig.off_y);
@@ -320,11 +332,24 @@ __device__ void interp_tile(const float2* __restrict__ src, long long src_stride
     __syncthreads();
 
     // columns: out[f q][p] = |Y[q][p]|, out[f q + s][p] interpolated
+    using Sum = std::conditional_t<SUMS == kChipSums, double, float>;
+    Sum s1 = 0, s2 = 0, pivot = 0;
+    int terms = 0;
+    auto put = [&](long long at, float re, float im) {
+        const float a = sqrtf(re * re + im * im);
+        out[at] = a;
+        if constexpr (SUMS != kNoSums) {
+            if (SUMS == kWindowSums && terms == 0) pivot = a;
+            const Sum v = (Sum)a - pivot;
+            s1 += v;
+            s2 = fma(v, v, s2);
+            ++terms;
+        }
+    };
     for (int idx = threadIdx.x; idx < N * F; idx += kThreads) {
         const int q = idx / F, p = idx - q * F;
         const float2 y = Y[q * YS + p];
-        const float re = y.x + mu.x, im = y.y + mu.y;
-        out[(long long)(f * q) * F + p] = sqrtf(re * re + im * im);
+        put((long long)(f * q) * F + p, y.x + mu.x, y.y + mu.y);
     }
     const int npb = (F + 31) / 32;
     for (int t = warp; t < (f - 1) * nqb * npb; t += kWarps) {
@@ -339,13 +364,28 @@ __device__ void interp_tile(const float2* __restrict__ src, long long src_stride
             for (int q = 0; q < kQB; ++q) ar[q] = ai[q] = 0.0f;
             interp_ring(taps + (s - 1) * ig.taps_len + q0, Y + (N - 1) * YS + p, -YS, N, ar, ai);
 #pragma unroll
-            for (int q = 0; q < kQB; ++q) {
-                const float re = ar[q] + mu.x, im = ai[q] + mu.y;
-                out[(long long)(f * (q0 + q) + s) * F + p] = sqrtf(re * re + im * im);
-            }
+            for (int q = 0; q < kQB; ++q) put((long long)(f * (q0 + q) + s) * F + p, ar[q] + mu.x, ai[q] + mu.y);
         }
     }
     __syncthreads();
+    TileSums all{0.0, 0.0, 0.0};
+    if constexpr (SUMS != kNoSums) {
+        // (the row-interpolated buffer is free again)
+        double* red = reinterpret_cast<double*>(Y);
+        const double k = pivot, n = terms;
+        const double sum[3] = {warp_sum(n * k + (double)s1), warp_sum((double)s2 + k * (2.0 * (double)s1 + n * k)),
+                               warp_sum((double)s2)};
+        if (lane == 0)
+            for (int q = 0; q < 3; ++q) red[3 * warp + q] = sum[q];
+        __syncthreads();
+        for (int w = 0; w < kWarps; ++w) {
+            all.s1 += red[3 * w];
+            all.s2 += red[3 * w + 1];
+            all.about += red[3 * w + 2];
+        }
+        __syncthreads();
+    }
+    return all;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -512,10 +552,12 @@ coarse_kernel(PairSource src, long long pair0, long long pairs, NccGeom g, int m
     }
 }
 
+template <bool STATS>
 __global__ void __launch_bounds__(kThreads, 1)
 refine_kernel(PairSource src, long long pair0, long long pairs, const CoarseOut* coarse,
               InterpGeom chip_g, InterpGeom win_g, const float* chip_taps, const float* win_taps,
-              float* refined, long long refined_stride, int deramp)
+              float* refined, long long refined_stride, int deramp, double flat, TileStat* chip_stats,
+              TileStat* win_stats)
 {
     extern __shared__ __align__(16) float smem[];
     if (blockIdx.x >= pairs) return;
@@ -523,11 +565,26 @@ refine_kernel(PairSource src, long long pair0, long long pairs, const CoarseOut*
     const long long roff = src.ref_off[p], toff = src.tgt_off[p];
     if (roff < 0 || toff < 0) return;
     float* out = refined + (long long)blockIdx.x * refined_stride;
-    interp_tile(src.ref_base + roff, src.ref_stride, chip_g, chip_taps, smem, out, deramp);
+    const TileSums chip = interp_tile<STATS ? kChipSums : kNoSums>(src.ref_base + roff, src.ref_stride, chip_g,
+                                                                   chip_taps, smem, out, deramp);
     const CoarseOut co = coarse[p];
-    interp_tile(src.tgt_base + toff + co.top * src.tgt_stride + co.left, src.tgt_stride, win_g,
-                win_taps, smem, out + (long long)chip_g.F * chip_g.F, deramp);
+    const TileSums win = interp_tile<STATS ? kWindowSums : kNoSums>(
+        src.tgt_base + toff + co.top * src.tgt_stride + co.left, src.tgt_stride, win_g, win_taps, smem,
+        out + (long long)chip_g.F * chip_g.F, deramp);
+    if (STATS && threadIdx.x == 0) {
+        const double nc = (double)chip_g.F * chip_g.F, nw = (double)win_g.F * win_g.F;
+        chip_stats[blockIdx.x] = chip_stat(0.0, chip.s1, chip.s2, nc, flat);
+        // (a window's slack: the FP32 rounding of a thread's sum of squares, 50 terms of 160 x 160 samples)
+        win_stats[blockIdx.x] = window_stat(0.0, win.s1, win.s2, nw, 1e-5 * win.about);
+    }
 }
+
+template __global__ void refine_kernel<false>(PairSource, long long, long long, const CoarseOut*, InterpGeom, InterpGeom,
+                                              const float*, const float*, float*, long long, int, double, TileStat*,
+                                              TileStat*);
+template __global__ void refine_kernel<true>(PairSource, long long, long long, const CoarseOut*, InterpGeom, InterpGeom,
+                                             const float*, const float*, float*, long long, int, double, TileStat*,
+                                             TileStat*);
 
 __global__ void __launch_bounds__(kThreads, 1)
 fine_kernel(const float* refined, long long refined_stride, long long pair0, long long pairs,

@@ -95,6 +95,17 @@ struct CoarseOut {
     int top, left;     // nudged corner of the refinement neighbourhood inside the window
 };
 
+// statistics of an amplitude tile, FP64: its mean; of a chip, 1/|r - mean| (0 for a constant one);
+// of a window, |t - mean| from above (it only scales the transform's error bound)
+struct TileStat {
+    double mean;
+    double inv_norm;
+    double norm;
+};
+// the share of a chip's sum of squares up to which its deviations are its amplitudes' rounding: a
+// refined chip that one tile correlates counts as constant up to here
+constexpr double kFlatChip = 1e-14;
+
 // The coarse cell (u, v) and the corner of its refinement neighbourhood, nudged into the window
 // (nudge.cu:107-140; argument roles from nudge.cu:57: old = W, new = R + 2m).  A surface without a
 // maximum (NaN) hands in a cell far outside: its corner still lies inside.
@@ -167,10 +178,13 @@ __global__ void arena_offsets_kernel(long long pairs, long long ref_cells, long 
 __global__ void coarse_kernel(PairSource src, long long pair0, long long pairs, NccGeom g, int m,
                               CoarseOut* out, float* coarse_peak, float* surfaces);
 
+// (STATS: with the statistics of the refined tiles, for the spectral form)
+template <bool STATS>
 __global__ void refine_kernel(PairSource src, long long pair0, long long pairs,
                               const CoarseOut* coarse, InterpGeom chip_g, InterpGeom win_g,
                               const float* chip_taps, const float* win_taps, float* refined,
-                              long long refined_stride, int deramp);
+                              long long refined_stride, int deramp, double flat, TileStat* chip_stats,
+                              TileStat* win_stats);
 
 __global__ void fine_kernel(const float* refined, long long refined_stride, long long pair0,
                             long long pairs, const long long* ref_off, NccGeom g, ZoomGeom zg,
@@ -354,17 +368,6 @@ struct InvSource {
     long long stride;
 };
 
-// statistics of an amplitude tile, FP64: its mean; of a chip, 1/|r - mean| (0 for a constant one);
-// of a window, |t - mean| from above (it only scales the transform's error bound)
-struct TileStat {
-    double mean;
-    double inv_norm;
-    double norm;
-};
-// the share of a chip's sum of squares up to which its deviations are its amplitudes' rounding: a
-// refined chip that one tile correlates counts as constant up to here
-constexpr double kFlatChip = 1e-14;
-
 // the transform lengths that are compiled, with their radices
 bool spec_radices(int n, int& n1, int& n2);
 int spec_next_length(int w);
@@ -385,11 +388,8 @@ cudaError_t launch_refine_half(int n, unsigned blocks, cudaStream_t st, const fl
 // blocked spectral correlation (windows too large for one tile; see spectral.cu): per chunk of
 // pairs the chip statistics, the placement statistics when no raster gives them, the partial
 // numerators of every (pair, chip block) and their per-pair reduction to the stage's outputs
-// (the chips of src, R x R samples, or its windows, R x R too)
 cudaError_t launch_spec_chip_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                   long long pairs, const long long* valid, int R, double flat, TileStat* out);
-cudaError_t launch_spec_window_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                     long long pairs, const long long* valid, int R, TileStat* out);
+                                   long long pairs, const long long* valid, int R, TileStat* out);
 int spec_tile_stats_rows(int W, int C, int& smem);
 cudaError_t launch_spec_tile_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
                                    long long pairs, const long long* valid, int R, int W, float* inv);

@@ -1162,12 +1162,12 @@ spec_staged_kernel(SpecSource src, long long pair0, long long pairs, const long 
 // s is the mean of the s_k: the c do not sum to 0 but to their roundings, and a steady return's level
 // must not multiply those (128 px chips under a return of 300: off by up to 8.4e-6 with s = 0).
 
-// one CTA of 256 threads per pair: the FP64 statistics of the R x R chip, or (window) window, from sums
-// about its first sample (the differences and their squares are exact, so that a strong steady return
-// costs their sums no digits)
+// one CTA of 256 threads per pair: the FP64 statistics of the R x R chip, from sums about its first
+// sample (the differences and their squares are exact, so that a strong steady return costs their sums
+// no digits)
 __global__ void __launch_bounds__(256)
-spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, int R, bool window,
-                       double flat, TileStat* out)
+spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, int R,
+                       TileStat* out)
 {
     __shared__ double red[16];
     if (blockIdx.x >= pairs) return;
@@ -1177,8 +1177,8 @@ spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const l
         if (tid == 0) out[blockIdx.x] = TileStat{0.0, 0.0, 0.0};
         return;
     }
-    const float* chip = window ? spec_win(src, pair0, blockIdx.x) : spec_chip(src, pair0, blockIdx.x);
-    const long long cs = window ? src.win_stride : src.chip_stride;
+    const float* chip = spec_chip(src, pair0, blockIdx.x);
+    const long long cs = src.chip_stride;
     const double pivot = __ldg(chip);
     double s1 = 0.0, s2 = 0.0;
     for (int y = warp; y < R; y += 8)
@@ -1200,9 +1200,7 @@ spec_chip_stats_kernel(SpecSource src, long long pair0, long long pairs, const l
             a += red[2 * w];
             b += red[2 * w + 1];
         }
-        // (a window's slack: the rounding of up to 2^16 FP64 terms)
-        const double n = (double)R * (double)R;
-        out[blockIdx.x] = window ? window_stat(pivot, a, b, n, 1e-11 * b) : chip_stat(pivot, a, b, n, flat);
+        out[blockIdx.x] = chip_stat(pivot, a, b, (double)R * (double)R, 0.0);
     }
 }
 
@@ -1776,16 +1774,9 @@ cudaError_t spec_set_smem_limits()
 }
 
 cudaError_t launch_spec_chip_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                   long long pairs, const long long* valid, int R, double flat, TileStat* out)
+                                   long long pairs, const long long* valid, int R, TileStat* out)
 {
-    spec_chip_stats_kernel<<<blocks, 256, 0, st>>>(src, pair0, pairs, valid, R, false, flat, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_spec_window_stats(unsigned blocks, cudaStream_t st, SpecSource src, long long pair0,
-                                     long long pairs, const long long* valid, int R, TileStat* out)
-{
-    spec_chip_stats_kernel<<<blocks, 256, 0, st>>>(src, pair0, pairs, valid, R, true, 0.0, out);
+    spec_chip_stats_kernel<<<blocks, 256, 0, st>>>(src, pair0, pairs, valid, R, out);
     return cudaGetLastError();
 }
 
