@@ -525,7 +525,7 @@ zoom_kernel(const float* gam, long long pair0, long long pairs, const long long*
 // itself - their columns of T, the sampled rows, its list of kept rows and those - with one barrier, before
 // the list, so that every warp's largest cell bounds it.  The blocks are 8 NR columns by 4 NC rows, the
 // longer side on the 4 lanes whose loads cost two wavefronts (lanes next to each other read 8 rows there:
-// four); NC = 9 covers the 33 rows of the production surface at once.  Every second sampled row of an
+// four); NC = 9 covers the 33 rows of the production surface at once, NC = 5 those of 17.  Every second sampled row of an
 // even zoom is a row of T itself.  Few columns (a peak) go in sets of 8, so that more warps have some.
 template <int NR, int NC>
 __device__ __forceinline__ void wide_sets(const ZoomGeomCols& g, const float* U, const float* G, float* T, float* val,
@@ -786,7 +786,7 @@ cudaError_t zoom_set_smem_limits()
 {
     const int limit = 227 * 1024;
     cudaError_t e = cudaSuccess;
-    for (auto* k : {zoom_wide_kernel<5>, zoom_wide_kernel<9>})
+    for (auto* k : {zoom_wide_kernel<5>, zoom_wide_kernel<6>, zoom_wide_kernel<9>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     for (auto* k : {zoom_kernel<3, kZoomTeams>, zoom_kernel<9, 3>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
@@ -820,7 +820,11 @@ cudaError_t launch_zoom_kernel(unsigned sms, cudaStream_t st, const float* gam, 
     // (444 surfaces 16.3 us, 14.3 with teams of three).  More: teams of three, which wait for each other least,
     // and two sets of columns to a batch (noise 1,680 us against 1,747 with one, peaks the same).
     if (each == 1 && 4L * zoom_wide(g).floats <= room) {
-        auto* kernel = g.Cf <= 20 ? zoom_wide_kernel<5> : zoom_wide_kernel<9>;
+        // (blocks of 20, 24 or 36 rows: those that reach past Cf least)
+        auto past = [&](int nc) { return (g.Cf + 4 * nc - 1) / (4 * nc) * nc; };
+        auto* kernel = past(9) <= std::min(past(5), past(6)) ? zoom_wide_kernel<9>
+                       : past(6) <= past(5)                  ? zoom_wide_kernel<6>
+                                                             : zoom_wide_kernel<5>;
         kernel<<<n, kWideWarps * 32, g.off_team + 4 * zoom_wide(g).floats, st>>>(
             gam, pair0, ref_off, g, u, coarse, coarse_peak, fout, margin, refine_factor, refine_margin, ref_compat,
             offsets, diag, err_out, stall);

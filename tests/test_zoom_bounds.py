@@ -33,14 +33,16 @@ def corners(n):
 
 @pytest.mark.parametrize("each", ["one", "two", "five"])
 @pytest.mark.parametrize("kind", ["peak", "noise"])
-@pytest.mark.parametrize("m,z", [(4, 2), (4, 5), (4, 7), (8, 2), (8, 3), (8, 5), (8, 7), (8, 8), (12, 4)])
-def test_maximum(m, z, kind, each):
+# (surfaces of 17, 33 and 49 samples, and of 41 at the refinement factor 5)
+@pytest.mark.parametrize("m,z,f", [(4, 2, 2), (4, 5, 2), (4, 7, 2), (8, 2, 2), (8, 3, 2), (8, 5, 2), (8, 7, 2), (8, 8, 2),
+                                   (12, 4, 2), (4, 3, 5), (4, 4, 5)])
+def test_maximum(m, z, f, kind, each):
     n = pair_counts()[each]
     ref = synth.speckle((300, 300), 21)
     tgt = synth.fourier_shift(ref, 1.3, -2.2) if kind == "peak" else synth.speckle((300, 300), 22)
-    R = 32 if m < 12 else 40  # (chip and R + 2 m both compiled tiles of the refinement)
+    R = 16 if f == 5 else 32 if m < 12 else 40  # (at factor 2 chip and R + 2 m are compiled tiles of the refinement)
     ulhc = corners(n)
-    worker = Worker(n, (R, R), (64, 64), refine_factor=2, refine_margin=m, zoom_factor=z)
+    worker = Worker(n, (R, R), (64, 64), refine_factor=f, refine_margin=m, zoom_factor=z)
     if worker.form != "spectral":
         pytest.skip("no spectral form of this geometry")
     dev = torch.device("cuda:0")
