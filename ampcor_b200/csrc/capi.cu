@@ -435,8 +435,8 @@ bool plan_spec_block_staged(int K, SpecGeom& g)
 // R + Cq - 1 samples, Cq of C placements a side (the second ones from placement C - Cq on, a multiple of 4 so that
 // tensor copies start on 16 bytes), each an ordinary staged correlation with its own maximum.  That
 // pays where four such tiles are smaller than the K tiles of the chip's blocks: 64 px chips and
-// +-64 px are four tiles of 128 samples against four of 160 and a reduction, 900 pairs 1,094 -> 526 us
-// (the job 1,551 -> 988); 128 px chips and +-32 px would be four of 160 against four of 128.
+// +-64 px are four tiles of 128 samples against four of 160 and a reduction, 900 pairs 1,094 -> 560 us
+// (the job 1,551 -> 1,014); 128 px chips and +-32 px would be four of 160 against four of 128.
 bool plan_spec_parts(int R, int W, const SpecBlocks& b, int& Cq, SpecGeom& g)
 {
     std::string e;
@@ -1136,7 +1136,7 @@ bool tiles_map(CUtensorMap& m, const float* base, int n, long long pairs, long l
 
 // A raster whose lines are no whole 16-byte units of floats gets an amplitude raster of longer lines, so
 // that the copy engine can serve its windows: 2,028 pairs of 64 px chips on 1531 x 1999 samples, coarse stage
-// 318 -> 257 us, the job 1,120 -> 1,062.  The amplitudes (and statistics) then have strides and tile offsets of their own.
+// 318 -> 270 us, the job 1,120 -> 1,060.  The amplitudes (and statistics) then have strides and tile offsets of their own.
 void pad_lines(ampcor_handle* h, PairSource& src)
 {
     if (h->form != kFormSpectral || src.tgt_lines <= 0 || src.ref_stride <= 0 || src.tgt_stride <= 0) return;

@@ -13,12 +13,12 @@
 // of a 2 N x N one, so that two to eight CTAs share an SM for tiles up to 96 samples and the larger ones
 // need no buffer in global memory.
 //
-// What bounds it: instruction issue, with shared-memory wavefronts next (ncu, 80-sample tiles: 62 %
-// of issue slots, the FMA pipes 42 %, 10.7K wavefronts of 21K cycles a tile; 15 % of the time goes
-// into the IEEE square roots of the outputs, 15 % into the middle pass).  Measured on B200, a chip of
-// 64 and a window of 80 samples for each of 14,641 pairs: 2,426 us padded, 1,594 us by shifts, 1,458
-// us with packed sums and strips of 32 rows, 1,561 us with the tiles' statistics on the way out (which
-// save the correlation kernels more); 3,844 pairs of 128 and 144 samples 3,235 -> 1,912 us.
+// What bounds it: instruction issue (ncu: 68 % of the slots busy), with shared-memory wavefronts next;
+// 15 % of the time goes into the IEEE square roots of the outputs, 15 % into the middle pass.  Measured
+// on B200, a chip of 64 and a window of 80 samples for each of 14,641 pairs: 2,426 us padded, 1,594 us by
+// shifts, 1,458 us with packed sums and strips of 32 rows, 1,538 us with the tiles' statistics on the way
+// out (a chip's amplitudes summed in FP64; they save the fine stage more); 3,844 pairs of 128 and 144
+// samples 3,235 -> 1,904 us.
 #include <algorithm>
 #include <type_traits>
 

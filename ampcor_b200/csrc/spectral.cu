@@ -1346,8 +1346,9 @@ spec_block_kernel(SpecSource src, long long pair0, long long pairs, const long l
 // the centring are spec_block_kernel's.  Bounded waits as in spec_staged_kernel; the partial
 // numerators of pairs left out after one ran out are undefined, their maxima still placements.
 // Measured on B200, 3,844 pairs of 128 px chips: the coarse stage (four 128-sample tiles a pair) 2,136
-// us unstaged, 1,910 staged block by block, 1,534 with the spectra summed; the fine stage (four
-// 160-sample tiles, whose 104 KB spectrum fits nowhere beside them) 3,025 -> 2,603 us.
+// us unstaged, 1,910 staged block by block, 1,534 with the spectra summed (60 more with every sample of a
+// chip block summed in FP64); the fine stage (four 160-sample tiles, whose 104 KB spectrum fits nowhere
+// beside them) 3,025 -> 2,603 us.
 template <int N1, int N2, bool ACC>
 __global__ void __launch_bounds__(kSpecThreads, 1)
 spec_block_staged_kernel(SpecSource src, long long pair0, long long pairs, const long long* valid, SpecGeom g,
