@@ -26,6 +26,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "-shared", "-Xlinker", "--no-undefined",
+    "--threads", "0",  # the sources side by side
 ]
 
 LIB = os.path.join(HERE, "libampcor_b200.so")
